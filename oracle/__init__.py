@@ -28,7 +28,7 @@ def build(ref=True):
     """Builds liboracle.so, and where the reference sources are present the
     reference library and the drop-in checker (which links the GPU library)."""
     targets = ["oracle"]
-    if ref and os.path.isdir(os.environ.get("BIELCC_REF_SRC", "/root/reference")):
+    if ref and os.path.isdir(os.path.join(os.environ.get("BIELCC_REF_SRC", "/root/reference"), "electrodynamics")):
         targets.append("ref")
         if os.path.exists(os.path.join(HERE, "..", "bielcc_b200", "libbielcc_gpu.so")):
             targets.append("dropin")
