@@ -162,7 +162,27 @@ void free_mesh(MeshDev* m) {
     cudaFree(m->nodes64_hi);
     cudaFree(m->nodes32_hi);
     cudaFree(m->rho32_hi);
+    cudaFree(m->rules_mem);
+    cudaFree(m->rules_lo_mem);
+    cudaFree(m->rules_hi_mem);
     delete m;
+}
+
+// The compressed rules of an n-split table (rules.cu), in an allocation of their
+// own; without room for it the far pass runs on the full rows.
+int build_rules(MeshDev* m, int n, void** mem, FarRules* out, cudaStream_t s) {
+    cudaFree(*mem);
+    *mem = nullptr;
+    *out = FarRules();
+    const size_t b = rules_bytes(m->nv, n, m->n_cells);
+    if (!b) return BIELCC_OK;
+    if (cudaMalloc(mem, b) != cudaSuccess) {
+        cudaGetLastError();
+        *mem = nullptr;
+        return BIELCC_OK;
+    }
+    TRY_CUDA(launch_rules(m->verts, m->geo, m->rho32, m->nv, m->n_cells, n, *mem, out, s));
+    return BIELCC_OK;
 }
 
 // Node tables for split n, built on first use and cached on the mesh.
@@ -180,6 +200,7 @@ int ensure_tables(MeshDev* m, int n, cudaStream_t s) {
     TRY_CUDA(cudaMalloc(&m->nodes32, nn * sizeof(float4) + 16));
     TRY_CUDA(cudaMalloc(&m->rho32, (size_t)m->n_cells * sizeof(float) + 16));
     TRY_CUDA(launch_node_tables(m->verts, m->geo, m->nv, m->n_cells, n, m->nodes64, m->nodes32, m->rho32, s));
+    TRY(build_rules(m, n, &m->rules_mem, &m->rules, s));
     m->table_n = n;
     return BIELCC_OK;
 }
@@ -196,6 +217,7 @@ int ensure_far_tables(MeshDev* m, const NumParamH& np, cudaStream_t s) {
         TRY_CUDA(cudaMalloc(&m->nodes64_lo, (size_t)np.n_start * np.n_start * m->n_cells * sizeof(double4) + 16));
         TRY_CUDA(launch_node_tables(m->verts, m->geo, m->nv, m->n_cells, np.n_start, m->nodes64_lo, nullptr, nullptr,
                                     s));
+        TRY(build_rules(m, np.n_start, &m->rules_lo_mem, &m->rules_lo, s));
         m->table_lo_n = np.n_start;
     }
     const int n3 = 4 * np.n_start;
@@ -213,6 +235,7 @@ int ensure_far_tables(MeshDev* m, const NumParamH& np, cudaStream_t s) {
         TRY_CUDA(cudaMalloc(&m->rho32_hi, (size_t)m->n_cells * sizeof(float) + 16));
         TRY_CUDA(launch_node_tables(m->verts, m->geo, m->nv, m->n_cells, n3, m->nodes64_hi, m->nodes32_hi,
                                     m->rho32_hi, s));
+        TRY(build_rules(m, n3, &m->rules_hi_mem, &m->rules_hi, s));
         m->table_hi_n = n3;
     }
     return BIELCC_OK;
@@ -287,6 +310,7 @@ int field_device_batched(bielcc_ctx ctx, const FieldArgs& a, cudaStream_t s, bie
     d.nodes32 = a.m->nodes32;
     d.nodes64 = a.m->nodes64;
     d.rho32 = a.m->rho32;
+    d.rules = a.m->rules;
     d.verts = a.m->verts;
     d.nv = a.m->nv;
     d.n_cells = a.m->n_cells;
@@ -660,6 +684,9 @@ int bielcc_ctx_mem_used(bielcc_ctx ctx, int64_t* bytes) {
         if (m->table_n) b += (int64_t)m->n_cells * m->table_n * m->table_n * (32 + 16) + 4 * m->n_cells;
         if (m->table_lo_n) b += (int64_t)m->n_cells * m->table_lo_n * m->table_lo_n * 32;
         if (m->table_hi_n) b += (int64_t)m->n_cells * m->table_hi_n * m->table_hi_n * (32 + 16) + 4 * m->n_cells;
+        if (m->rules_mem) b += rules_bytes(m->nv, m->table_n, m->n_cells);
+        if (m->rules_lo_mem) b += rules_bytes(m->nv, m->table_lo_n, m->n_cells);
+        if (m->rules_hi_mem) b += rules_bytes(m->nv, m->table_hi_n, m->n_cells);
     }
     *bytes = b;
     return BIELCC_OK;
@@ -971,6 +998,7 @@ int jobs_to_dev(int n_jobs, const bielcc_field_job* jobs, const std::vector<Mesh
         d.nodes32 = m->nodes32;
         d.nodes64 = m->nodes64;
         d.rho32 = m->rho32;
+        d.rules = m->rules;
         d.verts = m->verts;
         d.nv = m->nv;
         d.n_cells = m->n_cells;

@@ -14,14 +14,121 @@
 // product leave the per-node work).
 #pragma once
 #include "common.cuh"
+#include "internal.h"
 
 namespace bielcc_gpu {
 
-// Near decision of get_field.h:58 with the reference's rounding.
+// Near decision of get_field.h:58 with the reference's rounding: sqrt_rn(s) < t
+// for the rounded sum of squares s of x - c and t = analytic_calc * diam. The
+// rounded root is monotone, so this is s < T with T the smallest FP64 number
+// whose rounded root reaches t: found once per staged cell from t^2 by a step or
+// two up or down, it leaves one comparison per pair.
+BIELCC_D double near_square(double t) {
+    if (!(t > 0.)) return t != t ? t : 0.;  // no distance is below a t <= 0 (or NaN)
+    double T = __dmul_rn(t, t);
+    while (T > 0. && __dsqrt_rn(__longlong_as_double(__double_as_longlong(T) - 1)) >= t)
+        T = __longlong_as_double(__double_as_longlong(T) - 1);
+    while (__dsqrt_rn(T) < t) T = __longlong_as_double(__double_as_longlong(T) + 1);
+    return T;
+}
+// cell row for near_exact: centre and T
+BIELCC_D double4 near_cell(const CellGeo& g, double analytic_calc) {
+    return make_double4(g.c[0], g.c[1], g.c[2], near_square(__dmul_rn(analytic_calc, g.diam)));
+}
+BIELCC_D bool near_exact(const double* x, const double4& cell, double (&d)[3], double* s) {
+    d[0] = __dsub_rn(x[0], cell.x);
+    d[1] = __dsub_rn(x[1], cell.y);
+    d[2] = __dsub_rn(x[2], cell.z);
+    *s = __dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2]));
+    return *s < cell.w;
+}
+
+// sqrt(s) in FP64 from the FP32 reciprocal root and one third-order step (about
+// an ulp; EXACT: with a correction, half an ulp and a bit); outside the FP32
+// range (and for NaN) the library root.
+template <bool EXACT = true>
+BIELCC_D double dist_from_sq(double s) {
+    const float sf = (float)s;
+    if (!(sf > 1e-30f && sf < 1e30f)) return sqrt(s);
+    double y = (double)rsqrtf(sf);
+    const double e = fma(-s * y, y, 1.0);
+    y = fma(y * e, fma(e, 0.375, 0.5), y);
+    const double d = s * y;
+    return EXACT ? fma(fma(-d, d, s), 0.5 * y, d) : d;
+}
+
+// e^{i 2 pi t} for FP32 use, t in turns: the quarter turn is taken off in FP64
+// (magic-number rounding; exact), sine and cosine of the rest, |a| <= pi / 4, from
+// their Taylor series (truncation below 2e-9), in FP64, scaled by `amp`.
+BIELCC_D void turn_f32(double t, double amp, float* c, float* s) {
+    const double big = fma(t, 4.0, 6755399441055744.0);  // 1.5 2^52: rounds to an integer
+    const int j = __double2loint(big);
+    const double a = fma(-0.25, big - 6755399441055744.0, t) * 6.283185307179586477;
+    const double q = a * a;
+    const double ps = fma(fma(fma(fma(q, 1.0 / 362880, -1.0 / 5040), q, 1.0 / 120), q, -1.0 / 6), q, 1.0);
+    const double pc =
+        fma(fma(fma(fma(fma(q, -1.0 / 3628800, 1.0 / 40320), q, -1.0 / 720), q, 1.0 / 24), q, -0.5), q, 1.0);
+    const float sf = (float)(a * ps * amp), cf = (float)(pc * amp);
+    const float c0 = (j & 1) ? sf : cf, s0 = (j & 1) ? cf : sf;
+    *c = ((j + 1) & 2) ? -c0 : c0;
+    *s = (j & 2) ? -s0 : s0;
+}
+constexpr double kInvTwoPi = 0.15915494309189533577;
+
+// The same decision from the root itself, which *d_out receives.
 BIELCC_D bool is_near(const double* x, const double* c, double diam, double analytic_calc, double* d_out) {
     double d = dist3_rn(x, c);
     *d_out = d;
     return d < __dmul_rn(analytic_calc, diam);
+}
+
+// Rows of the far pass's quadrature (rules.cu): level l < n_lev is a compressed
+// rule, level n_lev the full n^2-node table. The CTA keeps base and length of
+// every level in shared memory.
+template <typename NodeT>
+struct RuleTab {
+    const NodeT* base[kMaxRules + 1];
+    int cnt[kMaxRules + 1];
+    int n_lev;
+    // one thread fills it; the caller synchronises
+    BIELCC_D void fill(const FarRules& r, const NodeT* rows, const NodeT* full, int nn, int n_cells) {
+        n_lev = r.n_lev;
+        for (int l = 0; l < r.n_lev; l++) {
+            base[l] = rows + (size_t)r.off[l] * n_cells;
+            cnt[l] = r.cnt[l];
+        }
+        base[r.n_lev] = full;
+        cnt[r.n_lev] = nn;
+    }
+};
+BIELCC_D const float4* rule_rows(const FarRules& r, float4) { return r.n32; }
+BIELCC_D const double4* rule_rows(const FarRules& r, double4) { return r.n64; }
+BIELCC_D const float2* rule_limits(const FarRules& r, float4) { return r.thr32; }
+BIELCC_D const float2* rule_limits(const FarRules& r, double4) { return r.thr64; }
+// A node of a row in global memory (the same address for the whole warp).
+BIELCC_D double4 ldg_node(const double4* p) {
+    const double2* q = reinterpret_cast<const double2*>(p);
+    const double2 a = __ldg(q), b = __ldg(q + 1);
+    return make_double4(a.x, a.y, b.x, b.y);
+}
+// |k| as the limits take it, and a limit's smallest distance at that |k|.
+BIELCC_D float rule_kabs(cplx k) { return (float)(sqrt(cabs2(k)) * (1.0 + 1e-6)); }
+BIELCC_D float rule_rmin(float2 lim, float kabs) { return kabs <= lim.y ? lim.x : __int_as_float(0x7f800000); }
+
+// Smallest of the warp's values (all >= 0): every lane calls.
+BIELCC_D float warp_min_pos(float v) { return __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(v))); }
+// A lane's distance as that minimum takes it: infinity for a lane that does not
+// take part; finite otherwise (a NaN or infinite distance takes part, so that it
+// reaches the result: 0 asks for the full row).
+BIELCC_D float rule_key(bool far, double d) {
+    return far ? fminf(fmaxf((float)d, 0.f), 3e38f) : __int_as_float(0x7f800000);
+}
+// Shortest row usable from distance r (a warp's smallest, so the level is
+// uniform over the warp): rmin[l], l < n_lev, decreases with l.
+BIELCC_D int rule_level(const float* rmin, int n_lev, float r) {
+    int l = 0;
+    while (l < n_lev && !(r >= rmin[l])) l++;
+    return l;
 }
 
 // Per-thread moment accumulators of one cell.
@@ -238,6 +345,14 @@ BIELCC_HD int phase_mode(float th) {
     return th <= 0.25f ? 0 : (th <= 1.f ? 1 : (th <= 2.f ? 2 : (th <= 4.f ? 3 : 4)));
 }
 
+// One staged node of a row chunk: FP32 rows carry |y - centre|^2 beside the node.
+constexpr int kRowChunk = 32;
+template <typename NodeT>
+struct RowBuf {
+    NodeT nd[kRowChunk];
+    float yy[sizeof(NodeT) == 16 ? kRowChunk : 1];
+};
+
 // Per-pair FP32 state of the mixed far node, relative to the cell centre:
 // X = x - centre, X2 = -2 X, r0 = |X| (FP64 rounded), r0sq = r0^2, r0k = r0 / Re k.
 struct PairF32 {
@@ -251,10 +366,29 @@ struct PairF32 {
         r0sq = (float)(d * d);
         r0k = r0 * kf.ikr;
     }
+    // from x - centre (FP64), |x - centre|^2 and |x - centre|
+    BIELCC_D void set(const double (&dx)[3], double s, double d, const KF32& kf) {
+#pragma unroll
+        for (int g = 0; g < 3; g++) {
+            X[g] = (float)dx[g];
+            X2[g] = -2.f * X[g];
+        }
+        r0 = (float)d;
+        r0sq = (float)s;
+        r0k = r0 * kf.ikr;
+    }
 };
 
 // |y - centre|^2 of a staged node (computed once per node and CTA).
 BIELCC_D float node_yy(float4 nd) { return fmaf(nd.x, nd.x, fmaf(nd.y, nd.y, nd.z * nd.z)); }
+
+// a / b by the approximate reciprocal alone (b positive and normal here, so the
+// scaling that __fdividef adds for large divisors is not needed).
+BIELCC_D float fast_div(float a, float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return a * r;
+}
 
 // Shared head of the FP32 far node: nd = (y - centre, w), yy = |y - centre|^2.
 // q = |x - y|^2 - r0^2 = yy - 2 (y - centre).X carries no cancellation.
@@ -268,11 +402,11 @@ BIELCC_D float far_head_f32(const PairF32& p, float4 nd, float yy, const KF32& k
     const float r = r2 * ir;
     float s, c, w = nd.w;
     if (CK) {
-        const float dr = __fdividef(q, r + p.r0);  // r - r0 without cancellation
+        const float dr = fast_div(q, r + p.r0);  // r - r0 without cancellation
         phase_f32<MODE>(kf.kr * dr, &s, &c);
         w *= __expf(-kf.ki * dr);
     } else {
-        phase_f32<MODE>(__fdividef(q, fmaf(r, kf.ikr, p.r0k)), &s, &c);  // k (r - r0)
+        phase_f32<MODE>(fast_div(q, fmaf(r, kf.ikr, p.r0k)), &s, &c);  // k (r - r0)
     }
     dx = p.X[0] - nd.x;
     dy = p.X[1] - nd.y;

@@ -3,13 +3,15 @@
 // counterpart (examples/field/main0_field_test.cpp:237-311) on sm_100a.
 //
 // Pipeline (one stream, deterministic summation order):
-//   1. far kernel   — one observation point per thread, cell node tiles staged
-//                     in shared memory with 128-bit loads, cells split across
+//   1. far kernel   — one observation point per thread, cells split across
 //                     gridDim.y (the split count is chosen per launch so that
-//                     the last wave of CTAs fills the GPU: grid.h);
+//                     the last wave of CTAs fills the GPU: grid.h) and, on
+//                     problems too small for that, across the CTA's warps;
 //                     far cells only (near cells skipped). Per cell
 //                     the J-independent moments A1 = sum w e f1,
-//                     T = sum w e f2 d^d^T, G = sum w grad F are accumulated and
+//                     T = sum w e f2 d^d^T, G = sum w grad F are accumulated over
+//                     the nodes of the shortest quadrature row that reproduces
+//                     the n x n sum to rounding at this distance (rules.cu) and
 //                     contracted with each right-hand side once per cell:
 //                       K_RotRot_Far  (K.h:288-301)  = (A1 J + T J) / 4pi
 //                       R_Rot_Colloc  (R.h:89-111)   = (G x J) / 4pi
@@ -47,36 +49,39 @@ namespace bielcc_gpu {
 #define BIELCC_FAR_THREADS 128
 #endif
 constexpr int kFarThreads = BIELCC_FAR_THREADS;
-// Unrolling of the mixed node loop (far launch on 8192 cells x 20,000 points:
-// x2 26.07 ms, x4 25.41 ms, x8 25.93 ms).
+// Unrolling of the mixed node loop (rows of 8 - 20 nodes mostly; 8192 cells x
+// 20,000 points, whole call: x2 7.23, x3 7.50, x4 7.26, x8 7.29 ms).
 #ifndef BIELCC_FAR_UNROLL
 #define BIELCC_FAR_UNROLL 4
 #endif
 #define BIELCC_FAR_STR(x) #x
 #define BIELCC_FAR_PRAGMA(x) _Pragma(BIELCC_FAR_STR(unroll x))
 #define BIELCC_FAR_UNROLL_PRAGMA BIELCC_FAR_PRAGMA(BIELCC_FAR_UNROLL)
-// Unrolling of the FP64 split node loop (FP64 step on 8192 cells x 20,000
-// points: x1 57.7, x2 56.4, x4 54.6, x8 53.3, x16 52.8 ms; registers 152-166).
+// Unrolling of the FP64 split node loop (5120 triangles x 6001 points, whole
+// call: x2 7.62, x3 7.62, x4 7.51, x5 7.58 ms; with the cells over the warps, where
+// the warps are at different places in the code, x8 costs 70 % more than x2 in
+// instruction-cache misses).
 #ifndef BIELCC_FAR64_UNROLL
-#define BIELCC_FAR64_UNROLL 16
+#define BIELCC_FAR64_UNROLL 3
 #endif
 #define BIELCC_FAR64_UNROLL_PRAGMA BIELCC_FAR_PRAGMA(BIELCC_FAR64_UNROLL)
 // Minimum resident CTAs per SM asked of the 1-RHS real-k mixed far kernel
 // (0: none, the compiler's own register choice, which the other variants
-// keep). 5 caps it at 96 registers without spills: 20 warps per SM instead of
-// 16 (far launch on 8192 cells x 20,000 points 25.87 -> 25.42 ms).
+// keep). 5 caps it at 96 registers without spills: 20 warps per SM (6: 80
+// registers, 8192 cells x 20,000 points 8.1 -> 9.0 ms).
 #ifndef BIELCC_FAR_MINB
 #define BIELCC_FAR_MINB 5
 #endif
-// The same for the 1-RHS real-k FP64 far kernel: 4 (127 registers) measured
-// slower than the compiler's own 152 (FP64 step 63.1 against 58.7 ms).
+// The same for the 1-RHS real-k FP64 far kernel: 4 (128 registers) measured
+// slower than the compiler's own 168 (5120 triangles x 6001 points 9.6 against
+// 7.6 ms).
 #ifndef BIELCC_FAR64_MINB
 #define BIELCC_FAR64_MINB 0
 #endif
 #define BIELCC_FAR_BOUNDS(NRHS_, CK_, MIXED_) \
     __launch_bounds__(kFarThreads, NRHS_ == 1 && !CK_ ? (MIXED_ ? BIELCC_FAR_MINB : BIELCC_FAR64_MINB) : 0)
-constexpr int kStageNodes = 256;
-constexpr int kMaxStageCells = 32;
+constexpr int kStageCells = 32;  // cells staged at a time: one near-mask word
+constexpr int kFarWays = 4;      // warps that share a split's cells on small problems
 
 struct FarArgs {
     const double* pts;
@@ -87,11 +92,13 @@ struct FarArgs {
     const float4* nodes32;
     const float* rho32;
     int nn;  // nodes per cell
+    FarRules rules;
     const cplx* J;  // [S][N][3]
     int n_rhs, rhs0;
     cplx k;
     double analytic_calc;
-    int cells_per_split;  // a multiple of 32: near-mask words never straddle splits
+    int cells_per_split;  // a multiple of 32, or 16 or 8: a split's cells never straddle near-mask words in part
+    int ways;             // 1, or kFarWays: the CTA's warps share the cells, 32 points per CTA
     double* partial;      // [split][S][12][P]
     unsigned* nearmask;   // [ceil(N/32)][P]: bit c%32 of word c/32 set iff (p, c) is near
 };
@@ -110,42 +117,49 @@ struct FarArgsMarks : FarArgs {
 template <bool MARKS>
 using FarArgsOf = typename std::conditional<MARKS, FarArgsMarks, FarArgs>::type;
 
-// Contract one cell's moments (times the phase P = pr + i pi) with the RHS
-// currents and add into the FP64 accumulators acc[r][12] =
-// (Ex, Ey, Ez, Hx, Hy, Hz) x (re, im).
+// Contract one cell's moments with the RHS currents times the phase P = pr + i pi
+// and add into the FP64 accumulators acc[r][12] = (Ex, Ey, Ez, Hx, Hy, Hz) x
+// (re, im): E = W J P with W = A1 I + T, H = G x J P. Real k: m holds (S, T/3)
+// (farnode.cuh), so W_aa = 2 S - 3 (the other two diagonal entries of T/3) and
+// W_ab = 3 (T/3)_ab. sj: the currents of the cell, (re, im) of x, y, z per RHS.
 // takeE: bit r adds RHS r's E; takeH: the H of every RHS (convergence-test
 // marks, p_max >= 3; all set otherwise).
-template <int NRHS, typename F>
-BIELCC_D void contract(const Moments<F>& m, F pr, F pi, const cplx (*sj)[3], bool zeroR, double (*acc)[12],
+template <int NRHS, bool CK, typename F>
+BIELCC_D void contract(const Moments<F>& m, F pr, F pi, const F (*sj)[6], bool zeroR, double (*acc)[12],
                        unsigned takeE = ~0u, bool takeH = true) {
-    // moments x phase
-    F A1r = m.a1r * pr - m.a1i * pi, A1i = m.a1r * pi + m.a1i * pr;
-    F T[6][2], G[3][2];
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        T[q][0] = m.t[q][0] * pr - m.t[q][1] * pi;
-        T[q][1] = m.t[q][0] * pi + m.t[q][1] * pr;
-    }
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        G[q][0] = m.g[q][0] * pr - m.g[q][1] * pi;
-        G[q][1] = m.g[q][0] * pi + m.g[q][1] * pr;
-    }
     const int ti[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+    F W[6][2];
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const F a1 = c ? m.a1i : m.a1r;
+        if (CK) {
+#pragma unroll
+            for (int q = 0; q < 6; q++) W[q][c] = m.t[q][c] + (q == 0 || q == 3 || q == 5 ? a1 : F(0));
+        } else {
+            const F s2 = a1 + a1;
+            W[0][c] = fma(F(-3), m.t[3][c] + m.t[5][c], s2);
+            W[3][c] = fma(F(-3), m.t[0][c] + m.t[5][c], s2);
+            W[5][c] = fma(F(-3), m.t[0][c] + m.t[3][c], s2);
+            W[1][c] = F(3) * m.t[1][c];
+            W[2][c] = F(3) * m.t[2][c];
+            W[4][c] = F(3) * m.t[4][c];
+        }
+    }
 #pragma unroll
     for (int rr = 0; rr < NRHS; rr++) {
         F jr[3], ji[3];
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            jr[a] = (F)sj[rr][a].re;
-            ji[a] = (F)sj[rr][a].im;
+            const F re = sj[rr][2 * a], im = sj[rr][2 * a + 1];
+            jr[a] = re * pr - im * pi;
+            ji[a] = re * pi + im * pr;
         }
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            F er = A1r * jr[a] - A1i * ji[a], ei = A1r * ji[a] + A1i * jr[a];
+            F er = 0, ei = 0;
 #pragma unroll
             for (int b = 0; b < 3; b++) {
-                const F* t = T[ti[a][b]];
+                const F* t = W[ti[a][b]];
                 er += t[0] * jr[b] - t[1] * ji[b];
                 ei += t[0] * ji[b] + t[1] * jr[b];
             }
@@ -157,9 +171,9 @@ BIELCC_D void contract(const Moments<F>& m, F pr, F pi, const cplx (*sj)[3], boo
         if (!zeroR && takeH) {
 #pragma unroll
             for (int a = 0; a < 3; a++) {
-                int b = (a + 1) % 3, c = (a + 2) % 3;  // (G x J)_a = G_b J_c - G_c J_b
-                F hr = (G[b][0] * jr[c] - G[b][1] * ji[c]) - (G[c][0] * jr[b] - G[c][1] * ji[b]);
-                F hi = (G[b][0] * ji[c] + G[b][1] * jr[c]) - (G[c][0] * ji[b] + G[c][1] * jr[b]);
+                const int b = (a + 1) % 3, c = (a + 2) % 3;  // (G x J)_a = G_b J_c - G_c J_b
+                const F hr = (m.g[b][0] * jr[c] - m.g[b][1] * ji[c]) - (m.g[c][0] * jr[b] - m.g[c][1] * ji[b]);
+                const F hi = (m.g[b][0] * ji[c] + m.g[b][1] * jr[c]) - (m.g[c][0] * ji[b] + m.g[c][1] * jr[b]);
                 acc[rr][6 + 2 * a] += (double)hr;
                 acc[rr][6 + 2 * a + 1] += (double)hi;
             }
@@ -170,27 +184,56 @@ BIELCC_D void contract(const Moments<F>& m, F pr, F pi, const cplx (*sj)[3], boo
 // The far kernel. MIXED = false: FP64 nodes; true: FP32 nodes. MARKS: the
 // convergence-test marks of p_max >= 3 select the integrals this pass adds
 // (FarArgs::markG / markK); the other variants read no marks.
+// Per cell a warp takes the shortest row that its nearest far point allows
+// (rules.cu); lane i loads node i of a chunk of 32 into the warp's buffer, which
+// all lanes then walk (a broadcast load per node). The load is issued before the
+// pair's set-up, so its latency is covered without a second buffer (a pipelined
+// cp.async pair of buffers cost 100 instructions per cell and was slower).
+// Bound: issue slots. 8192 cells x 20,000 points, mixed, whole call: 26.0 ms with
+// all 64 nodes -> 8.3 with the rules -> 7.2 with the total-degree rules and a
+// shorter set-up (near test on the squared distance, e^{ik r0} in turns, phase
+// applied to J instead of the moments); ncu on 8000 points: 1114 warp instructions
+// per (warp, cell) before that last step, 76 % issue-active, FMA pipe 49 %. FP64,
+// 5120 triangles x 6001 points: 11.9 -> 7.6 ms, FP64 pipe 68 %.
+// ways = 1: a CTA holds 128 points and every warp takes all cells of the split,
+// so that the warps run the same code at about the same time (with each warp at a
+// cell of its own the same sums took 10.2 instead of 8.4 ms: 2.0 instead of 0.1
+// no-instruction stalls per issue). ways = 4: 32 points per CTA, each warp every
+// fourth cell, the warps' sums added in warp order: 80 triangles x 100 points in
+// FP64, a whole host call, 1216 -> 240 us.
 template <int NRHS, bool CK, bool MIXED, bool MARKS = false>
-__global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(FarArgsOf<MARKS> a) {
+__global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_constant__ FarArgsOf<MARKS> a) {
     using NodeT = typename std::conditional<MIXED, float4, double4>::type;
-    __shared__ __align__(16) NodeT s_nodes[kStageNodes];
-    __shared__ float s_yy[MIXED ? kStageNodes : 1];  // |y - centre|^2 of the staged nodes (mixed form)
-    __shared__ double4 s_cell[kMaxStageCells];  // centre xyz, near threshold
-    __shared__ cplx s_j[kMaxStageCells][NRHS][3];
-    __shared__ float s_rho[kMaxStageCells];
-    __shared__ double s_rho64[kMaxStageCells];
+    using F = typename std::conditional<MIXED, float, double>::type;
+    constexpr int kWarps = kFarThreads / 32;
+    static_assert(kWarps == kFarWays, "ways = 4 gives every warp its share of the cells");
+    __shared__ __align__(16) RowBuf<NodeT> s_rows[kWarps];
+    __shared__ RuleTab<NodeT> s_tab;
+    __shared__ double4 s_cell[kStageCells];  // centre xyz, near distance
+    __shared__ F s_j[kStageCells][NRHS][6];
+    __shared__ int s_mode[kStageCells];  // mixed: phase polynomial; FP64: Taylor length of the phase split, -1 none
+    __shared__ float s_rmin[kStageCells][kMaxRules];
+    __shared__ unsigned s_near[kWarps][32];
+    __shared__ double s_sum[kWarps][12][32];
 
-    const int p = blockIdx.x * kFarThreads + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool split_cells = a.ways > 1;
+    const int p = split_cells ? blockIdx.x * 32 + lane : blockIdx.x * kFarThreads + threadIdx.x;
     const bool live = p < a.n_pts;
     double x[3] = {0., 0., 0.};
     if (live)
         for (int g = 0; g < 3; g++) x[g] = a.pts[3 * (size_t)p + g];
-    const int cb = blockIdx.y * a.cells_per_split;
+    const int cb = blockIdx.y * a.cells_per_split;  // a stage never crosses a 32-cell mask word
     const int ce = min(a.n_cells, cb + a.cells_per_split);
-    const int nn = a.nn;
-    const int cps = nn <= kStageNodes ? max(1, min(kMaxStageCells, kStageNodes / nn)) : 1;
-    const int kchunk = nn <= kStageNodes ? nn : kStageNodes;
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
+    const double kturn = a.k.re * kInvTwoPi;
+    const int n_lev = a.rules.n_lev;
+    if (threadIdx.x == 0) {
+        const NodeT* full;
+        if constexpr (MIXED) full = a.nodes32;
+        else full = a.nodes64;
+        s_tab.fill(a.rules, rule_rows(a.rules, NodeT()), full, a.nn, a.n_cells);
+    }
 
     double acc[NRHS][12];
 #pragma unroll
@@ -198,176 +241,170 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(FarArgsOf<MARKS> a
 #pragma unroll
         for (int q = 0; q < 12; q++) acc[r][q] = 0.;
 
-    using F = typename std::conditional<MIXED, float, double>::type;
-    Moments<F> m;
-    m.zero();
-    bool far = false, zeroR = false;
-    unsigned takeE = ~0u;  // convergence-test marks (p_max >= 3): the RHS whose E this pass adds
-    bool takeH = true;     // and whether it adds H
-    unsigned nbits = 0;  // near bits of the current 32-cell word
-    // mixed-form per-pair state
-    PairF32 pf{};
     const KF32 kf = KF32::make(a.k.re, a.k.im);
-    double P0r = 1.0, P0i = 0.0, r0d = 0.0;
-    int mode = 0;
-    bool split64 = false;
-    int td64 = 0;  // Taylor length of the FP64 phase split (farnode.cuh sincos_taylor64)
+    // near bits of the stage at c0: a whole word, or the stage's bytes of it when a
+    // split is shorter than a word (the split of the last cell clears the rest)
+    auto write_mask = [&](int c0, unsigned bits) {
+        if (!live || !a.nearmask) return;
+        unsigned* word = a.nearmask + (size_t)(c0 >> 5) * a.n_pts + p;
+        if (a.cells_per_split >= 32) {
+            *word = bits;
+        } else {
+            const int b0 = (c0 & 31) >> 3, b1 = ce == a.n_cells ? 4 : ((c0 & 31) + a.cells_per_split) >> 3;
+            for (int b = b0; b < b1; b++) reinterpret_cast<unsigned char*>(word)[b] = (bits >> (8 * b)) & 0xffu;
+        }
+    };
 
-    for (int c0 = cb; c0 < ce; c0 += cps) {
-        const int nc = min(cps, ce - c0);
-        for (int k0 = 0; k0 < nn; k0 += kchunk) {
-            const int kc = min(kchunk, nn - k0);
-            __syncthreads();
-            // stage nodes (contiguous when kc == nn) with 128-bit loads
-            {
-                const int tot = nc * kc;
-                if constexpr (MIXED) {
-                    const float4* src = a.nodes32 + (size_t)c0 * nn + k0;
-                    for (int i = threadIdx.x; i < tot; i += kFarThreads) {
-                        int cc = i / kc, kk = i - cc * kc;
-                        const float4 v = __ldg(src + (size_t)cc * nn + kk);
-                        s_nodes[i] = v;
-                        s_yy[i] = node_yy(v);
-                    }
-                } else {
-                    const double2* src = reinterpret_cast<const double2*>(a.nodes64 + (size_t)c0 * nn + k0);
-                    double2* dst = reinterpret_cast<double2*>(s_nodes);
-                    for (int i = threadIdx.x; i < 2 * tot; i += kFarThreads) {
-                        int node = i >> 1, cc = node / kc, kk = node - cc * kc;
-                        dst[i] = __ldg(src + 2 * ((size_t)cc * nn + kk) + (i & 1));
-                    }
-                }
-            }
-            if (k0 == 0) {
-                for (int i = threadIdx.x; i < nc; i += kFarThreads) {
-                    const CellGeo& gg = a.geo[c0 + i];
-                    s_cell[i] = make_double4(gg.c[0], gg.c[1], gg.c[2], gg.diam);
-                    if (MIXED) s_rho[i] = a.rho32[c0 + i];
-                    else s_rho64[i] = (double)a.rho32[c0 + i] * (1.0 + 1e-6);
-                }
-                for (int i = threadIdx.x; i < nc * NRHS * 3; i += kFarThreads) {
-                    int cc = i / (NRHS * 3), rem = i - cc * NRHS * 3, rr = rem / 3, g = rem - rr * 3;
-                    int rhs = min(a.rhs0 + rr, a.n_rhs - 1);
-                    s_j[cc][rr][g] = a.J[((size_t)rhs * a.n_cells + (c0 + cc)) * 3 + g];
-                }
-            }
-            __syncthreads();
-            for (int cc = 0; cc < nc; cc++) {
-                if (k0 == 0) {
-                    double4 ci = s_cell[cc];
-                    double cen[3] = {ci.x, ci.y, ci.z}, d;
-                    const bool nr = is_near(x, cen, ci.w, a.analytic_calc, &d);
-                    far = !nr && live;
-                    if constexpr (MARKS) {
-                      if (far) {  // each integral's convergence test decides which pass adds it
-                        const int c = c0 + cc, nw = (a.n_cells + 31) >> 5;
-                        const size_t wi = (size_t)(c >> 5) * a.n_pts + p;
-                        const bool want = a.take_marked != 0;
-                        takeH = (((a.markG[wi] >> (c & 31)) & 1u) != 0) == want;
-                        takeE = 0u;
-                        for (int rr = 0; rr < NRHS && a.rhs0 + rr < a.n_rhs; rr++) {
-                            const unsigned mk = a.markK[(size_t)(a.rhs0 + rr) * nw * a.n_pts + wi];
-                            if ((((mk >> (c & 31)) & 1u) != 0) == want) takeE |= 1u << rr;
-                        }
-                        far = takeE != 0u || takeH;
-                      }
-                    }
-                    zeroR = d < kMachineZero;  // R_Rot_Colloc: R = 0 at the cell centre
-                    m.zero();
-                    const int c = c0 + cc;
-                    nbits |= (nr ? 1u : 0u) << (c & 31);
-                    if ((c & 31) == 31 || c == ce - 1) {
-                        if (live && a.nearmask) a.nearmask[(size_t)(c >> 5) * a.n_pts + p] = nbits;
-                        nbits = 0;
-                    }
-                    if (!MIXED && far) {  // FP64 phase split when the cell's phase range is small
-                        const double th64 = fabs(a.k.re) * s_rho64[cc];
-                        split64 = !CK && th64 <= 0.5;
-                        td64 = th64 <= 0.125 ? 2 : (th64 <= 0.25 ? 1 : 0);
-                        r0d = d;
-                        if (split64) {
-                            double sn, cs;
-                            sincos(a.k.re * d, &sn, &cs);
-                            P0r = cs;
-                            P0i = sn;
-                        } else {
-                            P0r = 1.0;
-                            P0i = 0.0;
-                        }
-                    }
-                    if (MIXED && far) {  // per-pair FP64 set-up of the phase split
-                        pf.set(x, cen, d, kf);
-                        double s, c;
-                        sincos(a.k.re * d, &s, &c);
-                        if (CK) {
-                            double am = exp(-a.k.im * d);
-                            s *= am;
-                            c *= am;
-                        }
-                        P0r = c;
-                        P0i = s;
-                        mode = phase_mode((float)fabs(a.k.re) * s_rho[cc]);
-                    }
-                }
-                if (far) {
-                    const NodeT* nd = s_nodes + cc * kc;
-                    if constexpr (MIXED) {
-                        const float* yy = s_yy + cc * kc;
-#define BIELCC_NODE_LOOP(MODE_)                                                                        \
-    BIELCC_FAR_UNROLL_PRAGMA for (int i = 0; i < kc; i++) far_node_f32<CK, MODE_>(m, pf, nd[i], yy[i], kf);
-                        switch (mode) {
-                            case 0: BIELCC_NODE_LOOP(0) break;
-                            case 1: BIELCC_NODE_LOOP(1) break;
-                            case 2: BIELCC_NODE_LOOP(2) break;
-                            case 3: BIELCC_NODE_LOOP(3) break;
-                            default: BIELCC_NODE_LOOP(4) break;
-                        }
-#undef BIELCC_NODE_LOOP
-                    } else {
-                        if (split64) {
-#define BIELCC_NODE64_LOOP(TD_)                                                                       \
-    BIELCC_FAR64_UNROLL_PRAGMA for (int i = 0; i < kc; i++) {                                          \
-        const double4 v = nd[i];                                                                       \
-        far_node_f64<CK, true, TD_>(m, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, a.k, k2r, k2i, r0d); \
-    }
-                            switch (td64) {
-                                case 2: BIELCC_NODE64_LOOP(2) break;
-                                case 1: BIELCC_NODE64_LOOP(1) break;
-                                default: BIELCC_NODE64_LOOP(0) break;
-                            }
-#undef BIELCC_NODE64_LOOP
-                        } else {
-#pragma unroll 2
-                            for (int i = 0; i < kc; i++) {
-                                double4 v = nd[i];
-                                far_node_f64<CK, false>(m, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, a.k, k2r, k2i,
-                                                        r0d);
-                            }
-                        }
-                    }
-                }
-                if (k0 + kc == nn && far) {
-                    if (!CK) m.finish_real_k();
-                    if constexpr (MARKS) {
-                        if constexpr (MIXED)
-                            contract<NRHS, float>(m, (float)P0r, (float)P0i, s_j[cc], zeroR, acc, takeE, takeH);
-                        else contract<NRHS, double>(m, P0r, P0i, s_j[cc], zeroR, acc, takeE, takeH);
-                    } else {
-                        if constexpr (MIXED) contract<NRHS, float>(m, (float)P0r, (float)P0i, s_j[cc], zeroR, acc);
-                        else contract<NRHS, double>(m, P0r, P0i, s_j[cc], zeroR, acc);
-                    }
-                }
+    for (int c0 = cb; c0 < ce; c0 += kStageCells) {
+        const int nc = min(kStageCells, ce - c0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < nc; i += kFarThreads) {
+            s_cell[i] = near_cell(a.geo[c0 + i], a.analytic_calc);
+            if constexpr (MIXED) {
+                s_mode[i] = phase_mode((float)fabs(a.k.re) * a.rho32[c0 + i]);
+            } else {  // FP64 phase split when the cell's phase range is small (farnode.cuh sincos_taylor64)
+                const double th = fabs(a.k.re) * (double)a.rho32[c0 + i] * (1.0 + 1e-6);
+                s_mode[i] = CK || !(th <= 0.5) ? -1 : (th <= 0.125 ? 2 : (th <= 0.25 ? 1 : 0));
             }
         }
+        {
+            const float kabs = rule_kabs(a.k);
+            const float2* lim = rule_limits(a.rules, NodeT()) + (size_t)c0 * n_lev;
+            for (int i = threadIdx.x; i < nc * n_lev; i += kFarThreads)
+                s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], kabs);
+        }
+        for (int i = threadIdx.x; i < nc * NRHS * 6; i += kFarThreads) {
+            const int cc = i / (NRHS * 6), rem = i - cc * NRHS * 6, rr = rem / 6, g = rem - rr * 6;
+            const int rhs = min(a.rhs0 + rr, a.n_rhs - 1);
+            s_j[cc][rr][g] = (F)reinterpret_cast<const double*>(a.J)[((size_t)rhs * a.n_cells + (c0 + cc)) * 6 + g];
+        }
+        __syncthreads();
+        unsigned nbits = 0;  // near bits of this warp's cells
+        for (int cc = split_cells ? warp : 0; cc < nc; cc += a.ways) {
+            double dx[3], s2;
+            const bool nr = near_exact(x, s_cell[cc], dx, &s2);
+            bool far = !nr && live;
+            nbits |= (nr ? 1u : 0u) << ((c0 + cc) & 31);
+            unsigned takeE = ~0u;  // convergence-test marks (p_max >= 3): the RHS whose E this pass adds
+            bool takeH = true;     // and whether it adds H
+            if constexpr (MARKS) {
+                if (far) {  // each integral's convergence test decides which pass adds it
+                    const int c = c0 + cc, nw = (a.n_cells + 31) >> 5;
+                    const size_t wi = (size_t)(c >> 5) * a.n_pts + p;
+                    const bool want = a.take_marked != 0;
+                    takeH = (((a.markG[wi] >> (c & 31)) & 1u) != 0) == want;
+                    takeE = 0u;
+                    for (int rr = 0; rr < NRHS && a.rhs0 + rr < a.n_rhs; rr++) {
+                        const unsigned mk = a.markK[(size_t)(a.rhs0 + rr) * nw * a.n_pts + wi];
+                        if ((((mk >> (c & 31)) & 1u) != 0) == want) takeE |= 1u << rr;
+                    }
+                    far = takeE != 0u || takeH;
+                }
+            }
+            const double d = dist_from_sq<!MIXED>(s2);
+            const float dmin = warp_min_pos(rule_key(far, d));
+            if (!(dmin < __int_as_float(0x7f800000))) continue;  // no lane takes part
+            const int lev = rule_level(s_rmin[cc], n_lev, dmin);
+            const int cnt = s_tab.cnt[lev];
+            const NodeT* row = s_tab.base[lev] + (size_t)(c0 + cc) * cnt;
+            NodeT v{};
+            if (lane < cnt) v = row[lane];  // on its way during the pair's set-up
+            Moments<F> m;
+            m.zero();
+            PairF32 pf{};
+            F P0r = 1, P0i = 0;
+            const int mode = s_mode[cc];
+            if constexpr (MIXED) {  // the phase taken out of the nodes: e^{ik r0}
+                pf.set(dx, s2, d, kf);
+                turn_f32(d * kturn, CK ? exp(-a.k.im * d) : 1.0, &P0r, &P0i);
+            } else if (mode >= 0) {
+                sincos(a.k.re * d, &P0i, &P0r);
+            }
+            for (int k0 = 0; k0 < cnt; k0 += kRowChunk) {
+                const int kc = min(kRowChunk, cnt - k0);
+                RowBuf<NodeT>& rb = s_rows[warp];
+                if (k0 && lane < kc) v = row[k0 + lane];
+                __syncwarp();  // the previous chunk has been read
+                rb.nd[lane] = v;
+                if constexpr (MIXED) rb.yy[lane] = node_yy(v);
+                __syncwarp();
+                if (!far) continue;
+                if constexpr (MIXED) {
+#define BIELCC_NODE_LOOP(MODE_)                                           \
+    BIELCC_FAR_UNROLL_PRAGMA for (int i = 0; i < kc; i++)                 \
+        far_node_f32<CK, MODE_>(m, pf, rb.nd[i], rb.yy[i], kf);
+                    switch (mode) {
+                        case 0: BIELCC_NODE_LOOP(0) break;
+                        case 1: BIELCC_NODE_LOOP(1) break;
+                        case 2: BIELCC_NODE_LOOP(2) break;
+                        case 3: BIELCC_NODE_LOOP(3) break;
+                        default: BIELCC_NODE_LOOP(4) break;
+                    }
+#undef BIELCC_NODE_LOOP
+                } else if (mode >= 0) {
+#define BIELCC_NODE64_LOOP(TD_)                                                                         \
+    BIELCC_FAR64_UNROLL_PRAGMA for (int i = 0; i < kc; i++) {                                            \
+        const double4 y = rb.nd[i];                                                                      \
+        far_node_f64<CK, true, TD_>(m, x[0] - y.x, x[1] - y.y, x[2] - y.z, y.w, a.k, k2r, k2i, d);       \
     }
-    if (!live) return;
+                    switch (mode) {
+                        case 2: BIELCC_NODE64_LOOP(2) break;
+                        case 1: BIELCC_NODE64_LOOP(1) break;
+                        default: BIELCC_NODE64_LOOP(0) break;
+                    }
+#undef BIELCC_NODE64_LOOP
+                } else {
+#pragma unroll 2
+                    for (int i = 0; i < kc; i++) {
+                        const double4 y = rb.nd[i];
+                        far_node_f64<CK, false>(m, x[0] - y.x, x[1] - y.y, x[2] - y.z, y.w, a.k, k2r, k2i, d);
+                    }
+                }
+            }
+            if (far) {
+                const bool zeroR = d < kMachineZero;  // R_Rot_Colloc: R = 0 at the cell centre
+                contract<NRHS, CK, F>(m, P0r, P0i, s_j[cc], zeroR, acc, takeE, takeH);
+            }
+        }
+        if (split_cells) {
+            s_near[warp][lane] = nbits;
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll
+                for (int w = 1; w < kWarps; w++) nbits |= s_near[w][lane];
+                write_mask(c0, nbits);
+            }
+        } else {
+            write_mask(c0, nbits);
+        }
+    }
     const size_t P = a.n_pts;
 #pragma unroll
     for (int r = 0; r < NRHS; r++) {
         if (a.rhs0 + r >= a.n_rhs) break;
         double* dst = a.partial + (((size_t)blockIdx.y * a.n_rhs + (a.rhs0 + r)) * 12) * P + p;
+        if (!split_cells) {
+            if (live) {
 #pragma unroll
-        for (int q = 0; q < 12; q++) dst[(size_t)q * P] = acc[r][q];
+                for (int q = 0; q < 12; q++) dst[(size_t)q * P] = acc[r][q];
+            }
+            continue;
+        }
+        // the warps' sums in warp order: warp w adds components 3 w .. 3 w + 2
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 12; q++) s_sum[warp][q][lane] = acc[r][q];
+        __syncthreads();
+        if (live) {
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const int q = 3 * warp + j;
+                double v = s_sum[0][q][lane];
+#pragma unroll
+                for (int w = 1; w < kWarps; w++) v += s_sum[w][q][lane];
+                dst[(size_t)q * P] = v;
+            }
+        }
     }
 }
 
@@ -387,11 +424,10 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(FarArgsOf<MARKS> a
 // far_refine_sum_kernel.
 
 // Unrolling of the decision kernel's node loops (the node rows come from
-// global memory: unrolled, their loads issue ahead of the arithmetic).
-// 2000 x 8192 at p_max = 3, mixed / FP64: x1 ~92 / 131 ms, x4 88.3 / 129.3 ms,
-// x8 88.4 / 127.9 ms.
+// global memory: unrolled, their loads issue ahead of the arithmetic). 3200 cells
+// x 1000 points at p_max = 3, FP64, whole call: x1 13.7, x3 11.3, x5 12.2 ms.
 #ifndef BIELCC_DECIDE_UNROLL
-#define BIELCC_DECIDE_UNROLL 8
+#define BIELCC_DECIDE_UNROLL 3
 #endif
 
 // One pass of the FP64 far node loop over a cell's node table row (far_kernel's
@@ -403,7 +439,7 @@ BIELCC_D void far_pass_f64(Moments<double>& m, const double4* __restrict__ nd, i
     if (split) {
 #define BIELCC_PASS64(TD_)                                                                              \
     BIELCC_FAR_PRAGMA(BIELCC_DECIDE_UNROLL) for (int i = 0; i < nn; i++) {                              \
-        const double4 v = nd[i];                                                                \
+        const double4 v = ldg_node(nd + i);                                                             \
         far_node_f64<CK, true, TD_>(m, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, k, k2r, k2i, r0);       \
     }
         switch (td) {
@@ -414,7 +450,7 @@ BIELCC_D void far_pass_f64(Moments<double>& m, const double4* __restrict__ nd, i
 #undef BIELCC_PASS64
     } else {
         BIELCC_FAR_PRAGMA(BIELCC_DECIDE_UNROLL) for (int i = 0; i < nn; i++) {
-            const double4 v = nd[i];
+            const double4 v = ldg_node(nd + i);
             far_node_f64<CK, false>(m, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, k, k2r, k2i, r0);
         }
     }
@@ -444,44 +480,52 @@ BIELCC_D double far_delta2(const cplx* a, const cplx* b) {
 }
 
 // markK and this split's slot of a.partial must be zero on entry (set bits
-// only; the passing integrals are added); markG is written in full.
-// STAGED: the CTA stages each cell's two node rows in shared memory
-// ((nn_lo + nn) double4, dynamic) before its threads use them; otherwise every
-// thread reads them from global memory (rows too long to stage).
-template <bool STAGED>
-__global__ void far_refine_decide_kernel(FarArgs a, const double4* __restrict__ lo, int nn_lo, double eps2,
+// only; the passing integrals are added); markG is written in full. Each pass
+// takes the shortest row its table's rules allow (rules.cu, FP64 limits).
+__global__ void far_refine_decide_kernel(const __grid_constant__ FarArgs a, const __grid_constant__ FarRules rules_lo,
+                                         const double4* __restrict__ lo, int nn_lo, double eps2,
                                          unsigned* __restrict__ markG, unsigned* __restrict__ markK) {
-    extern __shared__ double4 s_rows[];  // STAGED: [nn_lo] then [nn] of the current cell
+    __shared__ RuleTab<double4> s_lo, s_hi;
+    __shared__ float s_rmin[2][kStageCells][kMaxRules];
     const int p = blockIdx.x * kFarThreads + threadIdx.x;
     const bool live = p < a.n_pts;
-    if (!STAGED && !live) return;
     double x[3] = {0., 0., 0.};
     if (live)
         for (int g = 0; g < 3; g++) x[g] = a.pts[3 * (size_t)p + g];
-    const int cb = blockIdx.y * a.cells_per_split;
+    const int cb = blockIdx.y * a.cells_per_split;  // a multiple of 32
     const int ce = min(a.n_cells, cb + a.cells_per_split);
     const bool ck = a.k.im != 0.0;
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
     const int nw = (a.n_cells + 31) >> 5;
     const size_t P = a.n_pts;
+    const int nlo = rules_lo.n_lev, nhi = a.rules.n_lev;
+    if (threadIdx.x == 0) {
+        s_lo.fill(rules_lo, rules_lo.n64, lo, nn_lo, a.n_cells);
+        s_hi.fill(a.rules, a.rules.n64, a.nodes64, a.nn, a.n_cells);
+    }
     unsigned nbits = 0, gbits = 0;
     for (int c = cb; c < ce; c++) {
-        const double4* row_lo = lo + (size_t)c * nn_lo;
-        const double4* row_hi = a.nodes64 + (size_t)c * a.nn;
-        if constexpr (STAGED) {
-            __syncthreads();  // the previous cell's rows are no longer read
-            for (int i = threadIdx.x; i < nn_lo; i += kFarThreads) s_rows[i] = row_lo[i];
-            for (int i = threadIdx.x; i < a.nn; i += kFarThreads) s_rows[nn_lo + i] = row_hi[i];
+        if ((c & 31) == 0) {
+            const int nc = min(kStageCells, ce - c);
+            const float kabs = rule_kabs(a.k);
+            __syncthreads();  // the previous cells' limits are no longer read
+            for (int i = threadIdx.x; i < nc * nlo; i += kFarThreads)
+                s_rmin[0][i / nlo][i % nlo] = rule_rmin(rules_lo.thr64[(size_t)c * nlo + i], kabs);
+            for (int i = threadIdx.x; i < nc * nhi; i += kFarThreads)
+                s_rmin[1][i / nhi][i % nhi] = rule_rmin(a.rules.thr64[(size_t)c * nhi + i], kabs);
             __syncthreads();
-            row_lo = s_rows;
-            row_hi = s_rows + nn_lo;
-            if (!live) continue;  // after the barriers: every thread stages
         }
         const CellGeo& gg = a.geo[c];
         double d;
         const bool nr = is_near(x, gg.c, gg.diam, a.analytic_calc, &d);
         bool gfail = false;
-        if (!nr) {
+        const bool far = !nr && live;
+        const float dmin = warp_min_pos(rule_key(far, d));
+        const int llo = rule_level(s_rmin[0][c & 31], nlo, dmin), lhi = rule_level(s_rmin[1][c & 31], nhi, dmin);
+        if (far) {
+            const int n_lo = s_lo.cnt[llo], n_hi = s_hi.cnt[lhi];
+            const double4* row_lo = s_lo.base[llo] + (size_t)c * n_lo;
+            const double4* row_hi = s_hi.base[lhi] + (size_t)c * n_hi;
             const double th64 = fabs(a.k.re) * (double)a.rho32[c] * (1.0 + 1e-6);
             const bool split = !ck && th64 <= 0.5;
             const int td = th64 <= 0.125 ? 2 : (th64 <= 0.25 ? 1 : 0);
@@ -489,11 +533,11 @@ __global__ void far_refine_decide_kernel(FarArgs a, const double4* __restrict__ 
             if (split) sincos(a.k.re * d, &pi, &pr);
             Moments<double> m0, m1;
             if (ck) {
-                far_pass_f64<true>(m0, row_lo, nn_lo, x, a.k, k2r, k2i, d, false, 0);
-                far_pass_f64<true>(m1, row_hi, a.nn, x, a.k, k2r, k2i, d, false, 0);
+                far_pass_f64<true>(m0, row_lo, n_lo, x, a.k, k2r, k2i, d, false, 0);
+                far_pass_f64<true>(m1, row_hi, n_hi, x, a.k, k2r, k2i, d, false, 0);
             } else {
-                far_pass_f64<false>(m0, row_lo, nn_lo, x, a.k, k2r, k2i, d, split, td);
-                far_pass_f64<false>(m1, row_hi, a.nn, x, a.k, k2r, k2i, d, split, td);
+                far_pass_f64<false>(m0, row_lo, n_lo, x, a.k, k2r, k2i, d, split, td);
+                far_pass_f64<false>(m1, row_hi, n_hi, x, a.k, k2r, k2i, d, split, td);
             }
             const bool zeroR = d < kMachineZero;  // R_Rot_Colloc integrates grad F away from the centre only
             cplx g1[3];
@@ -533,8 +577,10 @@ __global__ void far_refine_decide_kernel(FarArgs a, const double4* __restrict__ 
         nbits |= (nr ? 1u : 0u) << (c & 31);
         gbits |= (gfail ? 1u : 0u) << (c & 31);
         if ((c & 31) == 31 || c == ce - 1) {
-            if (a.nearmask) a.nearmask[(size_t)(c >> 5) * a.n_pts + p] = nbits;
-            markG[(size_t)(c >> 5) * a.n_pts + p] = gbits;
+            if (live) {
+                if (a.nearmask) a.nearmask[(size_t)(c >> 5) * a.n_pts + p] = nbits;
+                markG[(size_t)(c >> 5) * a.n_pts + p] = gbits;
+            }
             nbits = gbits = 0;
         }
     }
@@ -873,14 +919,43 @@ static int far_slots(int n_rhs, bool ck, bool mixed) {
     return v;
 }
 
+// Cells per split of the far kernel: whole 32-cell mask words, or 16 or 8 cells
+// (bytes of a word) when the splits outnumber the words.
+static int far_cells_per_split(int n_cells, int splits) {
+    if (splits > (n_cells + 31) / 32) return (n_cells + 15) / 16 == splits ? 16 : 8;
+    return round_cells_per_split(n_cells, splits);
+}
+
+// The far kernel's grid. 128-point tiles with whole-warp cell sweeps when they
+// fill the GPU at one mask word (32 cells) per split, the finest a sweep can be
+// cut; below that a resident CTA slot would stay empty, so 32-point tiles whose
+// warps share the cells, and if that is still short 16 or 8 cells per split (the
+// decision kernel of p_max >= 3 keeps whole words).
+struct FarGrid {
+    int tiles, splits, ways;
+};
+static FarGrid far_grid(const FieldLaunch& f, int max_splits) {
+    const int N = f.mesh->n_cells, slots = far_slots(f.n_rhs, f.k.im != 0.0, f.precision == 1);
+    FarGrid g;
+    g.tiles = (f.n_pts + kFarThreads - 1) / kFarThreads;
+    g.ways = (size_t)g.tiles * std::min((N + 31) / 32, max_splits) < (size_t)slots ? kFarWays : 1;
+    if (g.ways > 1) g.tiles = (f.n_pts + 31) / 32;
+    g.splits = choose_cell_splits(g.tiles, N, slots, max_splits);
+    if (g.ways > 1 && !far_adaptive(f.np))
+        for (int cps = 16; cps >= 8 && g.splits >= N / 32 && (size_t)g.tiles * g.splits < (size_t)slots; cps -= 8) {
+            const int fine = (N + cps - 1) / cps;
+            if (fine > max_splits) break;
+            if (fine > (N + 31) / 32) g.splits = fine;
+        }
+    return g;
+}
+
 size_t field_ws_base_bytes(const FieldLaunch& f, int* splits_out, size_t partial_cap) {
-    const int tiles = (f.n_pts + kFarThreads - 1) / kFarThreads;
     const int N = f.mesh->n_cells;
     const size_t P = f.n_pts;
     const size_t per_split = (size_t)f.n_rhs * 12 * P * sizeof(double);
-    const int slots = far_slots(f.n_rhs, f.k.im != 0.0, f.precision == 1);
     const int max_splits = (int)std::max<size_t>(1, partial_cap / std::max<size_t>(1, per_split));
-    int splits = choose_cell_splits(tiles, N, slots, max_splits);
+    int splits = far_grid(f, max_splits).splits;
     if (far_third_pass(f.np)) {
         // p_max = 3: the third pass's work sits on the points whose integrals
         // failed the test (near-field points, a few tiles), so a grid balanced
@@ -954,16 +1029,20 @@ cudaError_t field_stage1(const FieldLaunch& f, void* ws, int splits, long long* 
     a.nodes64 = m.nodes64;
     a.nodes32 = m.nodes32;
     a.rho32 = m.rho32;
+    a.rules = m.rules;
     a.nn = far_split_n(f.np) * far_split_n(f.np);
     a.J = reinterpret_cast<const cplx*>(f.J);
     a.n_rhs = f.n_rhs;
     a.rhs0 = 0;
     a.k = f.k;
     a.analytic_calc = f.np.analytic_calc;
-    a.cells_per_split = round_cells_per_split(m.n_cells, splits);
+    a.cells_per_split = far_cells_per_split(m.n_cells, splits);
     a.partial = partial;
     a.nearmask = mask;
-    int tiles = (f.n_pts + kFarThreads - 1) / kFarThreads;
+    const int tiles128 = (f.n_pts + kFarThreads - 1) / kFarThreads;  // one point per thread
+    // the split count is the caller's; fewer 128-point CTAs than slots: shared cells
+    a.ways = (size_t)tiles128 * std::min(n_words, splits) < (size_t)far_slots(f.n_rhs, f.k.im != 0.0, f.precision == 1) ? kFarWays : 1;
+    const int tiles = a.ways > 1 ? (f.n_pts + 31) / 32 : tiles128;
     bool ck = f.k.im != 0.0;
     bool mixed = f.precision == 1;
     int nl = 0;
@@ -981,13 +1060,8 @@ cudaError_t field_stage1(const FieldLaunch& f, void* ws, int splits, long long* 
         if (e == cudaSuccess) e = cudaMemsetAsync(partial, 0, (size_t)splits * f.n_rhs * 12 * P * sizeof(double), s);
         if (e != cudaSuccess) return e;
         const int nn_lo = f.np.n_start * f.np.n_start;
-        const size_t rows = (size_t)(nn_lo + a.nn) * sizeof(double4);
-        if (rows <= 48 * 1024)
-            far_refine_decide_kernel<true><<<dim3(tiles, splits), kFarThreads, rows, s>>>(
-                a, m.nodes64_lo, nn_lo, f.np.eps * f.np.eps, markG, markK);
-        else
-            far_refine_decide_kernel<false><<<dim3(tiles, splits), kFarThreads, 0, s>>>(
-                a, m.nodes64_lo, nn_lo, f.np.eps * f.np.eps, markG, markK);
+        far_refine_decide_kernel<<<dim3(tiles128, splits), kFarThreads, 0, s>>>(
+            a, m.rules_lo, m.nodes64_lo, nn_lo, f.np.eps * f.np.eps, markG, markK);
         nl++;
     }
     FarArgsMarks am;
@@ -1005,6 +1079,7 @@ cudaError_t field_stage1(const FieldLaunch& f, void* ws, int splits, long long* 
         a3.nodes64 = m.nodes64_hi;
         a3.nodes32 = m.nodes32_hi;
         a3.rho32 = m.rho32_hi;
+        a3.rules = m.rules_hi;
         a3.nn = 16 * f.np.n_start * f.np.n_start;
         a3.partial = partial + (size_t)splits * f.n_rhs * 12 * P;
         a3.take_marked = 1;
@@ -1018,7 +1093,7 @@ cudaError_t field_stage1(const FieldLaunch& f, void* ws, int splits, long long* 
         nl++;
     }
     if (far_end) cudaEventRecord(far_end, s);
-    if (tiles > 0) near_count_kernel<<<tiles, kFarThreads, 0, s>>>(mask, n_words, f.n_pts, counts);
+    if (tiles > 0) near_count_kernel<<<tiles128, kFarThreads, 0, s>>>(mask, n_words, f.n_pts, counts);
     *far_launches = nl;
     *launches = nl + (tiles > 0 ? 1 : 0) + 1;
     scan_kernel<<<1, 1024, 0, s>>>(counts, f.n_pts, offs, d_total);

@@ -40,6 +40,22 @@ inline bool far_adaptive(const NumParamH& np) { return np.p_max > 2; }
 // with no further test, so they too run the table-driven far kernels.
 inline bool far_third_pass(const NumParamH& np) { return np.p_max == 3; }
 
+// Compressed rules of one node table (rules.cu): levels of increasing length;
+// cell c's row of level l is cnt[l] nodes at off[l] * n_cells + c * cnt[l]. A
+// row may stand in for the n^2-node row at distance r0 and wave number k when
+// r0 >= thr.x and |k| <= thr.y of (cell, level): thr32 for FP32 sums, thr64 for
+// FP64 ones, [N][n_lev] each. n_lev = 0: no rules, the full rows are used.
+constexpr int kMaxRules = 8;
+struct FarRules {
+    int n_lev = 0;
+    int cnt[kMaxRules] = {0};
+    int off[kMaxRules] = {0};
+    const double4* n64 = nullptr;  // (y, weight)
+    const float4* n32 = nullptr;   // (y - centre, weight)
+    const float2* thr32 = nullptr;
+    const float2* thr64 = nullptr;
+};
+
 // Device-resident mesh with its per-cell geometry and cached node tables.
 struct MeshDev {
     int nv = 0, n_cells = 0;
@@ -60,6 +76,11 @@ struct MeshDev {
     double4* nodes64_hi = nullptr;
     float4* nodes32_hi = nullptr;
     float* rho32_hi = nullptr;
+    // compressed rules of the three tables, each in one allocation (null: none)
+    FarRules rules, rules_lo, rules_hi;
+    void* rules_mem = nullptr;
+    void* rules_lo_mem = nullptr;
+    void* rules_hi_mem = nullptr;
     size_t bytes = 0;
 };
 
@@ -73,6 +94,12 @@ int server_device(::bielcc_ctx_s* ctx);
 cudaError_t launch_cell_geometry(const double* verts, int nv, int n_cells, CellGeo* geo, cudaStream_t s);
 cudaError_t launch_node_tables(const double* verts, const CellGeo* geo, int nv, int n_cells, int n, double4* nodes64,
                                float4* nodes32, float* rho32, cudaStream_t s);
+
+// ---- rules.cu: device bytes of the rules of an n-split table (0: none) and
+// their construction in `mem` (rho32: the table's node radii)
+size_t rules_bytes(int nv, int n, int n_cells);
+cudaError_t launch_rules(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
+                         void* mem, FarRules* out, cudaStream_t s);
 
 // ---- field.cu
 struct FieldLaunch {
@@ -185,6 +212,7 @@ struct JobDev {
     const float4* nodes32;
     const double4* nodes64;
     const float* rho32;
+    FarRules rules;
     const double* verts;
     int nv, n_cells;
     const double* pts;

@@ -1,0 +1,107 @@
+"""Compressed rules of the far pass (csrc/rules.cu): the field from the shortest
+rule that a distance, cell and k allow equals the oracle's full n x n sum, over
+the splits where levels appear, and on cells where the Jacobian is no polynomial
+(twisted, reversed corner), vanishes (collapsed edge) or is strongly graded.
+
+Tolerances: a pair's truncation is at most 3e-17 (FP64) / 4e-9 (mixed) of
+sum w |F|; what remains is rounding, an ulp or so per operation: 1e-14 for
+the few cells summed here in FP64, plus the rounding of the phase, k r ulps on
+either side, and 1.5e-7 rms per pair in FP32."""
+import numpy as np
+import pytest
+
+import oracle
+from bielcc_b200 import abi
+from bielcc_b200 import workloads as W
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+TOL = {"fp64": 2e-14, "mixed": 5e-7}
+R_MAX = 100.0  # largest distance of _points
+
+QUADS = np.array([
+    [[0, 0, 0], [1, 0, 0], [1, 1, 0], [0, 1, 0]],                        # square
+    [[0, 0, 0], [3, 0, 0], [3, 1, 0], [0, 1, 0]],                        # rectangle
+    [[-1.1, -1, 0], [1.1, -1, 0], [0.9, 1, 0], [-0.9, 1, 0]],            # trapezoid
+    [[0, 0, 0], [1, 0, 0], [0.5, 2, 0], [0.5, 2, 0]],                    # collapsed edge
+    [[0, 0, 0], [1, 0, 0.2], [1.2, 1, -0.1], [0, 1, 0.15]],              # twisted
+    [[0, 0, 0], [1, 0, 0], [0.35, 0.35, 0.05], [0, 1, 0]],               # reversed corner
+], dtype=float)
+TRIS = np.array([
+    [[0, 0, 0], [1, 0, 0], [0.5, 0.866, 0]],
+    [[0, 0, 0], [1, 0, 0], [0, 1, 0.3]],
+    [[0, 0, 0], [1, 0, 0], [0.3, 0.03, 0]],                              # needle
+], dtype=float)
+
+
+def _cells(nv):
+    c = QUADS if nv == 4 else TRIS
+    off = 0.4 * np.arange(len(c))[:, None, None] * np.array([1.0, 0.3, 0.5])
+    return np.ascontiguousarray(0.1 * c + off)
+
+
+def _points(m, seed):
+    rng = np.random.default_rng(seed)
+    d = rng.standard_normal((m, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    # from just outside the near zone to a thousand radii, sorted and not
+    r = 0.3 + 1.2 * np.exp(rng.uniform(np.log(0.02), np.log(80.0), size=(m, 1)))
+    p = d * r + np.array([0.9, 0.3, 0.5])
+    return p if seed % 2 else p[np.argsort(r[:, 0])]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nv", [3, 4])
+@pytest.mark.parametrize("n_start,k", [(3, 1.0), (4, 1.0), (5, 2.0 + 0.3j), (7, 3.0), (8, 0.0), (8, 1.0), (8, 7.0),
+                                       (8, 30.0), (8, 4.0 + 0.3j), (10, 3.0), (16, 3.0), (17, 6.0), (20, 20.0)])
+def test_rules_equal_full_sum(gctx, n_start, k, nv, precision):
+    # Im k <= 0.3: e^{-Im k R_MAX} >= 1e-13, so that the FP32 products (>= 1e-3 times
+    # that) stay normal numbers; below 2^-126 the mixed form has no relative accuracy
+    cells = _cells(nv)
+    rng = np.random.default_rng(7)
+    J = rng.standard_normal((1, len(cells), 3)) + 1j * rng.standard_normal((1, len(cells), 3))
+    npm = abi.NumParam.default(n_start=n_start)
+    m = gctx.mesh(cells)
+    for pts in (_points(1, 3), _points(33, 4), _points(160, 5), _points(160, 6)):
+        E, H, rep = gctx.field_EH(m, J, k, pts, numparam=npm, precision=precision)
+        Eo, Ho = oracle.field_EH(cells, J, k, pts, npm)
+        # per point: a distant point's small field must be as good as a near one's
+        for a, b in ((E, Eo), (H, Ho)):
+            err = np.linalg.norm(a - b, axis=-1) / np.linalg.norm(b, axis=-1)
+            assert np.sqrt(np.mean(err ** 2)) < TOL[precision] + 2.0 ** -52 * abs(k) * R_MAX
+    m.close()
+
+
+@pytest.mark.parametrize("n_lat,points", [(2, 1), (3, 31), (4, 32), (6, 33), (5, 129), (24, 40), (24, 700)])
+@pytest.mark.parametrize("precision,tol", [("fp64", 2e-14), ("mixed", 5e-7)])
+def test_grids_of_small_problems(gctx, n_lat, points, precision, tol):
+    """32-point tiles whose warps share the cells, 8- and 16-cell splits that write
+    bytes of a near-mask word, and the first size with whole-warp sweeps."""
+    cells = W.uv_sphere(n_lat, 2 * n_lat)
+    J = W.po_currents(cells, 2.0, directions=2, seed=1)
+    rng = np.random.default_rng(points)
+    pts = np.concatenate([W.shell_points(points, 1.6, 5.0, rng), W.near_points(cells, points // 8, 0.05, 0.3, rng)])
+    m = gctx.mesh(cells)
+    E, H, rep = gctx.field_EH(m, J, 2.0, pts, precision=precision)
+    Eo, Ho = oracle.field_EH(cells, J, 2.0, pts)
+    assert rel_l2(E, Eo) < tol and rel_l2(H, Ho) < tol
+    d = np.linalg.norm(pts[:, None] - W.centres(cells)[None], axis=2)
+    assert rep.n_near_pairs == int((d < 3.0 * W.diameters(cells)[None]).sum())
+    m.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_non_finite_points_reach_the_result(gctx, precision):
+    cells = W.uv_sphere(8, 16)
+    J = W.po_currents(cells, 2.0)
+    pts = W.sphere_points(70, 3.0, 0)
+    pts[5, 1] = np.nan
+    pts[40] = np.inf
+    m = gctx.mesh(cells)
+    E, H, rep = gctx.field_EH(m, J, 2.0, pts, precision=precision, check=False)
+    bad = ~np.isfinite(E[0]).all(axis=1)
+    assert bad[5] and bad[40] and bad.sum() == 2 and rep.n_nonfinite == 2
+    keep = ~bad
+    Eo, _ = oracle.field_EH(cells, J, 2.0, pts[keep])
+    assert rel_l2(E[0][keep], Eo[0]) < (1e-12 if precision == "fp64" else 1e-6)
+    m.close()
