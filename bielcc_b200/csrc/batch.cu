@@ -94,15 +94,13 @@ struct BatchCfg {
     using F = typename std::conditional<MIXED, float, double>::type;
     using NodeT = typename std::conditional<MIXED, float4, double4>::type;
     static constexpr int CH = MIXED ? BIELCC_BATCH_CH32 : 8;            // cells per chunk (n_start <= 8)
-    static constexpr int NODES = MIXED ? 64 * BIELCC_BATCH_CH32 : 512;  // staged nodes
     static constexpr int R = MIXED ? BIELCC_BATCH_R : 2;  // RHS per thread in phase B
     // currents per (cell, RHS, component): FP32 (re, im, im, re) for the packed
     // contraction, FP64 (re, im)
     static constexpr int JW = MIXED ? 4 : 2;
-    static constexpr size_t YY = MIXED ? NODES : 0;  // |y - centre|^2 of the staged nodes (mixed form)
     static constexpr size_t smem_bytes() {
-        return sizeof(NodeT) * NODES + sizeof(float) * YY + sizeof(F) * CH * 20 * kBP + sizeof(F) * JW * CH * kSP * 3 +
-               sizeof(double4) * CH + sizeof(double) * CH + CH * kBP + 64;
+        return sizeof(F) * CH * 20 * kBP + sizeof(F) * JW * CH * kSP * 3 + sizeof(double4) * CH + sizeof(double) * CH +
+               CH * kBP + 64;
     }
 };
 static_assert(kSP % (kBW * BatchCfg<true>::R) == 0, "a phase-B pass covers whole groups of kBW x R RHS");
@@ -222,12 +220,23 @@ BIELCC_D void load_cell_moments(const F* s_mom, int cc, int lane, F (&m)[20]) {
     m[13] += m[1];
 }
 
+// x - centre (FP64), its squared length and length: one (point, cell) pair.
+struct FarDist {
+    double dx[3], s, d;
+    // the near decision of get_field.h:58; cell: near_cell's row
+    template <bool MIXED>
+    BIELCC_D bool near(const double* x, const double4& cell) {
+        const bool n = near_exact(x, cell, dx, &s);
+        d = dist_from_sq<!MIXED>(s);
+        return n;
+    }
+};
+
 // Moments of one cell, real-k form finished, times e^{ik r0} into mom[20];
 // R_Rot_Colloc is 0 at the cell centre.
 template <bool CK, typename F>
-BIELCC_D void store_moments(Moments<F>& m, double P0r, double P0i, double d, F* mom) {
+BIELCC_D void store_moments(Moments<F>& m, F pr, F pi, double d, F* mom) {
     if (!CK) m.finish_real_k();
-    const F pr = (F)P0r, pi = (F)P0i;
     mom[0] = m.a1r * pr - m.a1i * pi;
     mom[1] = m.a1r * pi + m.a1i * pr;
 #pragma unroll
@@ -247,19 +256,10 @@ BIELCC_D void store_moments(Moments<F>& m, double P0r, double P0i, double d, F* 
 // Mixed-form set-up of one (point, cell) pair: FP32 pair state, e^{ik r0} in
 // FP64, and the phase polynomial for the cell's phase range |k| rho.
 template <bool CK>
-BIELCC_D int mixed_pair_setup(const double* x, const double4& ci, double d, double rho, cplx k, const KF32& kf,
-                              PairF32& pf, double& P0r, double& P0i) {
-    const double cen[3] = {ci.x, ci.y, ci.z};
-    pf.set(x, cen, d, kf);
-    double sn, cs;
-    sincos(k.re * d, &sn, &cs);
-    if (CK) {
-        const double am = exp(-k.im * d);
-        sn *= am;
-        cs *= am;
-    }
-    P0r = cs;
-    P0i = sn;
+BIELCC_D int mixed_pair_setup(const FarDist& f, double rho, cplx k, const KF32& kf, PairF32& pf, float& P0r,
+                              float& P0i) {
+    pf.set(f.dx, f.s, f.d, kf);
+    turn_f32(f.d * (k.re * kInvTwoPi), CK ? exp(-k.im * f.d) : 1.0, &P0r, &P0i);
     return phase_mode((float)fabs(k.re) * (float)rho);
 }
 
@@ -267,19 +267,23 @@ BIELCC_D int mixed_pair_setup(const double* x, const double4& ci, double d, doub
 // CK (complex k) is a property of the job, so every item of a job takes the
 // same code path whatever else is in the batch.
 template <bool MIXED, bool CK>
-BIELCC_D void batch_moments(const typename BatchCfg<MIXED>::NodeT* nd, const float* yy, int nn, const double* x,
-                            const double4& ci, double d, double rho, cplx k, double k2r, double k2i,
+BIELCC_D void batch_moments(const typename BatchCfg<MIXED>::NodeT* __restrict__ nd, int nn, const double* x,
+                            const FarDist& fd, double rho, cplx k, double k2r, double k2i,
                             typename BatchCfg<MIXED>::F* mom) {
     using F = typename BatchCfg<MIXED>::F;
-    double P0r = 1.0, P0i = 0.0;
+    const double d = fd.d;
+    F P0r = 1, P0i = 0;
     Moments<F> m;
     m.zero();
     if constexpr (MIXED) {
         const KF32 kf = KF32::make(k.re, k.im);
         PairF32 pf;
-        const int mode = mixed_pair_setup<CK>(x, ci, d, rho, k, kf, pf, P0r, P0i);
-#define BIELCC_BNODE(MODE_) \
-    BIELCC_UNROLL(BIELCC_BATCH_U1) for (int i = 0; i < nn; i++) far_node_f32<CK, MODE_>(m, pf, nd[i], yy[i], kf);
+        const int mode = mixed_pair_setup<CK>(fd, rho, k, kf, pf, P0r, P0i);
+#define BIELCC_BNODE(MODE_)                                      \
+    BIELCC_UNROLL(BIELCC_BATCH_U1) for (int i = 0; i < nn; i++) { \
+        const float4 v = __ldg(nd + i);                           \
+        far_node_f32<CK, MODE_>(m, pf, v, node_yy(v), kf);        \
+    }
         switch (mode) {
             case 0: BIELCC_BNODE(0) break;
             case 1: BIELCC_BNODE(1) break;
@@ -291,19 +295,16 @@ BIELCC_D void batch_moments(const typename BatchCfg<MIXED>::NodeT* nd, const flo
     } else {
         const bool split = !CK && fabs(k.re) * rho * (1.0 + 1e-6) <= 0.5;
         if (split) {
-            double sn, cs;
-            sincos(k.re * d, &sn, &cs);
-            P0r = cs;
-            P0i = sn;
+            sincos(k.re * d, &P0i, &P0r);
             BIELCC_UNROLL(BIELCC_BATCH64_UNROLL)
             for (int i = 0; i < nn; i++) {
-                const double4 v = nd[i];
+                const double4 v = ldg_node(nd + i);
                 far_node_f64<CK, true>(m, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, k, k2r, k2i, d);
             }
         } else {
             BIELCC_UNROLL(BIELCC_BATCH64_UNROLL)
             for (int i = 0; i < nn; i++) {
-                const double4 v = nd[i];
+                const double4 v = ldg_node(nd + i);
                 far_node_f64<CK, false>(m, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, k, k2r, k2i, d);
             }
         }
@@ -311,27 +312,32 @@ BIELCC_D void batch_moments(const typename BatchCfg<MIXED>::NodeT* nd, const flo
     store_moments<CK, F>(m, P0r, P0i, d, mom);
 }
 
-// Phase A of two far pairs of the same point (cells A and B of one job, equal
-// node counts), mixed form: the two node loops are interleaved, so each thread
-// has two independent dependency chains per node. A cell's moments do not
-// depend on the other cell; the phase polynomial is the one for the larger
-// phase range of the two (exact over the smaller range too).
+// Phase A of two far pairs of the same point (cells A and B of one job, rows of
+// the same level), mixed form: the two node loops are interleaved, so each thread
+// has two independent dependency chains per node; the next pair of nodes is
+// loaded while the current one is evaluated. The phase polynomial is the one for
+// the larger phase range of the two (exact over the smaller range too).
 template <bool CK>
-BIELCC_D void batch_moments2(const float4* ndA, const float* yyA, const float4* ndB, const float* yyB, int nn,
-                             const double* x, const double4& ciA, double dA, double rhoA, const double4& ciB,
-                             double dB, double rhoB, cplx k, float* momA, float* momB) {
+BIELCC_D void batch_moments2(const float4* __restrict__ ndA, const float4* __restrict__ ndB, int nn,
+                             const FarDist& fA, double rhoA, const FarDist& fB, double rhoB, cplx k, float* momA,
+                             float* momB) {
     const KF32 kf = KF32::make(k.re, k.im);
     PairF32 pa, pb;
-    double PAr, PAi, PBr, PBi;
-    const int mode = max(mixed_pair_setup<CK>(x, ciA, dA, rhoA, k, kf, pa, PAr, PAi),
-                         mixed_pair_setup<CK>(x, ciB, dB, rhoB, k, kf, pb, PBr, PBi));
+    float PAr, PAi, PBr, PBi;
+    const int mode = max(mixed_pair_setup<CK>(fA, rhoA, k, kf, pa, PAr, PAi),
+                         mixed_pair_setup<CK>(fB, rhoB, k, kf, pb, PBr, PBi));
     Moments<float> ma, mb;
     ma.zero();
     mb.zero();
-#define BIELCC_BNODE2(MODE_)                                 \
+    float4 va = __ldg(ndA), vb = __ldg(ndB);
+#define BIELCC_BNODE2(MODE_)                                      \
     BIELCC_UNROLL(BIELCC_BATCH_U2) for (int i = 0; i < nn; i++) { \
-        far_node_f32<CK, MODE_>(ma, pa, ndA[i], yyA[i], kf); \
-        far_node_f32<CK, MODE_>(mb, pb, ndB[i], yyB[i], kf); \
+        const int nx = min(i + 1, nn - 1);                        \
+        const float4 ua = va, ub = vb;                            \
+        va = __ldg(ndA + nx);                                     \
+        vb = __ldg(ndB + nx);                                     \
+        far_node_f32<CK, MODE_>(ma, pa, ua, node_yy(ua), kf);     \
+        far_node_f32<CK, MODE_>(mb, pb, ub, node_yy(ub), kf);     \
     }
     switch (mode) {
         case 0: BIELCC_BNODE2(0) break;
@@ -341,8 +347,43 @@ BIELCC_D void batch_moments2(const float4* ndA, const float* yyA, const float4* 
         default: BIELCC_BNODE2(4) break;
     }
 #undef BIELCC_BNODE2
-    store_moments<CK, float>(ma, PAr, PAi, dA, momA);
-    store_moments<CK, float>(mb, PBr, PBi, dB, momB);
+    store_moments<CK, float>(ma, PAr, PAi, fA.d, momA);
+    store_moments<CK, float>(mb, PBr, PBi, fB.d, momB);
+}
+
+// Phase A of cells cc and cc + kBW (< nc) of a chunk for this warp's 32 points,
+// mixed form, shared by the fused and the split pipeline: near bits, the rows
+// (each cell's shortest usable rule, rules.cu; a lane far from both takes both
+// at the longer of the two levels) and the 2 x 20 moments.
+BIELCC_D bool batch_two_cells(const RuleTab<float4>& tab, const float (*s_rmin)[kMaxRules], const double4* s_cell,
+                              const double* s_rho, unsigned char* s_near, int c0, int cc, int nc, int lane, bool live,
+                              const double* x, cplx k, float (&moa)[20], float (&mob)[20]) {
+    const int cb2 = cc + kBW;
+    const bool two = cb2 < nc;
+    FarDist da, db;
+    const bool na = da.near<true>(x, s_cell[cc]), nb = db.near<true>(x, s_cell[two ? cb2 : cc]);
+    const bool fa = !na && live, fb = two && !nb && live;
+    s_near[cc * kBP + lane] = na ? 1 : 0;
+    if (two) s_near[cb2 * kBP + lane] = nb ? 1 : 0;
+    const int la = rule_level(s_rmin[cc], tab.n_lev, warp_min_pos(rule_key(fa, da.d)));
+    const int lb = rule_level(s_rmin[two ? cb2 : cc], tab.n_lev, warp_min_pos(rule_key(fb, db.d)));
+#pragma unroll
+    for (int q = 0; q < 20; q++) moa[q] = mob[q] = 0.f;
+    const bool ck = k.im != 0.0;
+    if (fa && fb) {
+        const int l = max(la, lb), nn = tab.cnt[l];
+        const float4* row = tab.base[l] + (size_t)(c0 + cc) * nn;
+        if (ck) batch_moments2<true>(row, row + (size_t)kBW * nn, nn, da, s_rho[cc], db, s_rho[cb2], k, moa, mob);
+        else batch_moments2<false>(row, row + (size_t)kBW * nn, nn, da, s_rho[cc], db, s_rho[cb2], k, moa, mob);
+    } else if (fa || fb) {
+        const int l = fa ? la : lb, nn = tab.cnt[l], c = fa ? cc : cb2;
+        const float4* row = tab.base[l] + (size_t)(c0 + c) * nn;
+        float* mo = fa ? moa : mob;
+        const FarDist& fd = fa ? da : db;
+        if (ck) batch_moments<true, true>(row, nn, x, fd, s_rho[c], k, 0., 0., mo);
+        else batch_moments<true, false>(row, nn, x, fd, s_rho[c], k, 0., 0., mo);
+    }
+    return two;
 }
 
 // Phase B of one chunk: the right-hand sides s0 + sb + warp + 4 j (j < R) of the
@@ -445,6 +486,22 @@ BIELCC_D void batch_phase_b(const typename BatchCfg<MIXED>::F* s_mom, const type
     }
 }
 
+// The row table of a job (thread `who` fills it; visible after the next barrier).
+BIELCC_D void batch_fill_tab(RuleTab<float4>& t, const JobDev& jb, int nn, bool who) {
+    if (who) t.fill(jb.rules, jb.rules.n32, jb.nodes32, nn, jb.n_cells);
+}
+BIELCC_D void batch_fill_tab(RuleTab<double4>& t, const JobDev& jb, int nn, bool who) {
+    if (who) t.fill(jb.rules, jb.rules.n64, jb.nodes64, nn, jb.n_cells);
+}
+// Smallest distances of the levels of cells c0 .. c0 + nc - 1 at |k| = kabs.
+template <typename NodeT>
+BIELCC_D void batch_stage_limits(float (*s_rmin)[kMaxRules], const JobDev& jb, int c0, int nc, float kabs, int tid,
+                                 int threads) {
+    const int n_lev = jb.rules.n_lev;
+    const float2* lim = rule_limits(jb.rules, NodeT()) + (size_t)c0 * n_lev;
+    for (int i = tid; i < nc * n_lev; i += threads) s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], kabs);
+}
+
 // Stages the currents of RHS s0 .. s0 + sp - 1 of cells c0 .. c0 + nc - 1
 // (FP32 (re, im, im, re) for the packed contraction; FP64 (re, im)); SP: the
 // staging stride in right-hand sides.
@@ -476,18 +533,18 @@ __global__ void __launch_bounds__(kBT, MIXED ? BIELCC_BATCH_MINB : BIELCC_BATCH6
     using F = typename C::F;
     using NodeT = typename C::NodeT;
     extern __shared__ __align__(16) unsigned char smem[];
-    NodeT* s_nodes = (NodeT*)smem;
-    float* s_yy = (float*)(s_nodes + C::NODES);          // [NODES] (mixed form only)
-    F* s_mom = (F*)(s_yy + C::YY);                       // [CH][20][kBP]
+    F* s_mom = (F*)smem;                                 // [CH][20][kBP]
     F* s_j = s_mom + C::CH * 20 * kBP;                   // [CH][kSP][3][JW]
     double4* s_cell = (double4*)(s_j + C::CH * kSP * 3 * C::JW);  // centre, diam
     double* s_rho = (double*)(s_cell + C::CH);
     unsigned char* s_near = (unsigned char*)(s_rho + C::CH);  // [CH][kBP]
+    __shared__ RuleTab<NodeT> s_tab;                          // rows of the item's job
+    __shared__ float s_rmin[C::CH][kMaxRules];                // the chunk's limits
     __shared__ int s_item;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nn = n_start * n_start;
-    const int ch = max(1, min(C::CH, C::NODES / nn));
+    constexpr int ch = C::CH;
 
     for (int taken = 0; taken < max_items; taken++) {
         __syncthreads();
@@ -507,6 +564,8 @@ __global__ void __launch_bounds__(kBT, MIXED ? BIELCC_BATCH_MINB : BIELCC_BATCH6
         const int ce = min(N, cb + jb.cells_per_range);
         const cplx k = jb.k;
         const double k2r = k.re * k.re - k.im * k.im, k2i = 2.0 * k.re * k.im;
+        const float kabs = rule_kabs(k);
+        batch_fill_tab(s_tab, jb, nn, threadIdx.x == 0);
         unsigned nbits = 0;
 
         for (int c0 = cb; c0 < ce; c0 += ch) {
@@ -518,22 +577,10 @@ __global__ void __launch_bounds__(kBT, MIXED ? BIELCC_BATCH_MINB : BIELCC_BATCH6
             };
             auto stage_j = [&](int s0, int sp) { batch_stage_j<MIXED>(s_j, jb, c0, nc, s0, sp, threadIdx.x); };
             __syncthreads();
-            // stage node tables, cell rows and the first RHS pass's currents
-            if constexpr (MIXED) {
-                const float4* src = jb.nodes32 + (size_t)c0 * nn;
-                for (int i = threadIdx.x; i < nc * nn; i += kBT) {
-                    const float4 v = __ldg(src + i);
-                    s_nodes[i] = v;
-                    s_yy[i] = node_yy(v);
-                }
-            } else {
-                const double2* src = reinterpret_cast<const double2*>(jb.nodes64 + (size_t)c0 * nn);
-                double2* dst = reinterpret_cast<double2*>(s_nodes);
-                for (int i = threadIdx.x; i < 2 * nc * nn; i += kBT) dst[i] = __ldg(src + i);
-            }
+            // stage cell rows, limits and the first RHS pass's currents
+            batch_stage_limits<NodeT>(s_rmin, jb, c0, nc, kabs, threadIdx.x, kBT);
             for (int i = threadIdx.x; i < nc; i += kBT) {
-                const CellGeo& gg = jb.geo[c0 + i];
-                s_cell[i] = make_double4(gg.c[0], gg.c[1], gg.c[2], gg.diam);
+                s_cell[i] = near_cell(jb.geo[c0 + i], analytic_calc);
                 s_rho[i] = (double)jb.rho32[c0 + i];
             }
             stage_j(0, min(kSP, S));
@@ -542,61 +589,33 @@ __global__ void __launch_bounds__(kBT, MIXED ? BIELCC_BATCH_MINB : BIELCC_BATCH6
             // mixed form takes them two at a time (cells cc and cc + 4)
             if constexpr (MIXED && BIELCC_BATCH_TWO) {
                 for (int cc = warp; cc < nc; cc += 2 * kBW) {
-                    const int cb2 = cc + kBW;
-                    const bool two = cb2 < nc;
-                    const double4 ca = s_cell[cc], cbb = s_cell[two ? cb2 : cc];
-                    const double cena[3] = {ca.x, ca.y, ca.z}, cenb[3] = {cbb.x, cbb.y, cbb.z};
-                    double da, db;
-                    const bool na = is_near(x, cena, ca.w, analytic_calc, &da);
-                    const bool nb = is_near(x, cenb, cbb.w, analytic_calc, &db);
-                    const bool fa = !na && live, fb = two && !nb && live;
-                    s_near[cc * kBP + lane] = na ? 1 : 0;
-                    if (two) s_near[cb2 * kBP + lane] = nb ? 1 : 0;
                     F moa[20], mob[20];
-#pragma unroll
-                    for (int q = 0; q < 20; q++) moa[q] = mob[q] = 0;
-                    const NodeT *nda = s_nodes + cc * nn, *ndb = s_nodes + (two ? cb2 : cc) * nn;
-                    const float *ya = s_yy + cc * nn, *yb = s_yy + (two ? cb2 : cc) * nn;
-                    const bool ck = k.im != 0.0;
-                    if (fa && fb) {
-                        if (ck) batch_moments2<true>(nda, ya, ndb, yb, nn, x, ca, da, s_rho[cc], cbb, db,
-                                                     s_rho[cb2], k, moa, mob);
-                        else batch_moments2<false>(nda, ya, ndb, yb, nn, x, ca, da, s_rho[cc], cbb, db,
-                                                   s_rho[cb2], k, moa, mob);
-                    } else if (fa || fb) {
-                        const NodeT* nd = fa ? nda : ndb;
-                        const float* yy = fa ? ya : yb;
-                        const double4 ci = fa ? ca : cbb;
-                        const double d = fa ? da : db, rho = s_rho[fa ? cc : cb2];
-                        F* mo = fa ? moa : mob;
-                        if (ck) batch_moments<MIXED, true>(nd, yy, nn, x, ci, d, rho, k, k2r, k2i, mo);
-                        else batch_moments<MIXED, false>(nd, yy, nn, x, ci, d, rho, k, k2r, k2i, mo);
-                    }
+                    const bool two = batch_two_cells(s_tab, s_rmin, s_cell, s_rho, s_near, c0, cc, nc, lane, live, x, k,
+                                                     moa, mob);
 #pragma unroll
                     for (int q = 0; q < 20; q++) s_mom[(cc * 20 + q) * kBP + lane] = moa[q];
                     if (two) {
 #pragma unroll
-                        for (int q = 0; q < 20; q++) s_mom[(cb2 * 20 + q) * kBP + lane] = mob[q];
+                        for (int q = 0; q < 20; q++) s_mom[((cc + kBW) * 20 + q) * kBP + lane] = mob[q];
                     }
                 }
             } else {
                 for (int cc = warp; cc < nc; cc += kBW) {
-                    const double4 ci = s_cell[cc];
-                    const double cen[3] = {ci.x, ci.y, ci.z};
-                    double d;
-                    const bool nr = is_near(x, cen, ci.w, analytic_calc, &d);
+                    FarDist fd{};
+                    const bool nr = fd.template near<MIXED>(x, s_cell[cc]);
                     const bool far = !nr && live;
                     s_near[cc * kBP + lane] = nr ? 1 : 0;
                     F mom[20];
 #pragma unroll
                     for (int q = 0; q < 20; q++) mom[q] = 0;
+                    const int l = rule_level(s_rmin[cc], s_tab.n_lev, warp_min_pos(rule_key(far, fd.d)));
                     if (far) {
-                        const NodeT* nd = s_nodes + cc * nn;
-                        const float* yy = s_yy + (MIXED ? cc * nn : 0);
+                        const int kc = s_tab.cnt[l];
+                        const NodeT* nd = s_tab.base[l] + (size_t)(c0 + cc) * kc;
                         if (k.im != 0.0)
-                            batch_moments<MIXED, true>(nd, yy, nn, x, ci, d, s_rho[cc], k, k2r, k2i, mom);
+                            batch_moments<MIXED, true>(nd, kc, x, fd, s_rho[cc], k, k2r, k2i, mom);
                         else
-                            batch_moments<MIXED, false>(nd, yy, nn, x, ci, d, s_rho[cc], k, k2r, k2i, mom);
+                            batch_moments<MIXED, false>(nd, kc, x, fd, s_rho[cc], k, k2r, k2i, mom);
                     }
 #pragma unroll
                     for (int q = 0; q < 20; q++) s_mom[(cc * 20 + q) * kBP + lane] = mom[q];
@@ -646,8 +665,8 @@ __global__ void __launch_bounds__(kBT, BIELCC_MOM_MINB)
     batch_moments_kernel(const JobDev* __restrict__ jobs, const BatchItem* __restrict__ items, int n_items,
                          int* __restrict__ counter, double analytic_calc, int n_start, int max_items,
                          float* __restrict__ mom) {
-    __shared__ __align__(16) float4 s_nodes[kMomCells * 64];
-    __shared__ float s_yy[kMomCells * 64];
+    __shared__ RuleTab<float4> s_tab;
+    __shared__ float s_rmin[kMomCells][kMaxRules];
     __shared__ double4 s_cell[kMomCells];
     __shared__ double s_rho[kMomCells];
     __shared__ unsigned char s_near[kMomCells * kBP];
@@ -673,64 +692,32 @@ __global__ void __launch_bounds__(kBT, BIELCC_MOM_MINB)
         const int cb = bi.range * jb.cells_per_range;
         const int ce = min(N, cb + jb.cells_per_range);
         const cplx k = jb.k;
-        const double k2r = k.re * k.re - k.im * k.im, k2i = 2.0 * k.re * k.im;
-        const bool ck = k.im != 0.0;
+        const float kabs = rule_kabs(k);
+        batch_fill_tab(s_tab, jb, nn, threadIdx.x == 0);
         float* mo = mom + (size_t)bi.pad * kMomBlock;  // the item's blocks, in cell order
         unsigned nbits = 0;
 
         for (int c0 = cb; c0 < ce; c0 += kMomCells) {
             const int nc = min(kMomCells, ce - c0);
-            __syncthreads();  // the previous chunk's reads of the staged nodes are done
+            __syncthreads();  // the previous chunk's reads of the staged rows are done
             {
-                const float4* src = jb.nodes32 + (size_t)c0 * nn;
-                for (int i = threadIdx.x; i < nc * nn; i += kBT) {
-                    const float4 v = __ldg(src + i);
-                    s_nodes[i] = v;
-                    s_yy[i] = node_yy(v);
-                }
+                batch_stage_limits<float4>(s_rmin, jb, c0, nc, kabs, threadIdx.x, kBT);
                 for (int i = threadIdx.x; i < nc; i += kBT) {
-                    const CellGeo& gg = jb.geo[c0 + i];
-                    s_cell[i] = make_double4(gg.c[0], gg.c[1], gg.c[2], gg.diam);
+                    s_cell[i] = near_cell(jb.geo[c0 + i], analytic_calc);
                     s_rho[i] = (double)jb.rho32[c0 + i];
                 }
             }
             __syncthreads();
             // cells warp and warp + 4 of the block, two at a time (batch_far_kernel's pairing)
             for (int cc = warp; cc < nc; cc += 2 * kBW) {
-                const int cb2 = cc + kBW;
-                const bool two = cb2 < nc;
-                const double4 ca = s_cell[cc], cbb = s_cell[two ? cb2 : cc];
-                const double cena[3] = {ca.x, ca.y, ca.z}, cenb[3] = {cbb.x, cbb.y, cbb.z};
-                double da, db;
-                const bool na = is_near(x, cena, ca.w, analytic_calc, &da);
-                const bool nb = is_near(x, cenb, cbb.w, analytic_calc, &db);
-                const bool fa = !na && live, fb = two && !nb && live;
-                s_near[cc * kBP + lane] = na ? 1 : 0;
-                if (two) s_near[cb2 * kBP + lane] = nb ? 1 : 0;
                 float moa[20], mob[20];
-#pragma unroll
-                for (int q = 0; q < 20; q++) moa[q] = mob[q] = 0.f;
-                const float4 *nda = s_nodes + cc * nn, *ndb = s_nodes + (two ? cb2 : cc) * nn;
-                const float *ya = s_yy + cc * nn, *yb = s_yy + (two ? cb2 : cc) * nn;
-                if (fa && fb) {
-                    if (ck) batch_moments2<true>(nda, ya, ndb, yb, nn, x, ca, da, s_rho[cc], cbb, db, s_rho[cb2], k,
+                const bool two = batch_two_cells(s_tab, s_rmin, s_cell, s_rho, s_near, c0, cc, nc, lane, live, x, k,
                                                  moa, mob);
-                    else batch_moments2<false>(nda, ya, ndb, yb, nn, x, ca, da, s_rho[cc], cbb, db, s_rho[cb2], k,
-                                               moa, mob);
-                } else if (fa || fb) {
-                    const float4* nd = fa ? nda : ndb;
-                    const float* yy = fa ? ya : yb;
-                    const double4 ci = fa ? ca : cbb;
-                    const double d = fa ? da : db, rho = s_rho[fa ? cc : cb2];
-                    float* mo1 = fa ? moa : mob;
-                    if (ck) batch_moments<true, true>(nd, yy, nn, x, ci, d, rho, k, k2r, k2i, mo1);
-                    else batch_moments<true, false>(nd, yy, nn, x, ci, d, rho, k, k2r, k2i, mo1);
-                }
                 float* da_ = mo + (size_t)(c0 - cb + cc) * 20 * kBP + lane;
 #pragma unroll
                 for (int q = 0; q < 20; q++) da_[q * kBP] = moa[q];
                 if (two) {
-                    float* db_ = mo + (size_t)(c0 - cb + cb2) * 20 * kBP + lane;
+                    float* db_ = mo + (size_t)(c0 - cb + cc + kBW) * 20 * kBP + lane;
 #pragma unroll
                     for (int q = 0; q < 20; q++) db_[q * kBP] = mob[q];
                 }
@@ -871,11 +858,11 @@ constexpr uint32_t kTmemAlloc = kGroups * kTmemCols;    // per CTA (all 512 colu
 constexpr uint32_t kAbytes = kRows * kK * 4;     // one of A hi / A lo
 constexpr uint32_t kBbytes = 2 * kG * kK * 4;    // one of B hi / B lo of one buffer
 constexpr uint32_t kSbo = (kK / 4) * 128;        // byte distance of 8-row groups
-constexpr int kNodes = kRound * 64;              // n_start <= 8
 // per group: A hi, A lo, then B (2 buffers x hi, lo): the second M block of A
 // lo reads its 64 unused rows from the B buffers, which are larger than that.
-constexpr size_t kOffAl = kAbytes, kOffB = 2 * (size_t)kAbytes, kOffNodes = kOffB + 4 * (size_t)kBbytes;
-constexpr size_t kOffYY = kOffNodes + 16 * (size_t)kNodes, kOffCell = kOffYY + 4 * (size_t)kNodes;
+constexpr size_t kOffAl = kAbytes, kOffB = 2 * (size_t)kAbytes, kOffTab = kOffB + 4 * (size_t)kBbytes;
+constexpr size_t kOffLim = kOffTab + 128, kOffCell = kOffLim + 256;  // row table, limits
+static_assert(sizeof(RuleTab<float4>) <= 128 && kRound * kMaxRules * sizeof(float) <= 256, "row table and limits fit");
 constexpr size_t kOffRho = kOffCell + 32 * kRound, kOffNear = kOffRho + 8 * kRound;
 constexpr size_t kSmemGroup = kOffNear + kRound * 32;
 constexpr size_t kGroupStride = (kSmemGroup + 1023) & ~(size_t)1023;
@@ -1017,8 +1004,8 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
     unsigned char* sAh = smem;
     unsigned char* sAl = smem + tcb::kOffAl;
     unsigned char* sB = smem + tcb::kOffB;  // buffer q: hi at 2 q kBbytes, lo at (2 q + 1) kBbytes
-    float4* s_nodes = reinterpret_cast<float4*>(smem + tcb::kOffNodes);
-    float* s_yy = reinterpret_cast<float*>(smem + tcb::kOffYY);
+    RuleTab<float4>& s_tab = *reinterpret_cast<RuleTab<float4>*>(smem + tcb::kOffTab);
+    float(*s_rmin)[kMaxRules] = reinterpret_cast<float(*)[kMaxRules]>(smem + tcb::kOffLim);
     double4* s_cell = reinterpret_cast<double4*>(smem + tcb::kOffCell);
     double* s_rho = reinterpret_cast<double*>(smem + tcb::kOffRho);
     unsigned char* s_near = smem + tcb::kOffNear;
@@ -1090,6 +1077,8 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
         const double k2r = k.re * k.re - k.im * k.im, k2i = 2.0 * k.re * k.im;
         const bool ck = k.im != 0.0;
         const float* mo = BUF ? mom + (size_t)bi.pad * kMomBlock : nullptr;
+        const float kabs = rule_kabs(k);
+        if constexpr (!BUF) batch_fill_tab(s_tab, jb, nn, gt == 0);
         const int G = (S + tcb::kG - 1) / tcb::kG;
         const int Spad = (S + 7) & ~7;
         unsigned nbits = 0;
@@ -1130,16 +1119,10 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
                 const int nc = min(tcb::kRound, ce - rc0);
                 if (nc <= 0) break;
                 if constexpr (!BUF) {
-                    group_sync(bar_id);  // the previous round's reads of the staged nodes are done
-                    const float4* src = jb.nodes32 + (size_t)rc0 * nn;
-                    for (int i = gt; i < nc * nn; i += tcb::kGroupThreads) {
-                        const float4 v = __ldg(src + i);
-                        s_nodes[i] = v;
-                        s_yy[i] = node_yy(v);
-                    }
+                    group_sync(bar_id);  // the previous round's reads of the staged rows are done
+                    batch_stage_limits<float4>(s_rmin, jb, rc0, nc, kabs, gt, tcb::kGroupThreads);
                     for (int i = gt; i < nc; i += tcb::kGroupThreads) {
-                        const CellGeo& gg = jb.geo[rc0 + i];
-                        s_cell[i] = make_double4(gg.c[0], gg.c[1], gg.c[2], gg.diam);
+                        s_cell[i] = near_cell(jb.geo[rc0 + i], analytic_calc);
                         s_rho[i] = (double)jb.rho32[rc0 + i];
                     }
                     group_sync(bar_id);
@@ -1155,16 +1138,16 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
                         for (int q = 0; q < 20; q++) mom[q] = __ldcs(src + q * kBP);
                     }
                 } else if (warp < nc) {
-                    const double4 ci = s_cell[warp];
-                    const double cen[3] = {ci.x, ci.y, ci.z};
-                    double d;
-                    const bool nr = is_near(x, cen, ci.w, analytic_calc, &d);
+                    FarDist fd{};
+                    const bool nr = fd.near<true>(x, s_cell[warp]);
                     s_near[warp * 32 + lane] = nr ? 1 : 0;
-                    if (!nr && live) {
-                        const float4* nd = s_nodes + warp * nn;
-                        const float* yy = s_yy + warp * nn;
-                        if (ck) batch_moments<true, true>(nd, yy, nn, x, ci, d, s_rho[warp], k, k2r, k2i, mom);
-                        else batch_moments<true, false>(nd, yy, nn, x, ci, d, s_rho[warp], k, k2r, k2i, mom);
+                    const bool far = !nr && live;
+                    const int l = rule_level(s_rmin[warp], s_tab.n_lev, warp_min_pos(rule_key(far, fd.d)));
+                    if (far) {
+                        const int kc = s_tab.cnt[l];
+                        const float4* nd = s_tab.base[l] + (size_t)(rc0 + warp) * kc;
+                        if (ck) batch_moments<true, true>(nd, kc, x, fd, s_rho[warp], k, k2r, k2i, mom);
+                        else batch_moments<true, false>(nd, kc, x, fd, s_rho[warp], k, k2r, k2i, mom);
                     }
                 }
                 // A and B are free once the previous round's MMAs completed; D of

@@ -366,6 +366,7 @@ cudaError_t start_field_batch(bielcc_server_s* sv, Slot& sl) {
         d.nodes32 = m->nodes32;
         d.nodes64 = m->nodes64;
         d.rho32 = m->rho32;
+        d.rules = m->rules;
         d.verts = m->verts;
         d.nv = m->nv;
         d.n_cells = m->n_cells;
