@@ -23,8 +23,9 @@
 namespace bielcc_gpu {
 
 constexpr int kAsmThreads = 128;
-constexpr int kAsmStageNodes = 256;
-constexpr int kAsmMaxCells = 32;
+constexpr int kAsmStageCells = 32;  // column cells staged at a time: one mask word
+constexpr int kAsmWays = 4;         // warps that share the columns on small matrices
+constexpr size_t kAsmOutBytes = (size_t)(kAsmThreads / 32) * 2 * 32 * 8 * 16;  // staged blocks of a CTA (32 KB)
 
 struct AsmArgs {
     const CellGeo* geo;
@@ -33,9 +34,11 @@ struct AsmArgs {
     const float4* nodes32;
     const float* rho32;
     int nn;
+    FarRules rules;
     cplx k;
     double analytic_calc;
     int cols_per_split;
+    int ways;  // 1, or kAsmWays: the CTA's warps share the columns, 32 rows per CTA
     int m;  // 2 (tau) or 3 (full)
     int c64;
     void* A;
@@ -59,18 +62,14 @@ BIELCC_D bool asm_is_near(const double* x, const CellGeo& g, double analytic_cal
     return *d < __dmul_rn(analytic_calc, g.diam);
 }
 
-// Writes the M x M block of (row cell i, column cell j) from the 3x3 complex
-// operator matrix K (already / 4pi): M = 2 projects on tau1, tau2 of both
-// cells, M = 3 keeps the Cartesian block. M is a template argument so that the
-// block stays in registers.
+// The M x M block of (row cell i, column cell j) from the 3x3 complex operator
+// matrix K (already / 4pi): M = 2 projects on tau1, tau2 of both cells, M = 3 keeps
+// the Cartesian block. M is a template argument so that the block stays in registers.
 template <int M>
-BIELCC_D void write_block_m(const AsmArgs& a, int i, int j, const double (&Kr)[3][3], const double (&Ki)[3][3],
-                            const double* ti1, const double* ti2, const double* tj1, const double* tj2,
-                            unsigned cols = ~0u) {
-    const size_t dim = (size_t)M * a.n_cells;
+BIELCC_D void block_f64(const double (&Kr)[3][3], const double (&Ki)[3][3], const double* ti1, const double* ti2,
+                        const double* tj1, const double* tj2, double (&o)[M][M][2]) {
 #pragma unroll
     for (int aa = 0; aa < M; aa++) {
-        double rv[M][2];
 #pragma unroll
         for (int b = 0; b < M; b++) {
             double vr = 0., vi = 0.;
@@ -88,35 +87,50 @@ BIELCC_D void write_block_m(const AsmArgs& a, int i, int j, const double (&Kr)[3
                     vi += ta[p] * ki;
                 }
             }
-            rv[b][0] = vr;
-            rv[b][1] = vi;
+            o[aa][b][0] = vr;
+            o[aa][b][1] = vi;
         }
+    }
+}
+
+// Writes a block; cols: bit b writes column b (the convergence-test passes of
+// p_max >= 3; all otherwise).
+template <int M, typename F>
+BIELCC_D void store_block(const AsmArgs& a, int i, int j, const F (&o)[M][M][2], unsigned cols) {
+    const size_t dim = (size_t)M * a.n_cells;
+#pragma unroll
+    for (int aa = 0; aa < M; aa++) {
         const size_t off = ((size_t)i * M + aa) * dim + (size_t)j * M;
         if (a.c64) {
             float2* dst = reinterpret_cast<float2*>(a.A) + off;
 #pragma unroll
             for (int b = 0; b < M; b++)
-                if ((cols >> b) & 1u) dst[b] = make_float2((float)rv[b][0], (float)rv[b][1]);
+                if ((cols >> b) & 1u) dst[b] = make_float2((float)o[aa][b][0], (float)o[aa][b][1]);
         } else {
             double2* dst = reinterpret_cast<double2*>(a.A) + off;
 #pragma unroll
             for (int b = 0; b < M; b++)
-                if ((cols >> b) & 1u) dst[b] = make_double2(rv[b][0], rv[b][1]);
+                if ((cols >> b) & 1u) dst[b] = make_double2(o[aa][b][0], o[aa][b][1]);
         }
     }
+}
+
+template <int M>
+BIELCC_D void write_block_m(const AsmArgs& a, int i, int j, const double (&Kr)[3][3], const double (&Ki)[3][3],
+                            const double* ti1, const double* ti2, const double* tj1, const double* tj2,
+                            unsigned cols = ~0u) {
+    double o[M][M][2];
+    block_f64<M>(Kr, Ki, ti1, ti2, tj1, tj2, o);
+    store_block<M, double>(a, i, j, o, cols);
 }
 
 // The mixed form's far block, in FP32 (the moments are FP32 sums already):
 // K = A1 I + T with T symmetric (xx, xy, xz, yy, yz, zz), projected on the two
 // cells' tangents (M = 2: u_b = K t_b, A_ab = t_a . u_b) or kept Cartesian
 // (M = 3), times ph = e^{ik r0} / 4pi.
-// cols: bit b writes column b of the block (the convergence-test passes of
-// p_max >= 3; all otherwise).
 template <int M>
-BIELCC_D void write_block_f32(const AsmArgs& a, int i, int j, float a1r, float a1i, const float (&t)[6][2], float phr,
-                              float phi, const float (&ti)[2][3], const double* tj1, const double* tj2,
-                              unsigned cols = ~0u) {
-    const size_t dim = (size_t)M * a.n_cells;
+BIELCC_D void block_f32(float a1r, float a1i, const float (&t)[6][2], float phr, float phi, const float (&ti)[2][3],
+                        const double* tj1, const double* tj2, float (&out)[M][M][2]) {
     const int sym[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
     float kr[6], ki[6];
 #pragma unroll
@@ -125,7 +139,6 @@ BIELCC_D void write_block_f32(const AsmArgs& a, int i, int j, float a1r, float a
         kr[q] = diag ? t[q][0] + a1r : t[q][0];
         ki[q] = diag ? t[q][1] + a1i : t[q][1];
     }
-    float out[M][M][2];
     if constexpr (M == 3) {
 #pragma unroll
         for (int p = 0; p < 3; p++)
@@ -154,21 +167,15 @@ BIELCC_D void write_block_f32(const AsmArgs& a, int i, int j, float a1r, float a
             }
         }
     }
-#pragma unroll
-    for (int aa = 0; aa < M; aa++) {
-        const size_t off = ((size_t)i * M + aa) * dim + (size_t)j * M;
-        if (a.c64) {
-            float2* dst = reinterpret_cast<float2*>(a.A) + off;
-#pragma unroll
-            for (int b = 0; b < M; b++)
-                if ((cols >> b) & 1u) dst[b] = make_float2(out[aa][b][0], out[aa][b][1]);
-        } else {
-            double2* dst = reinterpret_cast<double2*>(a.A) + off;
-#pragma unroll
-            for (int b = 0; b < M; b++)
-                if ((cols >> b) & 1u) dst[b] = make_double2(out[aa][b][0], out[aa][b][1]);
-        }
-    }
+}
+
+template <int M>
+BIELCC_D void write_block_f32(const AsmArgs& a, int i, int j, float a1r, float a1i, const float (&t)[6][2], float phr,
+                              float phi, const float (&ti)[2][3], const double* tj1, const double* tj2,
+                              unsigned cols = ~0u) {
+    float out[M][M][2];
+    block_f32<M>(a1r, a1i, t, phr, phi, ti, tj1, tj2, out);
+    store_block<M, float>(a, i, j, out, cols);
 }
 
 BIELCC_D void write_block(const AsmArgs& a, int i, int j, const double (&Kr)[3][3], const double (&Ki)[3][3],
@@ -184,133 +191,137 @@ BIELCC_D void write_block(const AsmArgs& a, int i, int j, const double (&Kr)[3][
 #ifndef BIELCC_ASM_MINB
 #define BIELCC_ASM_MINB 5
 #endif
-template <bool CK, bool MIXED, bool MARKS = false>
+// A warp (32 rows, one per lane) takes each column cell's row of nodes from the
+// shortest rule that its nearest far row cell allows (rules.cu), staged as in
+// far_kernel. ways = 1: 128 rows per CTA, every warp all columns; ways = 4, for
+// matrices too small to fill the GPU: 32 rows, each warp every fourth column.
+// STAGE (TAU2, ways = 1): a lane's 2 x 2 block is 16 bytes (complex64) of two
+// matrix rows, so writing it directly touches 64 lines per warp and cell for
+// half a sector each. Blocks go to shared memory instead (row chunks of 128 bytes,
+// rotated by the lane so that neither side conflicts) and are written eight
+// (complex128: four) columns at a time in whole lines; near blocks are written
+// too (as zeros) and overwritten by asm_near_kernel, which always follows.
+// 20,480 triangles, mixed, complex64, whole call: 65.6 ms with all 64 nodes and
+// direct writes, 28.2 with the rules, 23.3 with rows staged per warp and whole-line
+// writes (this kernel 17.1 of it; bound by issue slots, 13.4 GB written).
+// ways = 4: 80 triangles, FP64, 0.70 -> 0.28 ms.
+template <bool CK, bool MIXED, bool MARKS = false, bool STAGE = false>
 __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB : 0)
-    assemble_far_kernel(AsmArgsOf<MARKS> a) {
+    assemble_far_kernel(const __grid_constant__ AsmArgsOf<MARKS> a) {
     using NodeT = typename std::conditional<MIXED, float4, double4>::type;
-    __shared__ __align__(16) NodeT s_nodes[kAsmStageNodes];
-    __shared__ float s_yy[MIXED ? kAsmStageNodes : 1];  // |y - centre|^2 of the staged nodes (mixed form)
-    __shared__ CellGeo s_geo[kAsmMaxCells];
-    __shared__ float s_rho[kAsmMaxCells];
+    constexpr int kWarps = kAsmThreads / 32;
+    static_assert(kWarps == kAsmWays, "ways = 4 gives every warp its share of the columns");
+    __shared__ __align__(16) RowBuf<NodeT> s_rows[kWarps];
+    __shared__ RuleTab<NodeT> s_tab;
+    __shared__ CellGeo s_geo[kAsmStageCells];
+    __shared__ double4 s_cell[kAsmStageCells];  // centre, near square
+    __shared__ int s_mode[kAsmStageCells];      // mixed: phase polynomial; FP64: 1 phase split, 0 sincos per node
+    __shared__ float s_rmin[kAsmStageCells][kMaxRules];
+    __shared__ unsigned s_near[kWarps][32];
+    extern __shared__ __align__(16) uint4 s_out[];  // STAGE: [warp][2][32][8] 16-byte pieces
 
-    const int i = blockIdx.x * kAsmThreads + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool split_cols = !STAGE && a.ways > 1;
+    const int i = split_cols ? blockIdx.x * 32 + lane : blockIdx.x * kAsmThreads + threadIdx.x;
     const bool live = i < a.n_cells;
-    CellGeo gi;
-    if (live) gi = a.geo[i];
-    else gi = a.geo[0];
-    const double* x = gi.c;
-    const int cb = blockIdx.y * a.cols_per_split;
+    const CellGeo& gi = a.geo[live ? i : 0];
+    const double x[3] = {gi.c[0], gi.c[1], gi.c[2]};
+    const int cb = blockIdx.y * a.cols_per_split;  // a multiple of 32
     const int ce = min(a.n_cells, cb + a.cols_per_split);
-    const int nn = a.nn;
-    const int cps = nn <= kAsmStageNodes ? max(1, min(kAsmMaxCells, kAsmStageNodes / nn)) : 1;
-    const int kchunk = nn <= kAsmStageNodes ? nn : kAsmStageNodes;
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
+    const int n_lev = a.rules.n_lev;
+    if (threadIdx.x == 0) {
+        const NodeT* full;
+        if constexpr (MIXED) full = a.nodes32;
+        else full = a.nodes64;
+        s_tab.fill(a.rules, rule_rows(a.rules, NodeT()), full, a.nn, a.n_cells);
+    }
 
-    using F = typename std::conditional<MIXED, float, double>::type;
-    F a1r = 0, a1i = 0, t[6][2];
-    bool far = false;
     unsigned cols = ~0u;  // MARKS: the block columns this pass writes
-    PairF32 pf{};
     const KF32 kf = KF32::make(a.k.re, a.k.im);
     // the row cell's tangents in FP32 (mixed-form block projection)
-    const float tif[2][3] = {{(float)gi.t1[0], (float)gi.t1[1], (float)gi.t1[2]},
-                             {(float)gi.t2[0], (float)gi.t2[1], (float)gi.t2[2]}};
-    double P0r = 1., P0i = 0.;
-    int mode = 0;  // phase polynomial of the current cell (farnode.cuh phase_mode)
-    bool split64 = false;
-    double r0d = 0.;
-    unsigned nbits = 0;  // near bits of the current 32-column word
+    float tif[2][3];
+    if constexpr (MIXED) {
+#pragma unroll
+        for (int g = 0; g < 3; g++) {
+            tif[0][g] = (float)gi.t1[g];
+            tif[1][g] = (float)gi.t2[g];
+        }
+    }
+    const int group = a.c64 ? 8 : 4;  // STAGE: columns per 128-byte row chunk
+    uint4* out = STAGE ? s_out + warp * 512 : nullptr;
 
-    for (int c0 = cb; c0 < ce; c0 += cps) {
-        const int nc = min(cps, ce - c0);
-        for (int k0 = 0; k0 < nn; k0 += kchunk) {
-            const int kc = min(kchunk, nn - k0);
-            __syncthreads();
-            const int tot = nc * kc;
-            if constexpr (MIXED) {
-                const float4* src = a.nodes32 + (size_t)c0 * nn + k0;
-                for (int q = threadIdx.x; q < tot; q += kAsmThreads) {
-                    int cc = q / kc, kk = q - cc * kc;
-                    const float4 v = __ldg(src + (size_t)cc * nn + kk);
-                    s_nodes[q] = v;
-                    s_yy[q] = node_yy(v);
-                }
-            } else {
-                const double2* src = reinterpret_cast<const double2*>(a.nodes64 + (size_t)c0 * nn + k0);
-                double2* dst = reinterpret_cast<double2*>(s_nodes);
-                for (int q = threadIdx.x; q < 2 * tot; q += kAsmThreads) {
-                    int node = q >> 1, cc = node / kc, kk = node - cc * kc;
-                    dst[q] = __ldg(src + 2 * ((size_t)cc * nn + kk) + (q & 1));
+    for (int c0 = cb; c0 < ce; c0 += kAsmStageCells) {
+        const int nc = min(kAsmStageCells, ce - c0);
+        unsigned nbits = 0;  // near bits of this 32-column word
+        __syncthreads();
+        for (int q = threadIdx.x; q < nc * 16; q += kAsmThreads)
+            reinterpret_cast<double*>(s_geo)[q] = reinterpret_cast<const double*>(a.geo + c0)[q];
+        for (int q = threadIdx.x; q < nc; q += kAsmThreads) {
+            s_cell[q] = near_cell(a.geo[c0 + q], a.analytic_calc);
+            if constexpr (MIXED) s_mode[q] = phase_mode((float)fabs(a.k.re) * a.rho32[c0 + q]);
+            else s_mode[q] = !CK && fabs(a.k.re) * (double)a.rho32[c0 + q] * (1.0 + 1e-6) <= 0.5;
+        }
+        {
+            const float kabs = rule_kabs(a.k);
+            const float2* lim = rule_limits(a.rules, NodeT()) + (size_t)c0 * n_lev;
+            for (int q = threadIdx.x; q < nc * n_lev; q += kAsmThreads)
+                s_rmin[q / n_lev][q % n_lev] = rule_rmin(lim[q], kabs);
+        }
+        __syncthreads();
+        for (int cc = split_cols ? warp : 0; cc < nc; cc += split_cols ? kWarps : 1) {
+            double dx[3], s2;
+            const bool nr = near_exact(x, s_cell[cc], dx, &s2);
+            const double d = dist_from_sq<!MIXED>(s2);
+            bool far = live && !nr;
+            nbits |= (nr ? 1u : 0u) << cc;
+            if constexpr (MARKS) {
+                if (far) {
+                    const int c = c0 + cc;
+                    const size_t wi = (size_t)(c >> 5) * a.n_cells + i;
+                    const size_t plane = (size_t)((a.n_cells + 31) >> 5) * a.n_cells;
+                    cols = 0u;
+                    for (int b = 0; b < a.m; b++)
+                        if ((((a.mark[b * plane + wi] >> (c & 31)) & 1u) != 0) == (a.take_marked != 0)) cols |= 1u << b;
+                    far = cols != 0u;
                 }
             }
-            if (k0 == 0)
-                for (int q = threadIdx.x; q < nc; q += kAsmThreads) {
-                    s_geo[q] = a.geo[c0 + q];
-                    s_rho[q] = a.rho32[c0 + q];
+            const float dmin = warp_min_pos(rule_key(far, d));
+            const bool any = dmin < __int_as_float(0x7f800000);
+            const CellGeo& gj = s_geo[cc];
+            double Kr[3][3], Ki[3][3];     // FP64 form: the operator matrix
+            float a1r = 0, a1i = 0, t[6][2], phr = 0, phi = 0;  // mixed form: moments and phase / 4pi
+#pragma unroll
+            for (int q = 0; q < 6; q++) t[q][0] = t[q][1] = 0;
+            if (any) {
+                const int lev = rule_level(s_rmin[cc], n_lev, dmin);
+                const int cnt = s_tab.cnt[lev], mode = s_mode[cc];
+                const NodeT* row = s_tab.base[lev] + (size_t)(c0 + cc) * cnt;
+                NodeT v{};
+                if (lane < cnt) v = row[lane];  // on its way during the pair's set-up
+                PairF32 pf{};
+                Moments<double> mm;
+                double P0r = 1., P0i = 0.;
+                if constexpr (MIXED) {
+                    pf.set(dx, s2, d, kf);
+                    turn_f32(d * (a.k.re * kInvTwoPi), CK ? exp(-a.k.im * d) * kInvFourPi : kInvFourPi, &phr, &phi);
+                } else {
+                    mm.zero();
+                    if (mode) sincos(a.k.re * d, &P0i, &P0r);
                 }
-            __syncthreads();
-            for (int cc = 0; cc < nc; cc++) {
-                const CellGeo& gj = s_geo[cc];
-                if (k0 == 0) {
-                    double d;
-                    const bool nr = asm_is_near(x, gj, a.analytic_calc, &d);
-                    far = live && !nr;
-                    if constexpr (MARKS) {
-                        if (far) {
-                            const int c = c0 + cc;
-                            const size_t wi = (size_t)(c >> 5) * a.n_cells + i;
-                            const size_t plane = (size_t)((a.n_cells + 31) >> 5) * a.n_cells;
-                            cols = 0u;
-                            for (int b = 0; b < a.m; b++)
-                                if ((((a.mark[b * plane + wi] >> (c & 31)) & 1u) != 0) == (a.take_marked != 0))
-                                    cols |= 1u << b;
-                            far = cols != 0u;
-                        }
-                    }
-                    if (a.mask) {
-                        const int c = c0 + cc;
-                        nbits |= (nr ? 1u : 0u) << (c & 31);
-                        if ((c & 31) == 31 || c == ce - 1) {
-                            if (live) a.mask[(size_t)(c >> 5) * a.n_cells + i] = nbits;
-                            nbits = 0;
-                        }
-                    }
-                    a1r = a1i = 0;
-                    for (int q = 0; q < 6; q++) t[q][0] = t[q][1] = 0;
-                    if (!MIXED && far) {  // FP64 phase split when the cell's phase range is small
-                        split64 = !CK && fabs(a.k.re) * (double)s_rho[cc] * (1.0 + 1e-6) <= 0.5;
-                        r0d = d;
-                        if (split64) {
-                            double sn, cs;
-                            sincos(a.k.re * d, &sn, &cs);
-                            P0r = cs;
-                            P0i = sn;
-                        } else {
-                            P0r = 1.0;
-                            P0i = 0.0;
-                        }
-                    }
-                    if (MIXED && far) {
-                        pf.set(x, gj.c, d, kf);
-                        double sn, cs;
-                        sincos(a.k.re * d, &sn, &cs);
-                        if (CK) {
-                            double am = exp(-a.k.im * d);
-                            sn *= am;
-                            cs *= am;
-                        }
-                        P0r = cs;
-                        P0i = sn;
-                        mode = phase_mode((float)fabs(a.k.re) * s_rho[cc]);
-                    }
-                }
-                if (far) {
-                    const NodeT* nd = s_nodes + cc * kc;
+                for (int k0 = 0; k0 < cnt; k0 += kRowChunk) {
+                    const int kc = min(kRowChunk, cnt - k0);
+                    RowBuf<NodeT>& rb = s_rows[warp];
+                    if (k0 && lane < kc) v = row[k0 + lane];
+                    __syncwarp();  // the previous chunk has been read
+                    rb.nd[lane] = v;
+                    if constexpr (MIXED) rb.yy[lane] = node_yy(v);
+                    __syncwarp();
+                    if (!far) continue;
                     if constexpr (MIXED) {
-                        const float* yy = s_yy + cc * kc;
-#define BIELCC_ASM_LOOP(MODE_)         \
-    _Pragma("unroll 4") for (int q = 0; q < kc; q++) \
-        far_node_f32_K<CK, MODE_>(a1r, a1i, t, pf, nd[q], yy[q], kf);
+#define BIELCC_ASM_LOOP(MODE_)                                                \
+    _Pragma("unroll 4") for (int q = 0; q < kc; q++)                          \
+        far_node_f32_K<CK, MODE_>(a1r, a1i, t, pf, rb.nd[q], rb.yy[q], kf);
                         switch (mode) {
                             case 0: BIELCC_ASM_LOOP(0) break;
                             case 1: BIELCC_ASM_LOOP(1) break;
@@ -319,64 +330,109 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                             default: BIELCC_ASM_LOOP(4) break;
                         }
 #undef BIELCC_ASM_LOOP
-                    } else {
+                    } else if (mode) {
                         // FP64: the field kernel's node (phase relative to r0 with the Taylor
                         // series when |k| rho <= 0.5); its grad-F moments are unused here
-                        Moments<double> mm;
-                        mm.zero();
-                        if (split64) {
 #pragma unroll 2
-                            for (int q = 0; q < kc; q++) {
-                                const double4 v = nd[q];
-                                far_node_f64<CK, true>(mm, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, a.k, k2r, k2i,
-                                                       r0d);
-                            }
-                        } else {
-#pragma unroll 2
-                            for (int q = 0; q < kc; q++) {
-                                const double4 v = nd[q];
-                                far_node_f64<CK, false>(mm, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, a.k, k2r, k2i,
-                                                        r0d);
-                            }
+                        for (int q = 0; q < kc; q++) {
+                            const double4 y = rb.nd[q];
+                            far_node_f64<CK, true>(mm, x[0] - y.x, x[1] - y.y, x[2] - y.z, y.w, a.k, k2r, k2i, d);
                         }
-                        if (!CK) mm.finish_real_k();
-                        a1r += mm.a1r;
-                        a1i += mm.a1i;
-#pragma unroll
-                        for (int p = 0; p < 6; p++) {
-                            t[p][0] += mm.t[p][0];
-                            t[p][1] += mm.t[p][1];
+                    } else {
+#pragma unroll 2
+                        for (int q = 0; q < kc; q++) {
+                            const double4 y = rb.nd[q];
+                            far_node_f64<CK, false>(mm, x[0] - y.x, x[1] - y.y, x[2] - y.z, y.w, a.k, k2r, k2i, d);
                         }
                     }
                 }
-                if (k0 + kc == nn && far) {
-                    if constexpr (MIXED) {
-                        if constexpr (!CK) finish_real_k<F>(a1r, a1i, t);
-                        const float phr = (float)(P0r * kInvFourPi), phi = (float)(P0i * kInvFourPi);
-                        if constexpr (MARKS) {
-                            if (a.m == 2) write_block_f32<2>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2, cols);
-                            else write_block_f32<3>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2, cols);
-                        } else {
-                            if (a.m == 2) write_block_f32<2>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2);
-                            else write_block_f32<3>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2);
+                if constexpr (MIXED) {
+                    if constexpr (!CK) finish_real_k<float>(a1r, a1i, t);
+                } else {
+                    if (!CK) mm.finish_real_k();
+                    // K = (A1 I + T) * P0 / 4pi
+                    const int ti[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+#pragma unroll
+                    for (int p = 0; p < 3; p++)
+#pragma unroll
+                        for (int q = 0; q < 3; q++) {
+                            const double vr = mm.t[ti[p][q]][0] + (p == q ? mm.a1r : 0.);
+                            const double vi = mm.t[ti[p][q]][1] + (p == q ? mm.a1i : 0.);
+                            Kr[p][q] = (vr * P0r - vi * P0i) * kInvFourPi;
+                            Ki[p][q] = (vr * P0i + vi * P0r) * kInvFourPi;
                         }
-                    } else {
-                        // K = (A1 I + T) * P0 / 4pi
-                        const int ti[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
-                        double Kr[3][3], Ki[3][3];
-                        for (int p = 0; p < 3; p++)
-                            for (int q = 0; q < 3; q++) {
-                                double vr = (double)t[ti[p][q]][0] + (p == q ? (double)a1r : 0.);
-                                double vi = (double)t[ti[p][q]][1] + (p == q ? (double)a1i : 0.);
-                                Kr[p][q] = (vr * P0r - vi * P0i) * kInvFourPi;
-                                Ki[p][q] = (vr * P0i + vi * P0r) * kInvFourPi;
-                            }
-                        if constexpr (MARKS) write_block(a, i, c0 + cc, Kr, Ki, gi.t1, gi.t2, gj.t1, gj.t2, cols);
-                        else write_block(a, i, c0 + cc, Kr, Ki, gi.t1, gi.t2, gj.t1, gj.t2);
+                }
+            }
+            if constexpr (STAGE) {
+                const int g = cc & (group - 1);
+                // 16-byte pieces of matrix row r (0, 1) of this lane: complex64, piece g is the
+                // column cell's pair; complex128, pieces 2 g and 2 g + 1 its two entries
+                if constexpr (MIXED) {
+                    float o[2][2][2];
+                    block_f32<2>(a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2, o);
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        uint4* w = out + (r * 32 + lane) * 8;
+                        if (a.c64) {
+                            *reinterpret_cast<float4*>(w + ((g + lane) & 7)) =
+                                make_float4(o[r][0][0], o[r][0][1], o[r][1][0], o[r][1][1]);
+                        } else {
+#pragma unroll
+                            for (int b = 0; b < 2; b++)
+                                *reinterpret_cast<double2*>(w + ((2 * g + b + lane) & 7)) =
+                                    make_double2(o[r][b][0], o[r][b][1]);
+                        }
                     }
+                } else {
+                    double o[2][2][2] = {};
+                    if (any) block_f64<2>(Kr, Ki, gi.t1, gi.t2, gj.t1, gj.t2, o);
+#pragma unroll
+                    for (int r = 0; r < 2; r++) {
+                        uint4* w = out + (r * 32 + lane) * 8;
+                        if (a.c64) {
+                            *reinterpret_cast<float4*>(w + ((g + lane) & 7)) = make_float4(
+                                (float)o[r][0][0], (float)o[r][0][1], (float)o[r][1][0], (float)o[r][1][1]);
+                        } else {
+#pragma unroll
+                            for (int b = 0; b < 2; b++)
+                                *reinterpret_cast<double2*>(w + ((2 * g + b + lane) & 7)) =
+                                    make_double2(o[r][b][0], o[r][b][1]);
+                        }
+                    }
+                }
+                if (g == group - 1 || cc == nc - 1) {  // the group's columns, four matrix rows at a time
+                    __syncwarp();
+                    const int pieces = a.c64 ? g + 1 : 2 * (g + 1), piece = lane & 7;
+                    const size_t pitch = (size_t)2 * a.n_cells * (a.c64 ? 8 : 16);  // bytes of a matrix row
+                    char* base = (char*)a.A + (size_t)(c0 + cc - g) * (a.c64 ? 16 : 32) + 16 * piece;
+                    const int i0 = blockIdx.x * kAsmThreads + warp * 32;
+#pragma unroll 4
+                    for (int it = 0; it < 16; it++) {
+                        const int r = it >> 3, l = ((it & 7) << 2) + (lane >> 3);  // matrix row r of row cell i0 + l
+                        if (piece < pieces && i0 + l < a.n_cells)
+                            *reinterpret_cast<uint4*>(base + (size_t)(2 * (i0 + l) + r) * pitch) =
+                                out[(r * 32 + l) * 8 + ((piece + l) & 7)];
+                    }
+                    __syncwarp();
+                }
+            } else if (far) {
+                if constexpr (MIXED) {
+                    if (a.m == 2) write_block_f32<2>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2, cols);
+                    else write_block_f32<3>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2, cols);
+                } else {
+                    write_block(a, i, c0 + cc, Kr, Ki, gi.t1, gi.t2, gj.t1, gj.t2, cols);
                 }
             }
         }
+        if (split_cols) {
+            s_near[warp][lane] = nbits;
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll
+                for (int w = 1; w < kWarps; w++) nbits |= s_near[w][lane];
+            }
+        }
+        if (live && a.mask && (!split_cols || warp == 0)) a.mask[(size_t)(c0 >> 5) * a.n_cells + i] = nbits;
     }
 }
 
@@ -402,13 +458,13 @@ BIELCC_D void asm_pass_f64(Moments<double>& m, const double4* __restrict__ nd, i
     if (split) {
 #pragma unroll 8
         for (int q = 0; q < nn; q++) {
-            const double4 v = nd[q];
+            const double4 v = ldg_node(nd + q);
             far_node_f64<CK, true>(m, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, k, k2r, k2i, r0);
         }
     } else {
 #pragma unroll 8
         for (int q = 0; q < nn; q++) {
-            const double4 v = nd[q];
+            const double4 v = ldg_node(nd + q);
             far_node_f64<CK, false>(m, x[0] - v.x, x[1] - v.y, x[2] - v.z, v.w, k, k2r, k2i, r0);
         }
     }
@@ -436,50 +492,58 @@ BIELCC_D double asm_delta2(const Moments<double>& m0, const Moments<double>& m1,
     return d;
 }
 
-// STAGED: the CTA stages each column cell's two node rows in shared memory
-// ((nn_lo + nn) double4, dynamic); otherwise every thread reads them from
-// global memory (rows too long to stage).
-template <bool STAGED>
-__global__ void asm_refine_decide_kernel(AsmArgs a, const double4* __restrict__ lo, int nn_lo, double eps2,
+// Each pass takes the shortest row its table's rules allow (rules.cu, FP64 limits).
+__global__ void asm_refine_decide_kernel(const __grid_constant__ AsmArgs a, const __grid_constant__ FarRules rules_lo,
+                                         const double4* __restrict__ lo, int nn_lo, double eps2,
                                          unsigned* __restrict__ mark) {
-    extern __shared__ double4 s_rows[];
+    __shared__ RuleTab<double4> s_lo, s_hi;
+    __shared__ float s_rmin[2][kAsmStageCells][kMaxRules];
     const int i = blockIdx.x * kAsmThreads + threadIdx.x;
     const bool live = i < a.n_cells;
-    if (!STAGED && !live) return;
     const CellGeo gi = a.geo[live ? i : 0];
     const double* x = gi.c;
-    const int cb = blockIdx.y * a.cols_per_split;
+    const int cb = blockIdx.y * a.cols_per_split;  // a multiple of 32
     const int ce = min(a.n_cells, cb + a.cols_per_split);
     const bool ck = a.k.im != 0.0;
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
     const size_t plane = (size_t)((a.n_cells + 31) >> 5) * a.n_cells;
+    const int nlo = rules_lo.n_lev, nhi = a.rules.n_lev;
+    if (threadIdx.x == 0) {
+        s_lo.fill(rules_lo, rules_lo.n64, lo, nn_lo, a.n_cells);
+        s_hi.fill(a.rules, a.rules.n64, a.nodes64, a.nn, a.n_cells);
+    }
     unsigned nbits = 0, mb[3] = {0u, 0u, 0u};
     for (int j = cb; j < ce; j++) {
-        const double4* row_lo = lo + (size_t)j * nn_lo;
-        const double4* row_hi = a.nodes64 + (size_t)j * a.nn;
-        if constexpr (STAGED) {
-            __syncthreads();  // the previous column's rows are no longer read
-            for (int q = threadIdx.x; q < nn_lo; q += kAsmThreads) s_rows[q] = row_lo[q];
-            for (int q = threadIdx.x; q < a.nn; q += kAsmThreads) s_rows[nn_lo + q] = row_hi[q];
+        if ((j & 31) == 0) {
+            const int nc = min(kAsmStageCells, ce - j);
+            const float kabs = rule_kabs(a.k);
+            __syncthreads();  // the previous columns' limits are no longer read
+            for (int q = threadIdx.x; q < nc * nlo; q += kAsmThreads)
+                s_rmin[0][q / nlo][q % nlo] = rule_rmin(rules_lo.thr64[(size_t)j * nlo + q], kabs);
+            for (int q = threadIdx.x; q < nc * nhi; q += kAsmThreads)
+                s_rmin[1][q / nhi][q % nhi] = rule_rmin(a.rules.thr64[(size_t)j * nhi + q], kabs);
             __syncthreads();
-            row_lo = s_rows;
-            row_hi = s_rows + nn_lo;
-            if (!live) continue;  // after the barriers: every thread stages
         }
         const CellGeo& gj = a.geo[j];
         double d;
         const bool nr = asm_is_near(x, gj, a.analytic_calc, &d);
-        if (!nr) {
+        const bool far = live && !nr;
+        const float dmin = warp_min_pos(rule_key(far, d));
+        const int llo = rule_level(s_rmin[0][j & 31], nlo, dmin), lhi = rule_level(s_rmin[1][j & 31], nhi, dmin);
+        if (far) {
+            const int n_lo = s_lo.cnt[llo], n_hi = s_hi.cnt[lhi];
+            const double4* row_lo = s_lo.base[llo] + (size_t)j * n_lo;
+            const double4* row_hi = s_hi.base[lhi] + (size_t)j * n_hi;
             const bool split = !ck && fabs(a.k.re) * (double)a.rho32[j] * (1.0 + 1e-6) <= 0.5;
             double pr = 1.0, pi = 0.0;
             if (split) sincos(a.k.re * d, &pi, &pr);
             Moments<double> m0, m1;
             if (ck) {
-                asm_pass_f64<true>(m0, row_lo, nn_lo, x, a.k, k2r, k2i, d, false);
-                asm_pass_f64<true>(m1, row_hi, a.nn, x, a.k, k2r, k2i, d, false);
+                asm_pass_f64<true>(m0, row_lo, n_lo, x, a.k, k2r, k2i, d, false);
+                asm_pass_f64<true>(m1, row_hi, n_hi, x, a.k, k2r, k2i, d, false);
             } else {
-                asm_pass_f64<false>(m0, row_lo, nn_lo, x, a.k, k2r, k2i, d, split);
-                asm_pass_f64<false>(m1, row_hi, a.nn, x, a.k, k2r, k2i, d, split);
+                asm_pass_f64<false>(m0, row_lo, n_lo, x, a.k, k2r, k2i, d, split);
+                asm_pass_f64<false>(m1, row_hi, n_hi, x, a.k, k2r, k2i, d, split);
             }
             for (int b = 0; b < a.m; b++) {
                 double J[3];
@@ -490,8 +554,10 @@ __global__ void asm_refine_decide_kernel(AsmArgs a, const double4* __restrict__ 
         nbits |= (nr ? 1u : 0u) << (j & 31);
         if ((j & 31) == 31 || j == ce - 1) {
             const size_t wi = (size_t)(j >> 5) * a.n_cells + i;
-            if (a.mask) a.mask[wi] = nbits;
-            for (int b = 0; b < a.m; b++) mark[b * plane + wi] = mb[b];
+            if (live) {
+                if (a.mask) a.mask[wi] = nbits;
+                for (int b = 0; b < a.m; b++) mark[b * plane + wi] = mb[b];
+            }
             nbits = 0;
             mb[0] = mb[1] = mb[2] = 0u;
         }
@@ -754,9 +820,11 @@ static AsmArgs make_args(const AssembleLaunch& a) {
     g.nodes64 = m.nodes64;
     g.nodes32 = m.nodes32;
     g.rho32 = m.rho32;
+    g.rules = m.rules;
     g.nn = far_split_n(a.np) * far_split_n(a.np);
     g.k = a.k;
     g.analytic_calc = a.np.analytic_calc;
+    g.ways = 1;
     g.m = a.layout == 1 ? 3 : 2;
     g.c64 = a.out_c64;
     g.A = a.A;
@@ -765,19 +833,20 @@ static AsmArgs make_args(const AssembleLaunch& a) {
 }
 
 // Resident CTAs (whole GPU) of the far assembly kernel variant.
-static int asm_slots(bool ck, bool mixed) {
-    static std::atomic<int> cache[2][2];
-    std::atomic<int>& c = cache[ck][mixed];
+static int asm_slots(bool ck, bool mixed, bool stage) {
+    static std::atomic<int> cache[2][2][2];
+    std::atomic<int>& c = cache[ck][mixed][stage];
     int v = c.load(std::memory_order_relaxed);
     if (v) return v;
     int dev = 0, sms = 148, per = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const void* fn = ck ? (mixed ? (const void*)assemble_far_kernel<true, true>
-                                 : (const void*)assemble_far_kernel<true, false>)
-                        : (mixed ? (const void*)assemble_far_kernel<false, true>
-                                 : (const void*)assemble_far_kernel<false, false>);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kAsmThreads, 0);
+#define BIELCC_AK(C, M) \
+    (stage ? (const void*)assemble_far_kernel<C, M, false, true> : (const void*)assemble_far_kernel<C, M, false, false>)
+    const void* fn = ck ? (mixed ? BIELCC_AK(true, true) : BIELCC_AK(true, false))
+                        : (mixed ? BIELCC_AK(false, true) : BIELCC_AK(false, false));
+#undef BIELCC_AK
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kAsmThreads, stage ? kAsmOutBytes : 0);
     v = std::max(1, sms * std::max(1, per));
     c.store(v, std::memory_order_relaxed);
     return v;
@@ -801,19 +870,23 @@ cudaError_t assemble_stage1(const AssembleLaunch& a, void* ws, long long* d_tota
         return cudaErrorInvalidValue;  // no n_start table for the convergence test
     if (far_third_pass(a.np) && (m.table_hi_n != 4 * a.np.n_start || !m.nodes64_hi))
         return cudaErrorInvalidValue;  // no 4 n_start tables for the third pass
-    int splits = choose_cell_splits(tiles, N, asm_slots(ck, a.precision == 1), N);
+    // staged blocks are written 16 bytes at a time: a complex64 matrix may start
+    // between 16-byte boundaries, which the direct writes take
+    const bool stage = g.m == 2 && !far_adaptive(a.np) && (reinterpret_cast<uintptr_t>(a.A) & 15) == 0;
+    const int slots = asm_slots(ck, a.precision == 1, stage);
+    // fewer 128-row CTAs than slots at one mask word (32 columns) per split: the
+    // warps share the columns (not under the marks of p_max >= 3, whose decision
+    // kernel sets the grid)
+    g.ways = !far_adaptive(a.np) && (size_t)tiles * n_words < (size_t)slots ? kAsmWays : 1;
+    const int far_tiles = g.ways > 1 ? (N + 31) / 32 : tiles;
+    const int splits = choose_cell_splits(far_tiles, N, slots, N);
     g.cols_per_split = round_cells_per_split(N, splits);
-    dim3 grid(tiles, splits);
+    const dim3 grid(far_tiles, splits);
     if (far_adaptive(a.np)) {
         unsigned* mark = (unsigned*)((char*)mask + al256((size_t)n_words * N * sizeof(unsigned)) + 256);
         const int nn_lo = a.np.n_start * a.np.n_start;
-        const size_t rows = (size_t)(nn_lo + g.nn) * sizeof(double4);
-        if (rows <= 48 * 1024)
-            asm_refine_decide_kernel<true><<<grid, kAsmThreads, rows, s>>>(g, m.nodes64_lo, nn_lo, a.np.eps * a.np.eps,
-                                                                           mark);
-        else
-            asm_refine_decide_kernel<false><<<grid, kAsmThreads, 0, s>>>(g, m.nodes64_lo, nn_lo, a.np.eps * a.np.eps,
-                                                                         mark);
+        asm_refine_decide_kernel<<<grid, kAsmThreads, 0, s>>>(g, m.rules_lo, m.nodes64_lo, nn_lo,
+                                                              a.np.eps * a.np.eps, mark);
         AsmArgsMarks gm;
         static_cast<AsmArgs&>(gm) = g;
         gm.mask = nullptr;  // written by the decision kernel
@@ -830,6 +903,7 @@ cudaError_t assemble_stage1(const AssembleLaunch& a, void* ws, long long* d_tota
             gm.nodes64 = m.nodes64_hi;
             gm.nodes32 = m.nodes32_hi;
             gm.rho32 = m.rho32_hi;
+            gm.rules = m.rules_hi;
             gm.nn = 16 * a.np.n_start * a.np.n_start;
             gm.take_marked = 1;
             if (a.precision == 1) {
@@ -843,6 +917,14 @@ cudaError_t assemble_stage1(const AssembleLaunch& a, void* ws, long long* d_tota
             DNP np{a.np.eps, a.np.rs, a.np.rs_seg, a.np.analytic_calc, a.np.n_start, a.np.n_start_seg, a.np.p_max,
                    a.np.p_max_seg};
             assemble_far_refine_kernel<<<grid, kAsmThreads, 0, s>>>(g, mark, m.verts, m.nv, np);
+        }
+    } else if (stage && g.ways == 1) {
+        if (a.precision == 1) {
+            if (ck) assemble_far_kernel<true, true, false, true><<<grid, kAsmThreads, kAsmOutBytes, s>>>(g);
+            else assemble_far_kernel<false, true, false, true><<<grid, kAsmThreads, kAsmOutBytes, s>>>(g);
+        } else {
+            if (ck) assemble_far_kernel<true, false, false, true><<<grid, kAsmThreads, kAsmOutBytes, s>>>(g);
+            else assemble_far_kernel<false, false, false, true><<<grid, kAsmThreads, kAsmOutBytes, s>>>(g);
         }
     } else if (a.precision == 1) {
         if (ck) assemble_far_kernel<true, true><<<grid, kAsmThreads, 0, s>>>(g);
