@@ -130,7 +130,7 @@ BIELCC_D void write_block_m(const AsmArgs& a, int i, int j, const double (&Kr)[3
 // (M = 3), times ph = e^{ik r0} / 4pi.
 template <int M>
 BIELCC_D void block_f32(float a1r, float a1i, const float (&t)[6][2], float phr, float phi, const float (&ti)[2][3],
-                        const double* tj1, const double* tj2, float (&out)[M][M][2]) {
+                        const float* tj1, const float* tj2, float (&out)[M][M][2]) {
     const int sym[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
     float kr[6], ki[6];
 #pragma unroll
@@ -148,8 +148,7 @@ BIELCC_D void block_f32(float a1r, float a1i, const float (&t)[6][2], float phr,
                 out[p][q][1] = kr[sym[p][q]] * phi + ki[sym[p][q]] * phr;
             }
     } else {
-        const float tb[2][3] = {{(float)tj1[0], (float)tj1[1], (float)tj1[2]},
-                                {(float)tj2[0], (float)tj2[1], (float)tj2[2]}};
+        const float tb[2][3] = {{tj1[0], tj1[1], tj1[2]}, {tj2[0], tj2[1], tj2[2]}};
 #pragma unroll
         for (int b = 0; b < 2; b++) {
             float ur[3], ui[3];
@@ -171,7 +170,7 @@ BIELCC_D void block_f32(float a1r, float a1i, const float (&t)[6][2], float phr,
 
 template <int M>
 BIELCC_D void write_block_f32(const AsmArgs& a, int i, int j, float a1r, float a1i, const float (&t)[6][2], float phr,
-                              float phi, const float (&ti)[2][3], const double* tj1, const double* tj2,
+                              float phi, const float (&ti)[2][3], const float* tj1, const float* tj2,
                               unsigned cols = ~0u) {
     float out[M][M][2];
     block_f32<M>(a1r, a1i, t, phr, phi, ti, tj1, tj2, out);
@@ -213,7 +212,8 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
     static_assert(kWarps == kAsmWays, "ways = 4 gives every warp its share of the columns");
     __shared__ __align__(16) RowBuf<NodeT> s_rows[kWarps];
     __shared__ RuleTab<NodeT> s_tab;
-    __shared__ CellGeo s_geo[kAsmStageCells];
+    using F = typename std::conditional<MIXED, float, double>::type;
+    __shared__ F s_tau[kAsmStageCells][6];      // the column cells' tangents
     __shared__ double4 s_cell[kAsmStageCells];  // centre, near square
     __shared__ int s_mode[kAsmStageCells];      // mixed: phase polynomial; FP64: 1 phase split, 0 sincos per node
     __shared__ float s_rmin[kAsmStageCells][kMaxRules];
@@ -255,8 +255,10 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
         const int nc = min(kAsmStageCells, ce - c0);
         unsigned nbits = 0;  // near bits of this 32-column word
         __syncthreads();
-        for (int q = threadIdx.x; q < nc * 16; q += kAsmThreads)
-            reinterpret_cast<double*>(s_geo)[q] = reinterpret_cast<const double*>(a.geo + c0)[q];
+        for (int q = threadIdx.x; q < nc * 6; q += kAsmThreads) {
+            const CellGeo& gg = a.geo[c0 + q / 6];
+            s_tau[q / 6][q % 6] = (F)(q % 6 < 3 ? gg.t1[q % 6] : gg.t2[q % 6 - 3]);
+        }
         for (int q = threadIdx.x; q < nc; q += kAsmThreads) {
             s_cell[q] = near_cell(a.geo[c0 + q], a.analytic_calc);
             if constexpr (MIXED) s_mode[q] = phase_mode((float)fabs(a.k.re) * a.rho32[c0 + q]);
@@ -288,7 +290,7 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
             }
             const float dmin = warp_min_pos(rule_key(far, d));
             const bool any = dmin < __int_as_float(0x7f800000);
-            const CellGeo& gj = s_geo[cc];
+            const F *tj1 = s_tau[cc], *tj2 = s_tau[cc] + 3;
             double Kr[3][3], Ki[3][3];     // FP64 form: the operator matrix
             float a1r = 0, a1i = 0, t[6][2], phr = 0, phi = 0;  // mixed form: moments and phase / 4pi
 #pragma unroll
@@ -369,7 +371,7 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                 // column cell's pair; complex128, pieces 2 g and 2 g + 1 its two entries
                 if constexpr (MIXED) {
                     float o[2][2][2];
-                    block_f32<2>(a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2, o);
+                    block_f32<2>(a1r, a1i, t, phr, phi, tif, tj1, tj2, o);
 #pragma unroll
                     for (int r = 0; r < 2; r++) {
                         uint4* w = out + (r * 32 + lane) * 8;
@@ -385,7 +387,7 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                     }
                 } else {
                     double o[2][2][2] = {};
-                    if (any) block_f64<2>(Kr, Ki, gi.t1, gi.t2, gj.t1, gj.t2, o);
+                    if (any) block_f64<2>(Kr, Ki, gi.t1, gi.t2, tj1, tj2, o);
 #pragma unroll
                     for (int r = 0; r < 2; r++) {
                         uint4* w = out + (r * 32 + lane) * 8;
@@ -417,10 +419,10 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                 }
             } else if (far) {
                 if constexpr (MIXED) {
-                    if (a.m == 2) write_block_f32<2>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2, cols);
-                    else write_block_f32<3>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, gj.t1, gj.t2, cols);
+                    if (a.m == 2) write_block_f32<2>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, tj1, tj2, cols);
+                    else write_block_f32<3>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, tj1, tj2, cols);
                 } else {
-                    write_block(a, i, c0 + cc, Kr, Ki, gi.t1, gi.t2, gj.t1, gj.t2, cols);
+                    write_block(a, i, c0 + cc, Kr, Ki, gi.t1, gi.t2, tj1, tj2, cols);
                 }
             }
         }
@@ -694,19 +696,28 @@ BIELCC_D void near_operator(const DCell& cl, const double* x, cplx k, const DNP&
 }
 
 // Near entries: K_RotRot_HS_Colloc as a 3x3 operator, FP64.
+template <int G>
 __global__ void asm_near_kernel(AsmArgs a, const double* __restrict__ verts, int nv, const int* __restrict__ pr,
                                 const int* __restrict__ pc, long long n_pairs, DNP np) {
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_pairs) return;
+    const Lanes<G> g = Lanes<G>::make();
+    const long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
+    if (q >= n_pairs) return;  // whole groups
     int i = pr[q], j = pc[q];
-    const CellGeo gi = a.geo[i], gj = a.geo[j];
+    const CellGeo &gi = a.geo[i], &gj = a.geo[j];
     DCell cl;
     cl.nv = nv;
     for (int v = 0; v < nv; v++)
-        for (int g = 0; g < 3; g++) cl.v[v][g] = verts[((size_t)j * nv + v) * 3 + g];
-    const double* x = gi.c;
+        for (int h = 0; h < 3; h++) cl.v[v][h] = verts[((size_t)j * nv + v) * 3 + h];
+    const double x[3] = {gi.c[0], gi.c[1], gi.c[2]};
+    cplx K[3][3];
+    group_hs_colloc<G>(g, x, cl, a.k, np, K);
+    if (g.l != 0) return;
     double Kr[3][3], Ki[3][3];
-    near_operator(cl, x, a.k, np, Kr, Ki);
+    for (int p = 0; p < 3; p++)
+        for (int r = 0; r < 3; r++) {
+            Kr[p][r] = K[p][r].re;
+            Ki[p][r] = K[p][r].im;
+        }
     write_block(a, i, j, Kr, Ki, gi.t1, gi.t2, gj.t1, gj.t2);
 }
 
@@ -733,6 +744,31 @@ __global__ void asm_error_sample_kernel(AsmArgs a, const double* __restrict__ ve
         double Kr[3][3], Ki[3][3];
         if (asm_is_near(x, gj, a.analytic_calc, &d)) {
             near_operator(cl, x, a.k, np, Kr, Ki);
+        } else if (np.p_max <= 2) {
+            // one FP64 pass over the shortest row of the far pass's table that this pair
+            // allows (p_max = 2: the pass at 2 n_start): 20,480 triangles, 16 rows,
+            // 2.46 ms with K_far_dev per column
+            const int nl = a.rules.n_lev;
+            float rmin[kMaxRules];
+            for (int l = 0; l < nl; l++) rmin[l] = rule_rmin(a.rules.thr64[(size_t)j * nl + l], rule_kabs(a.k));
+            const int l = rule_level(rmin, nl, rule_key(true, d));
+            const int cnt = l < nl ? a.rules.cnt[l] : a.nn;
+            const double4* row = (l < nl ? a.rules.n64 + (size_t)a.rules.off[l] * N : a.nodes64) + (size_t)j * cnt;
+            const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
+            const bool split = a.k.im == 0. && fabs(a.k.re) * (double)a.rho32[j] * (1.0 + 1e-6) <= 0.5;
+            double pr = 1., pi = 0.;
+            if (split) sincos(a.k.re * d, &pi, &pr);
+            Moments<double> mm;
+            if (a.k.im != 0.) asm_pass_f64<true>(mm, row, cnt, x, a.k, k2r, k2i, d, false);
+            else asm_pass_f64<false>(mm, row, cnt, x, a.k, k2r, k2i, d, split);
+            const int ti[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+            for (int p = 0; p < 3; p++)
+                for (int r = 0; r < 3; r++) {
+                    const cplx v = mk(mm.t[ti[p][r]][0] + (p == r ? mm.a1r : 0.), mm.t[ti[p][r]][1] + (p == r ? mm.a1i : 0.)) *
+                                   mk(pr, pi) * kInvFourPi;
+                    Kr[p][r] = v.re;
+                    Ki[p][r] = v.im;
+                }
         } else {
             for (int b = 0; b < 3; b++) {  // K_RotRot_Far is linear in the current: one column per basis vector
                 cplx e[3] = {mk(b == 0, 0.), mk(b == 1, 0.), mk(b == 2, 0.)}, col[3];
@@ -955,7 +991,9 @@ cudaError_t assemble_stage2(const AssembleLaunch& a, void* ws, long long n_near,
     AsmArgs g = make_args(a);
     DNP np{a.np.eps, a.np.rs, a.np.rs_seg, a.np.analytic_calc, a.np.n_start, a.np.n_start_seg, a.np.p_max,
            a.np.p_max_seg};
-    asm_near_kernel<<<(int)((n_near + 127) / 128), 128, 0, s>>>(g, m.verts, m.nv, pr, pc, n_near, np);
+    const int lanes = near_lanes(n_near), blocks = (int)((n_near * lanes + 127) / 128);
+    const auto near_blocks = lanes == 1 ? asm_near_kernel<1> : (lanes == 8 ? asm_near_kernel<8> : asm_near_kernel<32>);
+    near_blocks<<<blocks, 128, 0, s>>>(g, m.verts, m.nv, pr, pc, n_near, np);
     return cudaGetLastError();
 }
 

@@ -1277,7 +1277,7 @@ __global__ void batch_near_fill_kernel(const JobDev* __restrict__ jobs, const in
 __global__ void batch_near_pair_kernel(const JobDev* __restrict__ jobs, const int* __restrict__ pt_job,
                                        const int* __restrict__ pair_cell, const int* __restrict__ pair_gpt,
                                        long long n_pairs, DNP np, cplx* __restrict__ out) {
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n_pairs) return;
     const int g = pair_gpt[q], c = pair_cell[q];
     const JobDev& jb = jobs[pt_job[g]];
@@ -1287,7 +1287,7 @@ __global__ void batch_near_pair_kernel(const JobDev* __restrict__ jobs, const in
     for (int v = 0; v < jb.nv; v++)
         for (int a = 0; a < 3; a++) cl.v[v][a] = jb.verts[((size_t)c * jb.nv + v) * 3 + a];
     double x[3] = {jb.pts[3 * (size_t)p], jb.pts[3 * (size_t)p + 1], jb.pts[3 * (size_t)p + 2]};
-    near_pair_moments(x, cl, jb.k, np, out + q * 13);
+    near_pair_moments<1>(Lanes<1>::make(), x, cl, jb.k, np, out + q * 13);
 }
 
 // E and H of one (point, RHS): partial sums over the ranges in order, the

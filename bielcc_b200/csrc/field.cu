@@ -24,7 +24,7 @@
 //   2. near count + scan + fill — per point, the cells with
 //                     |x - centre| < analytic_calc * diam (get_field.h:58), in
 //                     cell order.
-//   3. near pair kernel — FP64, one pair per thread: the J-independent parts of
+//   3. near pair kernel — FP64, a group of lanes per pair: the J-independent parts of
 //                     K_RotRot_Near_Smooth (K.h:47-79) and R_Rot_Smooth
 //                     (R.h:46-61) with the reference's adaptive quadrature.
 //   4. near sums    — one warp per (point, RHS): the point's near pairs
@@ -725,19 +725,21 @@ __global__ void near_fill_kernel(const unsigned* __restrict__ mask, int n_words,
 }
 
 // Near pair: the J-independent parts of K_RotRot_Near_Smooth and R_Rot_Smooth
-// (near_pair_moments, ops.cuh), one pair per thread.
+// (near_pair_moments, ops.cuh), one pair per group of G lanes.
+template <int G>
 __global__ void near_pair_kernel(const double* __restrict__ pts, const double* __restrict__ verts, int nv,
                                  const int* __restrict__ pair_cell, const int* __restrict__ pair_pt, long long n_pairs,
                                  cplx k, DNP np, cplx* __restrict__ out) {
-    long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_pairs) return;
+    const Lanes<G> g = Lanes<G>::make();
+    const long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
+    if (q >= n_pairs) return;  // whole groups
     int c = pair_cell[q], p = pair_pt[q];
     DCell cl;
     cl.nv = nv;
     for (int v = 0; v < nv; v++)
-        for (int g = 0; g < 3; g++) cl.v[v][g] = verts[((size_t)c * nv + v) * 3 + g];
+        for (int h = 0; h < 3; h++) cl.v[v][h] = verts[((size_t)c * nv + v) * 3 + h];
     double x[3] = {pts[3 * (size_t)p], pts[3 * (size_t)p + 1], pts[3 * (size_t)p + 2]};
-    near_pair_moments(x, cl, k, np, out + q * 13);
+    near_pair_moments<G>(g, x, cl, k, np, out + q * 13);
 }
 
 // Near pairs of a point contracted with one RHS: one warp per (point, RHS).
@@ -1130,8 +1132,9 @@ cudaError_t field_stage2(const FieldLaunch& f, void* ws, int splits, long long n
         near_fill_kernel<<<(f.n_pts + 7) / 8, 256, 0, s>>>(mask, n_words, f.n_pts, offs, pair_cell, pair_pt);
         DNP np{f.np.eps, f.np.rs, f.np.rs_seg, f.np.analytic_calc, f.np.n_start, f.np.n_start_seg, f.np.p_max,
                f.np.p_max_seg};
-        int blocks = (int)((n_near + 127) / 128);
-        near_pair_kernel<<<blocks, 128, 0, s>>>(f.pts, m.verts, m.nv, pair_cell, pair_pt, n_near, f.k, np, moments);
+        const int lanes = near_lanes(n_near), blocks = (int)((n_near * lanes + 127) / 128);
+        const auto near_pairs = lanes == 1 ? near_pair_kernel<1> : (lanes == 8 ? near_pair_kernel<8> : near_pair_kernel<32>);
+        near_pairs<<<blocks, 128, 0, s>>>(f.pts, m.verts, m.nv, pair_cell, pair_pt, n_near, f.k, np, moments);
         near_sum_kernel<<<dim3((f.n_pts + 7) / 8, f.n_rhs), 256, 0, s>>>(
             offs, pair_cell, moments, reinterpret_cast<const cplx*>(f.J), f.n_pts, m.n_cells, near);
         *launches += 3;

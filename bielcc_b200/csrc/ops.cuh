@@ -366,55 +366,6 @@ BIELCC_D void integral_cell(int id, const double* x, const DCell& c, DKP& kp, in
     else integral_tri<T>(id, x, c.v, kp, idim, n_start, p_max, eps, res);
 }
 
-// One pass (p_max = 1) of IntegralUniversalPnt for F_SimplePot_H (F) and
-// F_GradSimplePot_H (G) over one cell with the same smoothing radius: the
-// nodes, weights and accumulation order of integral_quad / integral_tri, with
-// each node evaluated once for both integrands.
-BIELCC_D void integral_cell_pot_and_grad(const double* x, const DCell& c, const DKP& kp, int n, cplx* F, cplx* G) {
-    F[0] = mk(0, 0);
-    for (int g = 0; g < 3; g++) G[g] = mk(0, 0);
-    cplx f[1], gg[3];
-    if (c.nv == 4) {
-        for (int i = 0; i < n; i++)
-            for (int j = 0; j < n; j++) {
-                double y[3], s;
-                quad_node(c.v, i, j, n, y, &s);
-                eval_pot_and_grad(x, y, kp, f, gg);
-                F[0] = madd(F[0], f[0], s);
-                for (int g = 0; g < 3; g++) G[g] = madd(G[g], gg[g], s);
-            }
-        return;
-    }
-    const double(*cv)[3] = c.v;
-    double area = tri_area(cv[0], cv[1], cv[2]);
-    double pv[3], qv[3], rv[3];
-    for (int k = 0; k < 3; k++) {
-        pv[k] = (cv[1][k] - cv[0][k]) / n;
-        qv[k] = (cv[2][k] - cv[0][k]) / n;
-        rv[k] = (cv[2][k] - cv[1][k]) / n;
-    }
-    for (int i = 0; i < n; i++)
-        for (int j = 0; j < n - i; j++) {
-            double B[3], y[3];
-            for (int k = 0; k < 3; k++) {
-                B[k] = cv[0][k] + (i + 1) * pv[k] + j * qv[k];
-                double A = B[k] - pv[k];
-                y[k] = (B[k] + A + (A + qv[k])) / 3.0;
-            }
-            eval_pot_and_grad(x, y, kp, f, gg);
-            F[0] = madd(F[0], f[0], 1.0);
-            for (int g = 0; g < 3; g++) G[g] = madd(G[g], gg[g], 1.0);
-            if (j < n - 1 - i) {
-                for (int k = 0; k < 3; k++) y[k] = (B[k] + (B[k] + rv[k]) + (B[k] + qv[k])) / 3.0;
-                eval_pot_and_grad(x, y, kp, f, gg);
-                F[0] = madd(F[0], f[0], 1.0);
-                for (int g = 0; g < 3; g++) G[g] = madd(G[g], gg[g], 1.0);
-            }
-        }
-    F[0] = F[0] * area / (double)n / (double)n;
-    for (int g = 0; g < 3; g++) G[g] = G[g] * area / (double)n / (double)n;
-}
-
 // IntegralUniversalSegPnt (integral_universal_seg.h:38-98).
 template <typename T>
 BIELCC_D void integral_seg(int id, const double* a, const double* b, const double* x, DKP& kp, int idim, int n_start,
@@ -487,26 +438,27 @@ BIELCC_D void K0_common_dev(int id, const double* x, const DCell& c, DKP& kp, in
 //   sum_e P0 ln((R+ + l+)/(R- + l-)) - |h| sum_e [atan(P0 l+ / (R0^2 + |h| R+))
 //                                             - atan(P0 l- / (R0^2 + |h| R-))]
 // Same value as integral1Divr (integrators/integrals_analytic.cpp:37-235).
-BIELCC_D double int_1divr_tri(const double* P1, const double* P2, const double* P3, const double* x) {
-    const double* P[3] = {P1, P2, P3};
-    double e1[3], e2[3], nrm[3];
-    for (int i = 0; i < 3; i++) { e1[i] = P2[i] - P1[i]; e2[i] = P3[i] - P1[i]; }
-    cross3(e1, e2, nrm);
-    double nl = len3(nrm);
-    // zero-area triangle (collapsed half of a pole quad): the integral vanishes;
-    // relative test because e1 x e1 is rounding noise under FMA contraction
-    if (!(nl > 1e-13 * len3(e1) * len3(e2))) return 0.;
-    for (int i = 0; i < 3; i++) nrm[i] /= nl;
-    double w[3] = {x[0] - P1[0], x[1] - P1[1], x[2] - P1[2]};
-    double h = dot3(w, nrm), ah = fabs(h);
-    double rho[3] = {x[0] - h * nrm[0], x[1] - h * nrm[1], x[2] - h * nrm[2]};
-    double sum = 0.;
-    for (int e = 0; e < 3; e++) {
-        const double* A = P[e];
-        const double* B = P[(e + 1) % 3];
+struct InvRTri {  // plane of the triangle as seen from x
+    double nrm[3], rho[3], h, ah;
+    // false: a zero-area triangle (collapsed half of a pole quad), whose integral
+    // vanishes; relative test because e1 x e1 is rounding noise under FMA contraction
+    BIELCC_D bool set(const double* P1, const double* P2, const double* P3, const double* x) {
+        double e1[3], e2[3];
+        for (int i = 0; i < 3; i++) { e1[i] = P2[i] - P1[i]; e2[i] = P3[i] - P1[i]; }
+        cross3(e1, e2, nrm);
+        double nl = len3(nrm);
+        if (!(nl > 1e-13 * len3(e1) * len3(e2))) return false;
+        for (int i = 0; i < 3; i++) nrm[i] /= nl;
+        double w[3] = {x[0] - P1[0], x[1] - P1[1], x[2] - P1[2]};
+        h = dot3(w, nrm);
+        ah = fabs(h);
+        for (int i = 0; i < 3; i++) rho[i] = x[i] - h * nrm[i];
+        return true;
+    }
+    BIELCC_D double edge(const double* A, const double* B, const double* x) const {
         double lv[3] = {B[0] - A[0], B[1] - A[1], B[2] - A[2]};
         double L = len3(lv);
-        if (!(L > 0)) continue;
+        if (!(L > 0)) return 0.;
         for (int i = 0; i < 3; i++) lv[i] /= L;
         double u[3];
         cross3(lv, nrm, u);
@@ -515,12 +467,21 @@ BIELCC_D double int_1divr_tri(const double* P1, const double* P2, const double* 
         double P0 = dot3(am, u), lm = dot3(am, lv), lp = dot3(bm, lv);
         double Rm = dist3(x, A), Rp = dist3(x, B);
         double R02 = P0 * P0 + h * h;
+        double sum = 0.;
         if (fabs(P0) > 1e-14 * (L + Rm + Rp)) {
             double num = Rp + lp, den = Rm + lm;
             if (num > 0 && den > 0) sum += P0 * log(num / den);
             sum -= ah * (atan2(P0 * lp, R02 + ah * Rp) - atan2(P0 * lm, R02 + ah * Rm));
         }
+        return sum;
     }
+};
+BIELCC_D double int_1divr_tri(const double* P1, const double* P2, const double* P3, const double* x) {
+    InvRTri t;
+    if (!t.set(P1, P2, P3, x)) return 0.;
+    const double* P[3] = {P1, P2, P3};
+    double sum = 0.;
+    for (int e = 0; e < 3; e++) sum += t.edge(P[e], P[(e + 1) % 3], x);
     return sum;
 }
 // integral1Divr (integrals_analytic.cpp:218-235): quad = triangles 012 + 230
@@ -725,12 +686,157 @@ BIELCC_D void R_near_dev(const cplx* j, const double* x, const DCell& c, const D
     ccross_cc(j, t, res);
 }
 
+// ------------------------------------------------------------------ near pairs, a group of lanes per pair
+// The near operators' quadratures with the nodes of every pass spread over G lanes
+// of a warp (G a power of two, groups aligned): lane l takes nodes l, l + G, ...,
+// a fixed xor butterfly adds the lanes' sums, and every lane of the group holds
+// the same values after it, so the group follows the reference's refinement loop
+// together. One thread per pair ran 64 surface and 40 edge nodes in series, and a
+// few thousand pairs (3 passes: up to 1024 nodes) left most of the GPU idle.
+template <int G>
+struct Lanes {
+    int l;          // lane in the group
+    unsigned mask;  // the group's lanes of the warp
+    BIELCC_D static Lanes make() {
+        const int lane = threadIdx.x & 31;
+        return {lane & (G - 1), (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane & ~(G - 1) & 31))};
+    }
+    BIELCC_D double sum(double v) const {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+    BIELCC_D cplx sum(cplx v) const { return {sum(v.re), sum(v.im)}; }
+};
+
+// Calls f(y, weight) for this lane's nodes of the n x n split; triangles: weight 1
+// (the sum is scaled by area / n / n, cell_scale). Nodes as integral_quad / integral_tri.
+template <int G, typename Fn>
+BIELCC_D void cell_nodes(const Lanes<G>& g, const DCell& c, int n, Fn f) {
+    double y[3], s;
+    if (c.nv == 4) {
+        for (int q = g.l; q < n * n; q += G) {
+            quad_node(c.v, q / n, q % n, n, y, &s);
+            f(y, s);
+        }
+        return;
+    }
+    double pv[3], qv[3], rv[3];
+    for (int k = 0; k < 3; k++) {
+        pv[k] = (c.v[1][k] - c.v[0][k]) / n;
+        qv[k] = (c.v[2][k] - c.v[0][k]) / n;
+        rv[k] = (c.v[2][k] - c.v[1][k]) / n;
+    }
+    int i = 0, first = 0;  // row of the node (2 (n - i) - 1 of them) and its first node
+    for (int q = g.l; q < n * n; q += G) {
+        while (q >= first + 2 * (n - i) - 1) {
+            first += 2 * (n - i) - 1;
+            i++;
+        }
+        const int j = (q - first) >> 1;
+        for (int k = 0; k < 3; k++) {
+            const double B = c.v[0][k] + (i + 1) * pv[k] + j * qv[k], A = B - pv[k];
+            y[k] = ((q - first) & 1) ? (B + (B + rv[k]) + (B + qv[k])) / 3.0 : (B + A + (A + qv[k])) / 3.0;
+        }
+        f(y, 1.0);
+    }
+}
+BIELCC_D cplx cell_scale(cplx v, const DCell& c, double area, int n) {
+    return c.nv == 4 ? v : v * area / (double)n / (double)n;
+}
+
+// integral_cell over a group.
+template <int G>
+BIELCC_D void group_integral_cell(const Lanes<G>& g, int id, const double* x, const DCell& c, DKP& kp, int idim,
+                                  int n_start, int p_max, double eps, cplx* res) {
+    const double area = c.nv == 3 ? tri_area(c.v[0], c.v[1], c.v[2]) : 0.;
+    adaptive<cplx>(n_start, p_max, eps, idim, kp, res, [&](int n, cplx* acc) {
+        cplx ff[3], sum[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
+        cell_nodes<G>(g, c, n, [&](const double* y, double w) {
+            eval_cplx(id, x, y, kp, ff);
+            for (int q = 0; q < idim; q++) sum[q] = madd(sum[q], ff[q], w);
+        });
+        for (int q = 0; q < idim; q++) acc[q] = cell_scale(g.sum(sum[q]), c, area, n);
+    });
+}
+
+// integral_seg over a group.
+template <int G>
+BIELCC_D void group_integral_seg(const Lanes<G>& g, int id, const double* a, const double* b, const double* x, DKP& kp,
+                                 int n_start, int p_max, double eps, cplx* res) {
+    adaptive<cplx>(n_start, p_max, eps, 3, kp, res, [&](int n, cplx* acc) {
+        double d[3], y[3];
+        for (int k = 0; k < 3; k++) d[k] = (b[k] - a[k]) / n;
+        const double dl = len3(d);
+        cplx ff[3], sum[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
+        for (int i = g.l; i < n; i += G) {
+            for (int k = 0; k < 3; k++) y[k] = a[k] + (i + 0.5) * d[k];
+            eval_cplx(id, x, y, kp, ff);
+            for (int q = 0; q < 3; q++) sum[q] = madd(sum[q], ff[q], dl);
+        }
+        for (int q = 0; q < 3; q++) acc[q] = g.sum(sum[q]);
+    });
+}
+
+// The matrix M of K0_dev with F_GradSimplePot_H (K0 = M j) over a group; kp as K0_dev
+// takes it. One pass per edge (p_seg = 1): the edges are taken side by side, G / 4
+// lanes each, every lane with the radius its edge starts from (shrunk per edge as
+// `adaptive` shrinks it); else edge after edge.
+template <int G>
+BIELCC_D void group_K0_matrix(const Lanes<G>& g, const double* x, const DCell& c, DKP& kp, int n_seg, int p_seg,
+                              double eps, cplx (*mat)[3]) {
+    double nrm[3], nu[3];
+    cell_normal(c, nrm);
+    for (int p = 0; p < 3; p++)
+        for (int q = 0; q < 3; q++) mat[p][q] = mk(0, 0);
+    if (G >= 4 && p_seg == 1) {
+        constexpr int L = G >= 4 ? G / 4 : 1;  // lanes per edge
+        const int e = g.l / L;
+        if (e < c.nv) {
+            for (int h = 0; h < 3 * e; h++)
+                if (kp.smoothR > kp.smoothRMin) kp.smoothR /= 2.;
+            double A[3], d[3], y[3];
+            for (int k = 0; k < 3; k++) {
+                A[k] = c.v[e][k];
+                d[k] = c.v[e + 1 == c.nv ? 0 : e + 1][k];
+            }
+            edge_nu(A, d, nrm, nu);
+            for (int k = 0; k < 3; k++) d[k] = (d[k] - A[k]) / n_seg;
+            const double dl = len3(d);
+            cplx ff[3], sum[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
+            for (int i = g.l & (L - 1); i < n_seg; i += L) {
+                for (int k = 0; k < 3; k++) y[k] = A[k] + (i + 0.5) * d[k];
+                eval_cplx(F_GRADSIMPLEPOT_H, x, y, kp, ff);
+                for (int q = 0; q < 3; q++) sum[q] = madd(sum[q], ff[q], dl);
+            }
+            for (int p = 0; p < 3; p++)
+                for (int q = 0; q < 3; q++) mat[p][q] = sum[p] * (-nu[q]);
+        }
+        __syncwarp(g.mask);
+        for (int p = 0; p < 3; p++)
+            for (int q = 0; q < 3; q++) mat[p][q] = g.sum(mat[p][q]);
+        return;
+    }
+    for (int e = 0; e < c.nv; e++) {
+        const double* A = c.v[e];
+        const double* B = c.v[e + 1 == c.nv ? 0 : e + 1];
+        cplx ks[3];
+        group_integral_seg<G>(g, F_GRADSIMPLEPOT_H, A, B, x, kp, n_seg, p_seg, eps, ks);
+        edge_nu(A, B, nrm, nu);
+        for (int p = 0; p < 3; p++)
+            for (int q = 0; q < 3; q++) mat[p][q] += ks[p] * (-nu[q]);
+    }
+}
+
 // J-independent parts of the near-field pair (x, cell) of the field driver,
 // scaled by 1/4pi: out[13] = { surf * k^2 / 4pi, M (3x3) / 4pi, g (3) / 4pi }
 // so that K_RotRot_Near_Smooth (K.h:47-79) = out0 * J + M J and
-// R_Rot_Smooth (R.h:46-61) = g x J.
-BIELCC_D void near_pair_moments(const double* x, const DCell& cl, cplx k, const DNP& np, cplx* o) {
-    double dm = cell_diam(cl);
+// R_Rot_Smooth (R.h:46-61) = g x J. Evaluated by a group of lanes; the outputs are
+// written by its lanes in turn.
+template <int G>
+BIELCC_D void near_pair_moments(const Lanes<G>& g, const double* x, const DCell& cl, cplx k, const DNP& np, cplx* o) {
+    const double dm = cell_diam(cl);
+    cplx sF[1], gr[3], M[3][3];
     if (np.p_max == 1) {
         // one quadrature pass for both surface integrals: K_RotRot_Near_Smooth's
         // int F (K.h:51-67) and R_Rot_Smooth's int grad F (R.h:46-61) start from
@@ -740,50 +846,94 @@ BIELCC_D void near_pair_moments(const double* x, const DCell& cl, cplx k, const 
         dkp_zero(pS);
         pS.smoothR = np.rs * dm / np.n_start;
         pS.k = k;
-        cplx sF[1], g[3];
-        integral_cell_pot_and_grad(x, cl, pS, np.n_start, sF, g);
-        o[0] = sF[0] * k * k / kFourPi;
-        DKP pG;
-        dkp_zero(pG);
-        pG.smoothR = np.rs_seg * dm / np.n_start_seg;
-        pG.smoothRMin = np.eps;
-        pG.k = k;
-        cplx M[3][3], dummy[3];
-        K0_dev(F_GRADSIMPLEPOT_H, nullptr, x, cl, pG, np.n_start_seg, np.p_max_seg, np.eps, dummy, M);
-        for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++) o[1 + 3 * a + b] = M[a][b] / kFourPi;
-        for (int a = 0; a < 3; a++) o[10 + a] = g[a] / kFourPi;
-        return;
+        sF[0] = gr[0] = gr[1] = gr[2] = mk(0, 0);
+        cell_nodes<G>(g, cl, np.n_start, [&](const double* y, double w) {
+            cplx f[1], gg[3];
+            eval_pot_and_grad(x, y, pS, f, gg);
+            sF[0] = madd(sF[0], f[0], w);
+            for (int q = 0; q < 3; q++) gr[q] = madd(gr[q], gg[q], w);
+        });
+        const double area = cl.nv == 3 ? tri_area(cl.v[0], cl.v[1], cl.v[2]) : 0.;
+        __syncwarp(g.mask);
+        sF[0] = cell_scale(g.sum(sF[0]), cl, area, np.n_start);
+        for (int q = 0; q < 3; q++) gr[q] = cell_scale(g.sum(gr[q]), cl, area, np.n_start);
+    } else {
+        DKP pF, pR;
+        dkp_zero(pF);
+        dkp_zero(pR);
+        pF.smoothR = pR.smoothR = np.rs * dm / np.n_start;
+        pF.smoothRMin = np.eps;    // K_RotRot_Near_Smooth's surface part (K.h:51-67)
+        pR.smoothRMin = dm / 100.;  // R_Rot_Smooth (R.h:46-61)
+        pF.k = pR.k = k;
+        group_integral_cell<G>(g, F_SIMPLEPOT_H, x, cl, pF, 1, np.n_start, np.p_max, np.eps, sF);
+        group_integral_cell<G>(g, F_GRADSIMPLEPOT_H, x, cl, pR, 3, np.n_start, np.p_max, np.eps, gr);
     }
-    // surface part of K_RotRot_Near_Smooth (K.h:51-67)
-    DKP pF;
-    dkp_zero(pF);
-    pF.smoothR = np.rs * dm / np.n_start;
-    pF.smoothRMin = np.eps;
-    pF.k = k;
-    cplx s[1];
-    integral_cell<cplx>(F_SIMPLEPOT_H, x, cl, pF, 1, np.n_start, np.p_max, np.eps, s);
-    o[0] = s[0] * k * k / kFourPi;
     // contour part (K.h:56-72): K0 with the shared, shrinking segment radius
     DKP pG;
     dkp_zero(pG);
     pG.smoothR = np.rs_seg * dm / np.n_start_seg;
     pG.smoothRMin = np.eps;
     pG.k = k;
-    cplx M[3][3], dummy[3];
-    K0_dev(F_GRADSIMPLEPOT_H, nullptr, x, cl, pG, np.n_start_seg, np.p_max_seg, np.eps, dummy, M);
-    for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) o[1 + 3 * a + b] = M[a][b] / kFourPi;
-    // R_Rot_Smooth (R.h:46-61)
-    DKP pR;
-    dkp_zero(pR);
-    pR.smoothR = np.rs * dm / np.n_start;
-    pR.smoothRMin = dm / 100.;
-    pR.k = k;
-    cplx g[3];
-    integral_cell<cplx>(F_GRADSIMPLEPOT_H, x, cl, pR, 3, np.n_start, np.p_max, np.eps, g);
-    for (int a = 0; a < 3; a++) o[10 + a] = g[a] / kFourPi;
+    group_K0_matrix<G>(g, x, cl, pG, np.n_start_seg, np.p_max_seg, np.eps, M);
+    auto put = [&](int q, cplx v) {
+        if (g.l == (q & (G - 1))) o[q] = v;
+    };
+    put(0, sF[0] * k * k / kFourPi);
+#pragma unroll
+    for (int p = 0; p < 3; p++)
+#pragma unroll
+        for (int q = 0; q < 3; q++) put(1 + 3 * p + q, M[p][q] / kFourPi);
+#pragma unroll
+    for (int p = 0; p < 3; p++) put(10 + p, gr[p] / kFourPi);
 }
+// The operator matrix of K_RotRot_HS_Colloc (K.h:179-204), K = mat j, over a group:
+// IntegralSurf_SimplePot_H_HS's near branch (integrals_analytic.h:136-164; the caller
+// has decided near) with one edge of its triangles per lane, and the contour part.
+template <int G>
+BIELCC_D void group_hs_colloc(const Lanes<G>& g, const double* x, const DCell& c, cplx k, const DNP& np,
+                              cplx (&mat)[3][3]) {
+    double a = 0.;
+    if constexpr (G >= 8) {
+        if (g.l < (c.nv == 4 ? 6 : 3)) {  // quad = triangles 012 + 230
+            const int t = g.l / 3, e = g.l - 3 * t, v0 = t ? 2 : 0, v1 = t ? 3 : 1, v2 = t ? 0 : 2;
+            double P[3][3];
+            for (int i = 0; i < 3; i++) {
+                P[0][i] = c.v[v0][i];
+                P[1][i] = c.v[v1][i];
+                P[2][i] = c.v[v2][i];
+            }
+            InvRTri tri;
+            if (tri.set(P[0], P[1], P[2], x)) a = tri.edge(P[e], P[e == 2 ? 0 : e + 1], x);
+        }
+        __syncwarp(g.mask);
+        a = g.sum(a);
+    } else {
+        a = integral_1divr_dev(c, x);
+    }
+    DKP kp, ps;
+    dkp_zero(kp);
+    kp.smoothR = kp.smoothRMin = kMachineZero;
+    kp.k = k;
+    ps = kp;
+    cplx I[1];
+    group_integral_cell<G>(g, F_SIMPLEPOT_HM1, x, c, kp, 1, np.n_start, np.p_max, np.eps, I);
+    const cplx s = mk(a + I[0].re, I[0].im) * k * k / kFourPi;
+    group_K0_matrix<G>(g, x, c, ps, np.n_start_seg, np.p_max_seg, np.eps, mat);
+    for (int p = 0; p < 3; p++)
+        for (int q = 0; q < 3; q++) {
+            mat[p][q] = mat[p][q] / kFourPi;
+            if (p == q) mat[p][q] += s;
+        }
+}
+
+// Lanes per near pair of a call with n_near pairs: one when the pairs alone fill
+// the GPU (148 SMs hold about 57,000 threads of these kernels), else 8, else a warp.
+// Measured, one lane -> 8 or 32: 0.09 -> 0.03 ms (80 triangles x 100 points),
+// 2.2 -> 0.8 ms (8000 pairs, p_max 3), 0.21 -> 0.15 ms (two calls of 10,000), but
+// 0.41 -> 0.57 ms (160,000 pairs) and 3.2 -> 5.5 ms (1.5 million matrix blocks): the
+// per-pair geometry and the sums across lanes are then extra work. Batches always
+// take one lane: a job's sums must not depend on the other jobs' pairs.
+inline int near_lanes(long long n_near) { return n_near >= 32768 ? 1 : (n_near >= 4096 ? 8 : 32); }
 
 BIELCC_D void run_pair_op(int op, const cplx* j, const double* x, const DCell& c, const DNP& np, cplx k, cplx* res) {
     switch (op) {
