@@ -30,8 +30,7 @@
 //   4. near sums    — one warp per (point, RHS): the point's near pairs
 //                     contracted with J, lane-strided in cell order, fixed
 //                     butterfly across the lanes.
-//   5. finalize     — per (point, RHS): far partials over splits (in order;
-//                     lane-strided with a fixed butterfly beyond 32 splits) +
+//   5. finalize     — per (point, RHS): far partials over splits (in order) +
 //                     the near sum, x mult, + incident field.
 #include <algorithm>
 #include <atomic>
@@ -804,81 +803,63 @@ struct FinalArgs {
     unsigned long long* nonfinite;
 };
 
-// Per (point, RHS): far partials over the splits, near sum, mult, incident
-// field. One thread per point sums the splits in order (coalesced over the
-// points); with many splits (a small point set spread over the whole GPU) one
-// warp per point takes splits lane-strided and combines the lanes with a fixed
-// xor butterfly, so the serial chain is splits / 32 loads long instead of splits.
-template <bool WARP>
-__global__ void finalize_kernel(FinalArgs a) {
-    const int s = blockIdx.y;
+// Per (point, RHS): far partials over the splits (in split order), near sum, mult,
+// incident field. A CTA takes 32 points: warp q sums component q (12 of them) of its
+// lanes' points, eight splits' loads in flight at a time, then warp 0 finishes E
+// and warp 1 H. With one thread per point all 12 components' loads of a split had to
+// return before the next split's were issued: 100 points x 10 splits 27 us, 3001 x 4
+// right-hand sides 75 us; with a warp per point and lanes over the splits every
+// 8-byte load fetched a sector of its own.
+constexpr int kFinalThreads = 12 * 32;
+__global__ void __launch_bounds__(kFinalThreads) finalize_kernel(const __grid_constant__ FinalArgs a) {
+    __shared__ double s_v[12][32];
+    __shared__ int s_bad[32];
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5, s = blockIdx.y;
+    const int p = blockIdx.x * 32 + lane;
     const size_t P = a.n_pts;
-    double v[12];
-#pragma unroll
-    for (int q = 0; q < 12; q++) v[q] = 0.;
-    int p;
-    if constexpr (WARP) {
-        p = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-        const int lane = threadIdx.x & 31;
-        if (p >= a.n_pts) return;  // whole warps
-        for (int sp = lane; sp < a.splits; sp += 32) {
-            const double* src = a.partial + (((size_t)sp * a.n_rhs + s) * 12) * P + p;
-#pragma unroll
-            for (int q = 0; q < 12; q++) v[q] += src[(size_t)q * P];
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-            for (int q = 0; q < 12; q++) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
-        if (lane != 0) return;
-    } else {
-        p = blockIdx.x * blockDim.x + threadIdx.x;
-        if (p >= a.n_pts) return;
-        for (int sp = 0; sp < a.splits; sp++) {
-            const double* src = a.partial + (((size_t)sp * a.n_rhs + s) * 12) * P + p;
-            for (int q = 0; q < 12; q++) v[q] += src[(size_t)q * P];
-        }
+    if (p < a.n_pts) {
+        const double* src = a.partial + ((size_t)s * 12 + q) * P + p;
+        const size_t step = (size_t)a.n_rhs * 12 * P;
+        double v = 0.;
+#pragma unroll 8
+        for (int sp = 0; sp < a.splits; sp++) v += src[sp * step];
+        s_v[q][lane] = v;
     }
-    cplx E[3], H[3];
-    for (int g = 0; g < 3; g++) {
-        E[g] = mk(v[2 * g], v[2 * g + 1]) * kInvFourPi;
-        H[g] = mk(v[6 + 2 * g], v[6 + 2 * g + 1]) * kInvFourPi;
-    }
-    if (a.offs && a.offs[p + 1] > a.offs[p]) {
-        const double* nv = a.near + (size_t)s * 12 * P + p;
-        for (int g = 0; g < 3; g++) {
-            E[g] += mk(nv[(size_t)(2 * g) * P], nv[(size_t)(2 * g + 1) * P]);
-            H[g] += mk(nv[(size_t)(6 + 2 * g) * P], nv[(size_t)(7 + 2 * g) * P]);
-        }
-    }
-    for (int g = 0; g < 3; g++) E[g] = E[g] * a.mult;
-    const double* x = a.pts + 3 * (size_t)p;
-    if (a.add_E || a.add_H) {
-        double ph = a.kvec[0] * x[0] + a.kvec[1] * x[1] + a.kvec[2] * x[2];
-        double sn, cs;
-        sincos(ph, &sn, &cs);
-        if (a.add_E)
-            for (int g = 0; g < 3; g++) E[g] += mk(a.e0[g] * cs, a.e0[g] * sn);
-        if (a.add_H) {
-            double kx0[3];
-            cross3(a.kvec, a.e0, kx0);
-            for (int g = 0; g < 3; g++) H[g] += mk(kx0[g] * cs * a.h_scale, kx0[g] * sn * a.h_scale);
-        }
-    }
+    __syncthreads();
     bool bad = false;
-    cplx* eo = reinterpret_cast<cplx*>(a.E) + ((size_t)s * P + p) * 3;
-    for (int g = 0; g < 3; g++) {
-        eo[g] = E[g];
-        bad |= !isfinite(E[g].re) || !isfinite(E[g].im);
-    }
-    if (a.H) {
-        cplx* ho = reinterpret_cast<cplx*>(a.H) + ((size_t)s * P + p) * 3;
-        for (int g = 0; g < 3; g++) {
-            ho[g] = H[g];
-            bad |= !isfinite(H[g].re) || !isfinite(H[g].im);
+    if (q < 2 && p < a.n_pts) {  // warp 0: E, warp 1: H
+        cplx F[3];
+        for (int g = 0; g < 3; g++) F[g] = mk(s_v[6 * q + 2 * g][lane], s_v[6 * q + 2 * g + 1][lane]) * kInvFourPi;
+        if (a.offs && a.offs[p + 1] > a.offs[p]) {
+            const double* nv = a.near + ((size_t)s * 12 + 6 * q) * P + p;
+            for (int g = 0; g < 3; g++) F[g] += mk(nv[(size_t)(2 * g) * P], nv[(size_t)(2 * g + 1) * P]);
+        }
+        if (q == 0)
+            for (int g = 0; g < 3; g++) F[g] = F[g] * a.mult;
+        if (q == 0 ? a.add_E : a.add_H) {
+            const double* x = a.pts + 3 * (size_t)p;
+            double sn, cs, f[3];
+            sincos(a.kvec[0] * x[0] + a.kvec[1] * x[1] + a.kvec[2] * x[2], &sn, &cs);
+            if (q == 0) {
+                for (int g = 0; g < 3; g++) F[g] += mk(a.e0[g] * cs, a.e0[g] * sn);
+            } else {
+                cross3(a.kvec, a.e0, f);
+                for (int g = 0; g < 3; g++) F[g] += mk(f[g] * cs * a.h_scale, f[g] * sn * a.h_scale);
+            }
+        }
+        double* out = q == 0 ? a.E : a.H;
+        if (out) {
+            cplx* o = reinterpret_cast<cplx*>(out) + ((size_t)s * P + p) * 3;
+            for (int g = 0; g < 3; g++) {
+                o[g] = F[g];
+                bad |= !isfinite(F[g].re) || !isfinite(F[g].im);
+            }
         }
     }
-    if (bad && a.nonfinite) atomicAdd(a.nonfinite, 1ull);
+    if (!a.nonfinite) return;
+    if (q == 1) s_bad[lane] = bad;
+    __syncthreads();
+    if (q == 0 && (bad || s_bad[lane])) atomicAdd(a.nonfinite, 1ull);  // once per (point, RHS)
 }
 
 // ---------------------------------------------------------------- host launchers
@@ -1160,8 +1141,7 @@ cudaError_t field_stage2(const FieldLaunch& f, void* ws, int splits, long long n
     fa.H = f.H;
     fa.nonfinite = d_nonfinite;
     if (tiles > 0 && f.n_rhs > 0) {
-        if (fa.splits > 32) finalize_kernel<true><<<dim3((f.n_pts + 7) / 8, f.n_rhs), 256, 0, s>>>(fa);
-        else finalize_kernel<false><<<dim3(tiles, f.n_rhs), kFarThreads, 0, s>>>(fa);
+        finalize_kernel<<<dim3((f.n_pts + 31) / 32, f.n_rhs), kFinalThreads, 0, s>>>(fa);
         *launches += 1;
     }
     return cudaGetLastError();
