@@ -991,7 +991,7 @@ cudaError_t assemble_stage2(const AssembleLaunch& a, void* ws, long long n_near,
     AsmArgs g = make_args(a);
     DNP np{a.np.eps, a.np.rs, a.np.rs_seg, a.np.analytic_calc, a.np.n_start, a.np.n_start_seg, a.np.p_max,
            a.np.p_max_seg};
-    const int lanes = near_lanes(n_near), blocks = (int)((n_near * lanes + 127) / 128);
+    const int lanes = near_lanes(n_near, np), blocks = (int)((n_near * lanes + 127) / 128);
     const auto near_blocks = lanes == 1 ? asm_near_kernel<1> : (lanes == 8 ? asm_near_kernel<8> : asm_near_kernel<32>);
     near_blocks<<<blocks, 128, 0, s>>>(g, m.verts, m.nv, pr, pc, n_near, np);
     return cudaGetLastError();

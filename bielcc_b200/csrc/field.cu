@@ -1113,7 +1113,7 @@ cudaError_t field_stage2(const FieldLaunch& f, void* ws, int splits, long long n
         near_fill_kernel<<<(f.n_pts + 7) / 8, 256, 0, s>>>(mask, n_words, f.n_pts, offs, pair_cell, pair_pt);
         DNP np{f.np.eps, f.np.rs, f.np.rs_seg, f.np.analytic_calc, f.np.n_start, f.np.n_start_seg, f.np.p_max,
                f.np.p_max_seg};
-        const int lanes = near_lanes(n_near), blocks = (int)((n_near * lanes + 127) / 128);
+        const int lanes = near_lanes(n_near, np), blocks = (int)((n_near * lanes + 127) / 128);
         const auto near_pairs = lanes == 1 ? near_pair_kernel<1> : (lanes == 8 ? near_pair_kernel<8> : near_pair_kernel<32>);
         near_pairs<<<blocks, 128, 0, s>>>(f.pts, m.verts, m.nv, pair_cell, pair_pt, n_near, f.k, np, moments);
         near_sum_kernel<<<dim3((f.n_pts + 7) / 8, f.n_rhs), 256, 0, s>>>(

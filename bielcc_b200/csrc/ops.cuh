@@ -929,11 +929,14 @@ BIELCC_D void group_hs_colloc(const Lanes<G>& g, const double* x, const DCell& c
 // Lanes per near pair of a call with n_near pairs: one when the pairs alone fill
 // the GPU (148 SMs hold about 57,000 threads of these kernels), else 8, else a warp.
 // Measured, one lane -> 8 or 32: 0.09 -> 0.03 ms (80 triangles x 100 points),
-// 2.2 -> 0.8 ms (8000 pairs, p_max 3), 0.21 -> 0.15 ms (two calls of 10,000), but
+// 2.2 -> 0.8 ms with 32 lanes, 0.9 with 8 (8000 pairs, p_max 3: up to 1024 nodes a
+// pass), 0.62 -> 0.51 with 32, 0.40 with 8 (16,000 pairs, p_max 2), but
 // 0.41 -> 0.57 ms (160,000 pairs) and 3.2 -> 5.5 ms (1.5 million matrix blocks): the
 // per-pair geometry and the sums across lanes are then extra work. Batches always
 // take one lane: a job's sums must not depend on the other jobs' pairs.
-inline int near_lanes(long long n_near) { return n_near >= 32768 ? 1 : (n_near >= 4096 ? 8 : 32); }
+inline int near_lanes(long long n_near, const DNP& np) {
+    return n_near >= 32768 ? 1 : (n_near >= (np.p_max > 2 ? 16384 : 4096) ? 8 : 32);
+}
 
 BIELCC_D void run_pair_op(int op, const cplx* j, const double* x, const DCell& c, const DNP& np, cplx k, cplx* res) {
     switch (op) {
