@@ -101,6 +101,11 @@ size_t rules_bytes(int nv, int n, int n_cells);
 cudaError_t launch_rules(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
                          void* mem, FarRules* out, cudaStream_t s);
 
+// The same for one precision, with only the shortest levels that fit in `bytes`
+// (none, if none does).
+cudaError_t launch_rules_within(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
+                                bool mixed, void* mem, size_t bytes, FarRules* out, cudaStream_t s);
+
 // ---- field.cu
 struct FieldLaunch {
     const MeshDev* mesh;

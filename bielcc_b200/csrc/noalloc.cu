@@ -165,6 +165,17 @@ extern "C" int bielcc_field_EH_noalloc(int n_vert, int n_cells, const double* ce
     if (e == cudaSuccess && m.nodes64_hi)
         e = launch_node_tables(m.verts, m.geo, n_vert, n_cells, m.table_hi_n, m.nodes64_hi, m.nodes32_hi, m.rho32_hi,
                                s);
+    // the far pass's compressed rules, as many levels as the rest of the array holds:
+    // they are read by stage 1 only, so stage 2's near pairs take their place and no
+    // size is refused for them. They are built anew by every call, at about the cost
+    // of 500 points' full rows of 64 nodes, so small point sets go without: from
+    // 1024 points (n_start 8, p_max 1) or 256 (p_max 2: rows of 256 nodes). p_max >= 3
+    // reads FP64 rows in the mixed form too and goes without.
+    // 8192 quads x 5000 points, mixed: 7.0 ms without, 2.2 with; 8192 x 2000, FP64:
+    // 6.1 without, 3.6 with; 2048 x 1000, p_max 2, mixed: 1.50 without, 0.55 with.
+    if (e == cudaSuccess && (long long)n_pts * n_rhs * far_split_n(n) * far_split_n(n) >= 65536 && !far_adaptive(n))
+        e = launch_rules_within(m.verts, m.geo, m.rho32, n_vert, n_cells, far_split_n(n), precision == BIELCC_PREC_MIXED,
+                                sp + off, BIELCC_NOALLOC_SCRATCH_BYTES - off, &m.rules, s);
     int l1 = 0, lf = 0, l2 = 0;
     if (e == cudaSuccess) e = field_stage1(f, ws, splits, d_total, s, &l1, nullptr, nullptr, &lf);
     long long n_near = 0;  // pageable host copy: no pinned staging is allocated

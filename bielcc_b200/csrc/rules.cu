@@ -55,7 +55,7 @@ namespace bielcc_gpu {
 // below the rounding of the FP32 node sum (1.1e-7 rms per pair, measured) and
 // of the FP64 one.
 #ifndef BIELCC_RULE_TOL32
-#define BIELCC_RULE_TOL32 4e-9
+#define BIELCC_RULE_TOL32 1e-8
 #endif
 constexpr double kRuleTol32 = BIELCC_RULE_TOL32, kRuleTol64 = 3e-17;
 // Moments agree to rounding only; differences below this are rounding (of the
@@ -477,8 +477,32 @@ __global__ void rule_nodes_kernel(const __grid_constant__ RuleHost h, const doub
     rule_node(v, nv, nv == 3 ? tri_area(v[0], v[1], v[2]) : 0., h.s[q], h.t[q], h.w[q], y, &w);
     const size_t o = (size_t)h.off[l] * n_cells + c * h.cnt[l] + (q - h.off[l]);
     const double* ctr = geo[c].c;
-    n64[o] = make_double4(y[0], y[1], y[2], w);
-    n32[o] = make_float4((float)(y[0] - ctr[0]), (float)(y[1] - ctr[1]), (float)(y[2] - ctr[2]), (float)w);
+    if (n64) n64[o] = make_double4(y[0], y[1], y[2], w);
+    if (n32) n32[o] = make_float4((float)(y[0] - ctr[0]), (float)(y[1] - ctr[1]), (float)(y[2] - ctr[2]), (float)w);
+}
+
+// FP32 weights of a row, rounded so that their sum is the FP64 sum's (the rounding
+// of each goes into the next): 7 - 20 weights rounded on their own left a cell up to
+// 2e-8 heavy, where the errors of 64 mostly cancel. One thread per (cell, level).
+__global__ void rule_weights_kernel(const __grid_constant__ RuleHost h, const double* __restrict__ verts, int nv,
+                                    int n_cells, float4* __restrict__ n32) {
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    const size_t c = i / h.n_lev;
+    if (c >= (size_t)n_cells) return;
+    const int l = (int)(i - c * h.n_lev);
+    double v[4][3], y[3], w, carry = 0.;
+    for (int a = 0; a < nv; a++)
+        for (int g = 0; g < 3; g++) v[a][g] = verts[(c * nv + a) * 3 + g];
+    const double area = nv == 3 ? tri_area(v[0], v[1], v[2]) : 0.;
+    float4* row = n32 + (size_t)h.off[l] * n_cells + c * h.cnt[l];
+    for (int q = 0; q < h.cnt[l]; q++) {
+        const int k = h.off[l] + q;
+        rule_node(v, nv, area, h.s[k], h.t[k], h.w[k], y, &w);
+        w += carry;
+        const float f = (float)w;
+        row[q].w = f;
+        carry = w - (double)f;
+    }
 }
 
 // Triangles: the limits are the same for every cell up to its radius rho.
@@ -635,21 +659,29 @@ __global__ void rule_limits_quad_kernel(const __grid_constant__ RuleHost h, cons
     }
 }
 
-size_t rules_bytes(int nv, int n, int n_cells) {
-    const RuleHost& h = rules_for(nv, n);
-    return h.n_lev ? (size_t)n_cells * (h.total * (sizeof(double4) + sizeof(float4)) + 2 * h.n_lev * sizeof(float2)) : 0;
+// Device bytes of h's levels with FP64 rows, FP32 rows or both.
+static size_t level_bytes(const RuleHost& h, int n_cells, bool f64, bool f32) {
+    return (size_t)n_cells * (h.total * ((f64 ? sizeof(double4) : 0) + (f32 ? sizeof(float4) : 0)) +
+                              2 * h.n_lev * sizeof(float2));
 }
 
-cudaError_t launch_rules(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
-                         void* mem, FarRules* out, cudaStream_t s) {
-    *out = FarRules();
+size_t rules_bytes(int nv, int n, int n_cells) {
     const RuleHost& h = rules_for(nv, n);
-    if (!h.n_lev || n_cells <= 0) return cudaSuccess;
-    double4* n64 = (double4*)mem;
-    float4* n32 = (float4*)(n64 + (size_t)h.total * n_cells);
-    float2* thr = (float2*)(n32 + (size_t)h.total * n_cells);
+    return level_bytes(h, n_cells, true, true);
+}
+
+// Builds the levels of h in `mem` ([FP64 rows][FP32 rows][limits]).
+static cudaError_t build_levels(const RuleHost& h, const double* verts, const CellGeo* geo, const float* rho32, int nv,
+                                int n_cells, int n, bool f64, bool f32, void* mem, FarRules* out, cudaStream_t s) {
+    double4* n64 = f64 ? (double4*)mem : nullptr;
+    char* end = (char*)mem + (f64 ? (size_t)h.total * n_cells * sizeof(double4) : 0);
+    float4* n32 = f32 ? (float4*)end : nullptr;
+    float2* thr = (float2*)(end + (f32 ? (size_t)h.total * n_cells * sizeof(float4) : 0));
     const size_t nodes = (size_t)h.total * n_cells;
     rule_nodes_kernel<<<(unsigned)((nodes + 127) / 128), 128, 0, s>>>(h, verts, geo, nv, n_cells, n64, n32);
+    if (f32)
+        rule_weights_kernel<<<(unsigned)(((size_t)n_cells * h.n_lev + 127) / 128), 128, 0, s>>>(h, verts, nv, n_cells,
+                                                                                                n32);
     if (nv == 4) rule_limits_quad_kernel<<<(n_cells + 3) / 4, 128, 0, s>>>(h, verts, geo, n_cells, n, thr);
     else rule_limits_tri_kernel<<<(n_cells + 127) / 128, 128, 0, s>>>(h, rho32, n_cells, thr);
     out->n_lev = h.n_lev;
@@ -662,6 +694,26 @@ cudaError_t launch_rules(const double* verts, const CellGeo* geo, const float* r
     out->thr32 = thr;
     out->thr64 = thr + (size_t)n_cells * h.n_lev;
     return cudaGetLastError();
+}
+
+cudaError_t launch_rules(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
+                         void* mem, FarRules* out, cudaStream_t s) {
+    *out = FarRules();
+    const RuleHost& h = rules_for(nv, n);
+    if (!h.n_lev || n_cells <= 0) return cudaSuccess;
+    return build_levels(h, verts, geo, rho32, nv, n_cells, n, true, true, mem, out, s);
+}
+
+cudaError_t launch_rules_within(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
+                                bool mixed, void* mem, size_t bytes, FarRules* out, cudaStream_t s) {
+    *out = FarRules();
+    RuleHost h = rules_for(nv, n);
+    while (h.n_lev > 0 && level_bytes(h, n_cells, !mixed, mixed) > bytes) {
+        h.n_lev--;
+        h.total = h.off[h.n_lev];
+    }
+    if (!h.n_lev || n_cells <= 0) return cudaSuccess;
+    return build_levels(h, verts, geo, rho32, nv, n_cells, n, !mixed, mixed, mem, out, s);
 }
 
 }  // namespace bielcc_gpu
