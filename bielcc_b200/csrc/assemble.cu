@@ -292,9 +292,9 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
             const bool any = dmin < __int_as_float(0x7f800000);
             const F *tj1 = s_tau[cc], *tj2 = s_tau[cc] + 3;
             double Kr[3][3], Ki[3][3];     // FP64 form: the operator matrix
-            float a1r = 0, a1i = 0, t[6][2], phr = 0, phi = 0;  // mixed form: moments and phase / 4pi
-#pragma unroll
-            for (int q = 0; q < 6; q++) t[q][0] = t[q][1] = 0;
+            Moments<float> m;              // mixed form: moments (A1, T)
+            float phr = 0, phi = 0;        // and phase / 4pi
+            m.zero();
             if (any) {
                 const int lev = rule_level(s_rmin[cc], n_lev, dmin);
                 const int cnt = s_tab.cnt[lev], mode = s_mode[cc];
@@ -316,14 +316,13 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                     RowBuf<NodeT>& rb = s_rows[warp];
                     if (k0 && lane < kc) v = row[k0 + lane];
                     __syncwarp();  // the previous chunk has been read
-                    rb.nd[lane] = v;
-                    if constexpr (MIXED) rb.yy[lane] = node_yy(v);
+                    rb.put(lane, v);
                     __syncwarp();
                     if (!far) continue;
                     if constexpr (MIXED) {
 #define BIELCC_ASM_LOOP(MODE_)                                                \
     _Pragma("unroll 4") for (int q = 0; q < kc; q++)                          \
-        far_node_f32_K<CK, MODE_>(a1r, a1i, t, pf, rb.nd[q], rb.yy[q], kf);
+        far_node_f32<CK, MODE_, false>(m, pf, rb.get(q), kf);
                         switch (mode) {
                             case 0: BIELCC_ASM_LOOP(0) break;
                             case 1: BIELCC_ASM_LOOP(1) break;
@@ -337,19 +336,19 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                         // series when |k| rho <= 0.5); its grad-F moments are unused here
 #pragma unroll 2
                         for (int q = 0; q < kc; q++) {
-                            const double4 y = rb.nd[q];
+                            const double4 y = rb.get(q);
                             far_node_f64<CK, true>(mm, x[0] - y.x, x[1] - y.y, x[2] - y.z, y.w, a.k, k2r, k2i, d);
                         }
                     } else {
 #pragma unroll 2
                         for (int q = 0; q < kc; q++) {
-                            const double4 y = rb.nd[q];
+                            const double4 y = rb.get(q);
                             far_node_f64<CK, false>(mm, x[0] - y.x, x[1] - y.y, x[2] - y.z, y.w, a.k, k2r, k2i, d);
                         }
                     }
                 }
                 if constexpr (MIXED) {
-                    if constexpr (!CK) finish_real_k<float>(a1r, a1i, t);
+                    if constexpr (!CK) finish_real_k<float>(m.a1r, m.a1i, m.t);
                 } else {
                     if (!CK) mm.finish_real_k();
                     // K = (A1 I + T) * P0 / 4pi
@@ -371,7 +370,7 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                 // column cell's pair; complex128, pieces 2 g and 2 g + 1 its two entries
                 if constexpr (MIXED) {
                     float o[2][2][2];
-                    block_f32<2>(a1r, a1i, t, phr, phi, tif, tj1, tj2, o);
+                    block_f32<2>(m.a1r, m.a1i, m.t, phr, phi, tif, tj1, tj2, o);
 #pragma unroll
                     for (int r = 0; r < 2; r++) {
                         uint4* w = out + (r * 32 + lane) * 8;
@@ -419,8 +418,8 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                 }
             } else if (far) {
                 if constexpr (MIXED) {
-                    if (a.m == 2) write_block_f32<2>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, tj1, tj2, cols);
-                    else write_block_f32<3>(a, i, c0 + cc, a1r, a1i, t, phr, phi, tif, tj1, tj2, cols);
+                    if (a.m == 2) write_block_f32<2>(a, i, c0 + cc, m.a1r, m.a1i, m.t, phr, phi, tif, tj1, tj2, cols);
+                    else write_block_f32<3>(a, i, c0 + cc, m.a1r, m.a1i, m.t, phr, phi, tif, tj1, tj2, cols);
                 } else {
                     write_block(a, i, c0 + cc, Kr, Ki, gi.t1, gi.t2, tj1, tj2, cols);
                 }

@@ -281,8 +281,7 @@ BIELCC_D void batch_moments(const typename BatchCfg<MIXED>::NodeT* __restrict__ 
         const int mode = mixed_pair_setup<CK>(fd, rho, k, kf, pf, P0r, P0i);
 #define BIELCC_BNODE(MODE_)                                      \
     BIELCC_UNROLL(BIELCC_BATCH_U1) for (int i = 0; i < nn; i++) { \
-        const float4 v = __ldg(nd + i);                           \
-        far_node_f32<CK, MODE_>(m, pf, v, node_yy(v), kf);        \
+        far_node_f32<CK, MODE_>(m, pf, node_f32(__ldg(nd + i)), kf); \
     }
         switch (mode) {
             case 0: BIELCC_BNODE(0) break;
@@ -343,16 +342,14 @@ BIELCC_D void batch_moments2(RowBuf<float4>* rb, const float4* __restrict__ rowA
             vb = rowB[k0 + lane];
         }
         __syncwarp();  // the previous chunk has been read
-        rb[0].nd[lane] = va;
-        rb[1].nd[lane] = vb;
-        rb[0].yy[lane] = node_yy(va);
-        rb[1].yy[lane] = node_yy(vb);
+        rb[0].put(lane, va);
+        rb[1].put(lane, vb);
         __syncwarp();
         if (!need) continue;
 #define BIELCC_BNODE2(MODE_)                                                   \
     BIELCC_UNROLL(BIELCC_BATCH_U2) for (int i = 0; i < kc; i++) {              \
-        far_node_f32<CK, MODE_>(ma, pa, rb[0].nd[i], rb[0].yy[i], kf);         \
-        far_node_f32<CK, MODE_>(mb, pb, rb[1].nd[i], rb[1].yy[i], kf);         \
+        far_node_f32<CK, MODE_>(ma, pa, rb[0].get(i), kf);                     \
+        far_node_f32<CK, MODE_>(mb, pb, rb[1].get(i), kf);                     \
     }
         switch (mode) {
             case 0: BIELCC_BNODE2(0) break;

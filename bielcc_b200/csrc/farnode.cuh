@@ -137,6 +137,7 @@ struct Moments {
     F a1r, a1i;
     F t[6][2];  // xx, xy, xz, yy, yz, zz
     F g[3][2];
+    static constexpr bool kNegG = sizeof(F) == 4;  // far_node_f32's real-k loop leaves -G
     BIELCC_D void zero() {
         a1r = a1i = 0;
         for (int i = 0; i < 6; i++) t[i][0] = t[i][1] = 0;
@@ -161,6 +162,13 @@ BIELCC_D void finish_real_k(F& a1r, F& a1i, F (&t)[6][2]) {
 template <typename F>
 BIELCC_D void Moments<F>::finish_real_k() {
     bielcc_gpu::finish_real_k<F>(a1r, a1i, t);
+    if (kNegG) {
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            g[q][0] = -g[q][0];
+            g[q][1] = -g[q][1];
+        }
+    }
 }
 
 // FP32 wavenumber constants of one launch (or one job).
@@ -168,7 +176,7 @@ struct KF32 {
     float kr, ki;    // k
     float k2r, k2i;  // k^2
     float ikr;       // 1 / Re k, 1e30 for Re k = 0 (phase k (r - r0) = q / ((r + r0) ikr) then rounds to 0)
-    float k2r3;      // Re k^2 / 3
+    float k2r3;      // -Re k^2 / 3
     static BIELCC_D KF32 make(double kre, double kim) {
         KF32 f;
         const double k2r = kre * kre - kim * kim;
@@ -177,7 +185,7 @@ struct KF32 {
         f.k2r = (float)k2r;
         f.k2i = (float)(2.0 * kre * kim);
         f.ikr = kre != 0.0 ? (float)(1.0 / kre) : 1e30f;
-        f.k2r3 = (float)(k2r / 3.0);
+        f.k2r3 = (float)(-k2r / 3.0);
         return f;
     }
 };
@@ -345,42 +353,52 @@ BIELCC_HD int phase_mode(float th) {
     return th <= 0.25f ? 0 : (th <= 1.f ? 1 : (th <= 2.f ? 2 : (th <= 4.f ? 3 : 4)));
 }
 
-// One staged node of a row chunk: FP32 rows carry |y - centre|^2 beside the node.
+// A row's chunk of staged nodes, one of every warp's buffers. FP32 nodes are held
+// as the packed arithmetic of far_node_f32 reads them: negated and doubled
+// (-x, -x, -y, -y), (-z, -z, w, |y - centre|^2), |.|^2 computed once per node.
 constexpr int kRowChunk = 32;
+struct NodeF32 {
+    float4 a, b;
+};
+BIELCC_D NodeF32 node_f32(float4 n) {  // n = (y - centre, w)
+    return {make_float4(-n.x, -n.x, -n.y, -n.y),
+            make_float4(-n.z, -n.z, n.w, fmaf(n.x, n.x, fmaf(n.y, n.y, n.z * n.z)))};
+}
 template <typename NodeT>
 struct RowBuf {
     NodeT nd[kRowChunk];
-    float yy[sizeof(NodeT) == 16 ? kRowChunk : 1];
+    BIELCC_D void put(int i, const NodeT& v) { nd[i] = v; }
+    BIELCC_D NodeT get(int i) const { return nd[i]; }
+};
+template <>
+struct RowBuf<float4> {
+    float4 a[kRowChunk], b[kRowChunk];
+    BIELCC_D void put(int i, float4 v) {
+        const NodeF32 n = node_f32(v);
+        a[i] = n.a;
+        b[i] = n.b;
+    }
+    BIELCC_D NodeF32 get(int i) const { return {a[i], b[i]}; }
 };
 
 // Per-pair FP32 state of the mixed far node, relative to the cell centre:
-// X = x - centre, X2 = -2 X, r0 = |X| (FP64 rounded), r0sq = r0^2, r0k = r0 / Re k.
+// X = x - centre (each component twice), X2 = 2 X, r0 = |X| (FP64 rounded), r0sq = r0^2, r0k = r0 / Re k.
 struct PairF32 {
-    float X[3], X2[3], r0, r0sq, r0k;
-    BIELCC_D void set(const double* x, const double* centre, double d, const KF32& kf) {
-        for (int g = 0; g < 3; g++) {
-            X[g] = (float)(x[g] - centre[g]);
-            X2[g] = -2.f * X[g];
-        }
-        r0 = (float)d;
-        r0sq = (float)(d * d);
-        r0k = r0 * kf.ikr;
-    }
+    float2 X[3];
+    float X2[3], r0, r0sq, r0k;
     // from x - centre (FP64), |x - centre|^2 and |x - centre|
     BIELCC_D void set(const double (&dx)[3], double s, double d, const KF32& kf) {
 #pragma unroll
         for (int g = 0; g < 3; g++) {
-            X[g] = (float)dx[g];
-            X2[g] = -2.f * X[g];
+            const float v = (float)dx[g];
+            X[g] = make_float2(v, v);
+            X2[g] = v + v;
         }
         r0 = (float)d;
         r0sq = (float)s;
         r0k = r0 * kf.ikr;
     }
 };
-
-// |y - centre|^2 of a staged node (computed once per node and CTA).
-BIELCC_D float node_yy(float4 nd) { return fmaf(nd.x, nd.x, fmaf(nd.y, nd.y, nd.z * nd.z)); }
 
 // a / b by the approximate reciprocal alone (b positive and normal here, so the
 // scaling that __fdividef adds for large divisors is not needed).
@@ -390,17 +408,21 @@ BIELCC_D float fast_div(float a, float b) {
     return a * r;
 }
 
-// Shared head of the FP32 far node: nd = (y - centre, w), yy = |y - centre|^2.
+// Two FP32 values at a time (add, mul and fma .f32x2: one issue slot each).
+BIELCC_D float2 dup2(float v) { return make_float2(v, v); }
+
+// Shared head of the FP32 far node: n = the node, yy = |y - centre|^2.
 // q = |x - y|^2 - r0^2 = yy - 2 (y - centre).X carries no cancellation.
-// Returns 1/r and sets r, the weighted phase factor e = w e^{ik(r - r0)} and d = x - y.
+// Returns 1/r and sets r, the weighted phase factor e = w e^{ik(r - r0)} and the
+// components of d = x - y, each twice.
 template <bool CK, int MODE>
-BIELCC_D float far_head_f32(const PairF32& p, float4 nd, float yy, const KF32& kf, float& r_out, float& er, float& ei,
-                            float& dx, float& dy, float& dz) {
-    const float q = fmaf(nd.x, p.X2[0], fmaf(nd.y, p.X2[1], fmaf(nd.z, p.X2[2], yy)));
+BIELCC_D float far_head_f32(const PairF32& p, const NodeF32& n, const KF32& kf, float& r_out, float2& e, float2& dx,
+                            float2& dy, float2& dz) {
+    const float q = fmaf(n.a.x, p.X2[0], fmaf(n.a.z, p.X2[1], fmaf(n.b.x, p.X2[2], n.b.w)));
     const float r2 = p.r0sq + q;
     const float ir = rsqrtf(r2);
     const float r = r2 * ir;
-    float s, c, w = nd.w;
+    float s, c, w = n.b.z;
     if (CK) {
         const float dr = fast_div(q, r + p.r0);  // r - r0 without cancellation
         phase_f32<MODE>(kf.kr * dr, &s, &c);
@@ -408,98 +430,75 @@ BIELCC_D float far_head_f32(const PairF32& p, float4 nd, float yy, const KF32& k
     } else {
         phase_f32<MODE>(fast_div(q, fmaf(r, kf.ikr, p.r0k)), &s, &c);  // k (r - r0)
     }
-    dx = p.X[0] - nd.x;
-    dy = p.X[1] - nd.y;
-    dz = p.X[2] - nd.z;
-    er = w * c;
-    ei = w * s;
+    dx = __fadd2_rn(p.X[0], make_float2(n.a.x, n.a.y));
+    dy = __fadd2_rn(p.X[1], make_float2(n.a.z, n.a.w));
+    dz = __fadd2_rn(p.X[2], make_float2(n.b.x, n.b.y));
+    e = make_float2(w * c, w * s);
     r_out = r;
     return ir;
 }
 
+// acc += v * w, acc an (re, im) pair of the moments.
+BIELCC_D void fma_into(float (&acc)[2], float2 v, float2 w) {
+    const float2 o = __ffma2_rn(v, w, make_float2(acc[0], acc[1]));
+    acc[0] = o.x;
+    acc[1] = o.y;
+}
+
 // T += b d^T over the 6 symmetric entries, b = a2 d (complex a2).
-BIELCC_D void acc_sym6(float (&t)[6][2], float a2r, float a2i, float dx, float dy, float dz) {
-    const float bx_r = a2r * dx, bx_i = a2i * dx, by_r = a2r * dy, by_i = a2i * dy, bz_r = a2r * dz, bz_i = a2i * dz;
-    t[0][0] = fmaf(bx_r, dx, t[0][0]);
-    t[0][1] = fmaf(bx_i, dx, t[0][1]);
-    t[1][0] = fmaf(bx_r, dy, t[1][0]);
-    t[1][1] = fmaf(bx_i, dy, t[1][1]);
-    t[2][0] = fmaf(bx_r, dz, t[2][0]);
-    t[2][1] = fmaf(bx_i, dz, t[2][1]);
-    t[3][0] = fmaf(by_r, dy, t[3][0]);
-    t[3][1] = fmaf(by_i, dy, t[3][1]);
-    t[4][0] = fmaf(by_r, dz, t[4][0]);
-    t[4][1] = fmaf(by_i, dz, t[4][1]);
-    t[5][0] = fmaf(bz_r, dz, t[5][0]);
-    t[5][1] = fmaf(bz_i, dz, t[5][1]);
+BIELCC_D void acc_sym6(float (&t)[6][2], float2 a2, float2 dx, float2 dy, float2 dz) {
+    const float2 bx = __fmul2_rn(a2, dx), by = __fmul2_rn(a2, dy), bz = __fmul2_rn(a2, dz);
+    fma_into(t[0], bx, dx);
+    fma_into(t[1], bx, dy);
+    fma_into(t[2], bx, dz);
+    fma_into(t[3], by, dy);
+    fma_into(t[4], by, dz);
+    fma_into(t[5], bz, dz);
 }
 
-// One far node, FP32 (E and H moments). Real k leaves (S, T/3) in (a1, t):
-// the caller runs finish_real_k once the cell's nodes are summed.
-template <bool CK, int MODE>
-BIELCC_D void far_node_f32(Moments<float>& m, const PairF32& p, float4 nd, float yy, const KF32& kf) {
-    float r, er, ei, dx, dy, dz;
-    const float ir = far_head_f32<CK, MODE>(p, nd, yy, kf, r, er, ei, dx, dy, dz);
+// One far node, FP32 (E and H moments; GRAD false: the K moments alone, for the
+// collocation matrix). Real k leaves (S, T/3, -G) in (a1, t, g): the caller runs
+// finish_real_k once the cell's nodes are summed. Re and im parts go through the
+// packed forms, each with the roundings of the scalar one (64 + 2 instructions per
+// real-k node in scalar form, about 48 so; the pipe time is the same, but the far
+// kernels are bound by issue slots). Field of 8192 cells x 20,000 points 7.08 ->
+// 6.82 ms, 6.55 with 128 registers.
+template <bool CK, int MODE, bool GRAD = true>
+BIELCC_D void far_node_f32(Moments<float>& m, const PairF32& p, const NodeF32& n, const KF32& kf) {
+    float r;
+    float2 e, dx, dy, dz;
+    const float ir = far_head_f32<CK, MODE>(p, n, kf, r, e, dx, dy, dz);
     const float ir2 = ir * ir, ir3 = ir2 * ir;
     if (!CK) {
         const float beta = kf.kr * ir2;
-        const float ear = fmaf(ei, beta, er * ir3), eai = fmaf(-er, beta, ei * ir3);  // e alpha
-        m.a1r += ear;  // S
-        m.a1i += eai;
-        const float u3 = kf.k2r3 * ir3;                                               // k^2 / (3 r^3)
-        const float a2r = fmaf(ear, ir2, -er * u3), a2i = fmaf(eai, ir2, -ei * u3);  // e (alpha - u/3) / r^2
-        acc_sym6(m.t, a2r, a2i, dx, dy, dz);
-        m.g[0][0] = fmaf(-ear, dx, m.g[0][0]);
-        m.g[0][1] = fmaf(-eai, dx, m.g[0][1]);
-        m.g[1][0] = fmaf(-ear, dy, m.g[1][0]);
-        m.g[1][1] = fmaf(-eai, dy, m.g[1][1]);
-        m.g[2][0] = fmaf(-ear, dz, m.g[2][0]);
-        m.g[2][1] = fmaf(-eai, dz, m.g[2][1]);
+        const float2 ea = make_float2(fmaf(e.y, beta, e.x * ir3), fmaf(-e.x, beta, e.y * ir3));  // e alpha
+        const float2 S = __fadd2_rn(make_float2(m.a1r, m.a1i), ea);
+        m.a1r = S.x;
+        m.a1i = S.y;
+        const float u3 = kf.k2r3 * ir3;  // -k^2 / (3 r^3)
+        // e (alpha - u/3) / r^2
+        acc_sym6(m.t, __ffma2_rn(ea, dup2(ir2), __fmul2_rn(e, dup2(u3))), dx, dy, dz);
+        if (GRAD) {
+            fma_into(m.g[0], ea, dx);
+            fma_into(m.g[1], ea, dy);
+            fma_into(m.g[2], ea, dz);
+        }
         return;
     }
     const float f1r = kf.k2r * ir - ir3 - kf.ki * ir2;
     const float f1i = kf.kr * ir2 + kf.k2i * ir;
     const float f2r = 3.f * ir3 + 3.f * kf.ki * ir2 - kf.k2r * ir;
     const float f2i = -3.f * kf.kr * ir2 - kf.k2i * ir;
-    m.a1r = fmaf(er, f1r, fmaf(-ei, f1i, m.a1r));
-    m.a1i = fmaf(er, f1i, fmaf(ei, f1r, m.a1i));
-    const float a2r = (er * f2r - ei * f2i) * ir2, a2i = (er * f2i + ei * f2r) * ir2;
-    acc_sym6(m.t, a2r, a2i, dx, dy, dz);
-    const float ur = -kf.ki * r - 1.f, ui = kf.kr * r;
-    const float gr = (er * ur - ei * ui) * ir3, gi = (er * ui + ei * ur) * ir3;
-    m.g[0][0] = fmaf(gr, dx, m.g[0][0]);
-    m.g[0][1] = fmaf(gi, dx, m.g[0][1]);
-    m.g[1][0] = fmaf(gr, dy, m.g[1][0]);
-    m.g[1][1] = fmaf(gi, dy, m.g[1][1]);
-    m.g[2][0] = fmaf(gr, dz, m.g[2][0]);
-    m.g[2][1] = fmaf(gi, dz, m.g[2][1]);
-}
-
-// The K moments only (A1, T; no grad F) of one far node, FP32: the node
-// arithmetic of far_node_f32 for the collocation matrix, whose entries need
-// K_RotRot_Far alone. Real k leaves (S, T/3) as far_node_f32 does.
-template <bool CK, int MODE>
-BIELCC_D void far_node_f32_K(float& a1r, float& a1i, float (&t)[6][2], const PairF32& p, float4 nd, float yy,
-                             const KF32& kf) {
-    float r, er, ei, dx, dy, dz;
-    const float ir = far_head_f32<CK, MODE>(p, nd, yy, kf, r, er, ei, dx, dy, dz);
-    const float ir2 = ir * ir, ir3 = ir2 * ir;
-    if (!CK) {
-        const float beta = kf.kr * ir2;
-        const float ear = fmaf(ei, beta, er * ir3), eai = fmaf(-er, beta, ei * ir3);
-        a1r += ear;
-        a1i += eai;
-        const float u3 = kf.k2r3 * ir3;
-        acc_sym6(t, fmaf(ear, ir2, -er * u3), fmaf(eai, ir2, -ei * u3), dx, dy, dz);
-        return;
+    m.a1r = fmaf(e.x, f1r, fmaf(-e.y, f1i, m.a1r));
+    m.a1i = fmaf(e.x, f1i, fmaf(e.y, f1r, m.a1i));
+    acc_sym6(m.t, make_float2((e.x * f2r - e.y * f2i) * ir2, (e.x * f2i + e.y * f2r) * ir2), dx, dy, dz);
+    if (GRAD) {
+        const float ur = -kf.ki * r - 1.f, ui = kf.kr * r;
+        const float2 gg = make_float2((e.x * ur - e.y * ui) * ir3, (e.x * ui + e.y * ur) * ir3);
+        fma_into(m.g[0], gg, dx);
+        fma_into(m.g[1], gg, dy);
+        fma_into(m.g[2], gg, dz);
     }
-    const float f1r = kf.k2r * ir - ir3 - kf.ki * ir2;
-    const float f1i = kf.kr * ir2 + kf.k2i * ir;
-    const float f2r = 3.f * ir3 + 3.f * kf.ki * ir2 - kf.k2r * ir;
-    const float f2i = -3.f * kf.kr * ir2 - kf.k2i * ir;
-    a1r = fmaf(er, f1r, fmaf(-ei, f1i, a1r));
-    a1i = fmaf(er, f1i, fmaf(ei, f1r, a1i));
-    acc_sym6(t, (er * f2r - ei * f2i) * ir2, (er * f2i + ei * f2r) * ir2, dx, dy, dz);
 }
 
 }  // namespace bielcc_gpu

@@ -66,10 +66,10 @@ constexpr int kFarThreads = BIELCC_FAR_THREADS;
 #define BIELCC_FAR64_UNROLL_PRAGMA BIELCC_FAR_PRAGMA(BIELCC_FAR64_UNROLL)
 // Minimum resident CTAs per SM asked of the 1-RHS real-k mixed far kernel
 // (0: none, the compiler's own register choice, which the other variants
-// keep). 5 caps it at 96 registers without spills: 20 warps per SM (6: 80
-// registers, 8192 cells x 20,000 points 8.1 -> 9.0 ms).
+// keep). 4 allows 128 registers, no spills; 8192 cells x 20,000 points 6.55 ms
+// (5: 96 registers, 6.82 ms).
 #ifndef BIELCC_FAR_MINB
-#define BIELCC_FAR_MINB 5
+#define BIELCC_FAR_MINB 4
 #endif
 // The same for the 1-RHS real-k FP64 far kernel: 4 (128 registers) measured
 // slower than the compiler's own 168 (5120 triangles x 6001 points 9.6 against
@@ -170,7 +170,9 @@ BIELCC_D void contract(const Moments<F>& m, F pr, F pi, const F (*sj)[6], bool z
         if (!zeroR && takeH) {
 #pragma unroll
             for (int a = 0; a < 3; a++) {
-                const int b = (a + 1) % 3, c = (a + 2) % 3;  // (G x J)_a = G_b J_c - G_c J_b
+                // (G x J)_a = G_b J_c - G_c J_b, b = a + 1, c = a + 2 (the other way round for -G)
+                constexpr int o = !CK && Moments<F>::kNegG ? 2 : 1;
+                const int b = (a + o) % 3, c = (a + 3 - o) % 3;
                 const F hr = (m.g[b][0] * jr[c] - m.g[b][1] * ji[c]) - (m.g[c][0] * jr[b] - m.g[c][1] * ji[b]);
                 const F hi = (m.g[b][0] * ji[c] + m.g[b][1] * jr[c]) - (m.g[c][0] * ji[b] + m.g[c][1] * jr[b]);
                 acc[rr][6 + 2 * a] += (double)hr;
@@ -191,8 +193,8 @@ BIELCC_D void contract(const Moments<F>& m, F pr, F pi, const F (*sj)[6], bool z
 // Bound: issue slots. 8192 cells x 20,000 points, mixed, whole call: 26.0 ms with
 // all 64 nodes -> 8.3 with the rules -> 7.2 with the total-degree rules and a
 // shorter set-up (near test on the squared distance, e^{ik r0} in turns, phase
-// applied to J instead of the moments); ncu on 8000 points: 1114 warp instructions
-// per (warp, cell) before that last step, 76 % issue-active, FMA pipe 49 %. FP64,
+// applied to J instead of the moments) -> 6.55 with packed node arithmetic; ncu on
+// 8000 points: 804 warp instructions per (warp, cell), 67 % issue-active. FP64,
 // 5120 triangles x 6001 points: 11.9 -> 7.6 ms, FP64 pipe 68 %.
 // ways = 1: a CTA holds 128 points and every warp takes all cells of the split,
 // so that the warps run the same code at about the same time (with each warp at a
@@ -324,14 +326,13 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
                 RowBuf<NodeT>& rb = s_rows[warp];
                 if (k0 && lane < kc) v = row[k0 + lane];
                 __syncwarp();  // the previous chunk has been read
-                rb.nd[lane] = v;
-                if constexpr (MIXED) rb.yy[lane] = node_yy(v);
+                rb.put(lane, v);
                 __syncwarp();
                 if (!far) continue;
                 if constexpr (MIXED) {
 #define BIELCC_NODE_LOOP(MODE_)                                           \
     BIELCC_FAR_UNROLL_PRAGMA for (int i = 0; i < kc; i++)                 \
-        far_node_f32<CK, MODE_>(m, pf, rb.nd[i], rb.yy[i], kf);
+        far_node_f32<CK, MODE_>(m, pf, rb.get(i), kf);
                     switch (mode) {
                         case 0: BIELCC_NODE_LOOP(0) break;
                         case 1: BIELCC_NODE_LOOP(1) break;
@@ -343,7 +344,7 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
                 } else if (mode >= 0) {
 #define BIELCC_NODE64_LOOP(TD_)                                                                         \
     BIELCC_FAR64_UNROLL_PRAGMA for (int i = 0; i < kc; i++) {                                            \
-        const double4 y = rb.nd[i];                                                                      \
+        const double4 y = rb.get(i);                                                                      \
         far_node_f64<CK, true, TD_>(m, x[0] - y.x, x[1] - y.y, x[2] - y.z, y.w, a.k, k2r, k2i, d);       \
     }
                     switch (mode) {
@@ -355,7 +356,7 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
                 } else {
 #pragma unroll 2
                     for (int i = 0; i < kc; i++) {
-                        const double4 y = rb.nd[i];
+                        const double4 y = rb.get(i);
                         far_node_f64<CK, false>(m, x[0] - y.x, x[1] - y.y, x[2] - y.z, y.w, a.k, k2r, k2i, d);
                     }
                 }
