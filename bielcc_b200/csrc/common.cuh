@@ -46,6 +46,32 @@ BIELCC_D cplx eikr(double r, cplx k) {
     return {m * c, m * s};
 }
 
+// e^{i t} in FP64 from its Taylor series; the length follows a bound on |t|
+// (a template level, uniform over a cell): TD 0 |t| <= 0.5 (sin to t^13, cos
+// to t^14), TD 1 |t| <= 0.25 (t^11, t^12), TD 2 |t| <= 0.125 (t^9, t^10);
+// truncation below 3e-17 in each case. Coefficients are +-1/n!.
+template <int TD = 0>
+BIELCC_D void sincos_taylor64(double t, double* s, double* c) {
+    double t2 = t * t;
+    double ps;
+    if (TD == 0) ps = fma(fma(t2, -1.6059043836821613e-10, 2.5052108385441720e-08), t2, -2.7557319223985893e-06);
+    else if (TD == 1) ps = fma(t2, 2.5052108385441720e-08, -2.7557319223985893e-06);
+    else ps = -2.7557319223985893e-06;
+    ps = fma(t2, ps, 1.9841269841269841e-04);
+    ps = fma(t2, ps, -8.3333333333333333e-03);
+    ps = fma(t2, ps, 1.6666666666666667e-01);
+    *s = t - t * t2 * ps;
+    double pc;
+    if (TD == 0) pc = fma(fma(t2, 1.1470745597729725e-11, -2.0876756987868099e-09), t2, 2.7557319223985891e-07);
+    else if (TD == 1) pc = fma(t2, -2.0876756987868099e-09, 2.7557319223985891e-07);
+    else pc = 2.7557319223985891e-07;
+    pc = fma(t2, pc, -2.4801587301587302e-05);
+    pc = fma(t2, pc, 1.3888888888888889e-03);
+    pc = fma(t2, pc, -4.1666666666666667e-02);
+    pc = fma(t2, pc, 0.5);
+    *c = 1.0 - t2 * pc;
+}
+
 // ------------------------------------------------------------------ complex FP32
 struct cplxf {
     float re, im;

@@ -709,23 +709,139 @@ struct Lanes {
     BIELCC_D cplx sum(cplx v) const { return {sum(v.re), sum(v.im)}; }
 };
 
+// sqrt(s) and 1 / sqrt(s), to about an ulp, from the FP32 reciprocal root and one
+// third-order step; false where FP32 does not reach (and for NaN).
+BIELCC_D bool root_and_inverse(double s, double* r, double* ir) {
+    const float sf = (float)s;
+    if (!(sf > 1e-30f && sf < 1e30f)) return false;
+    double y = (double)rsqrtf(sf);
+    const double e = fma(-s * y, y, 1.0);
+    y = fma(y * e, fma(e, 0.375, 0.5), y);
+    const double d = s * y;
+    *r = fma(fma(-d, d, s), 0.5 * y, d);
+    *ir = y;
+    return true;
+}
+
+// e^{ikr} of one near pair's nodes and edge points. All of them lie within `rad` of
+// the mean vertex, so |r - r0| <= rad: where |Re k| r (mode 0) or |Re k| (r - r0)
+// (mode 1, times e^{ik r0}) stays below 1/2 the Taylor series takes the place of
+// sincos and its range reduction; mode 2 is eikr.
+struct NearPhase {
+    cplx k;
+    double r0, c0, s0, kk;  // kk = |k|^2
+    int mode;
+    BIELCC_D static NearPhase make(const double* x, const DCell& c, cplx k) {
+        NearPhase p;
+        double m[3] = {0., 0., 0.}, rad = 0.;
+        for (int v = 0; v < c.nv; v++)
+            for (int g = 0; g < 3; g++) m[g] += c.v[v][g] * (c.nv == 4 ? 0.25 : 1.0 / 3.0);
+        for (int v = 0; v < c.nv; v++) rad = fmax(rad, dist3(c.v[v], m));
+        p.k = k;
+        p.kk = cabs2(k);
+        p.r0 = p.s0 = 0.;
+        p.c0 = 1.;
+        const double d = dist3(x, m), kr = fabs(k.re);
+        if (kr * (d + rad) <= 0.499) {
+            p.mode = 0;
+        } else if (kr * rad <= 0.499) {
+            p.mode = 1;
+            p.r0 = d;
+            sincos(k.re * d, &p.s0, &p.c0);
+        } else {
+            p.mode = 2;
+        }
+        return p;
+    }
+    BIELCC_D cplx operator()(double r) const {
+        if (mode == 2) return eikr(r, k);
+        double s, c;
+        sincos_taylor64<0>(k.re * (r - r0), &s, &c);
+        cplx e = mk(c, s);
+        if (mode == 1) e = mk(c * c0 - s * s0, fma(c, s0, s * c0));
+        if (k.im == 0.0) return e;
+        const double a = exp(-r * k.im);
+        return mk(a * e.re, a * e.im);
+    }
+};
+
+// Near pairs are bound by FP64 instructions: with the library sincos, sqrt and 4 - 9
+// divisions per node (eval_cplx, quad_node) the assembly of 20,480 triangles took 20.0
+// ms, 1800 quads in FP64 1.81, a 3-pass FP64 field with 8000 near pairs 4.4; without
+// them 19.1, 1.62 and 4.0.
+// F_SIMPLEPOT_H, F_SIMPLEPOT_HM1 and F_GRADSIMPLEPOT_H (eval_cplx, kernel_lib.h) at
+// one node of a near pair. Outside the smoothing radius their brackets are powers of
+// 1 / r; eval_cplx takes the nodes inside it and the limits it treats apart.
+// GRAD (with F_SIMPLEPOT_H): F into out[0] and grad F into grad.
+template <int ID, bool GRAD = false>
+BIELCC_D void near_eval(const NearPhase& ph, const double* x, const double* y, const DKP& kp, cplx* out,
+                        cplx* grad = nullptr) {
+    const double d[3] = {x[0] - y[0], x[1] - y[1], x[2] - y[2]};
+    const double s = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    double r, ir;
+    if (!root_and_inverse(s, &r, &ir) || !(r >= kp.smoothR) || (ID == F_SIMPLEPOT_HM1 && !(ph.kk * s > 1e-13))) {
+        if constexpr (GRAD) eval_pot_and_grad(x, y, kp, out, grad);
+        else eval_cplx(ID, x, y, kp, out);
+        return;
+    }
+    const cplx e = ph(r);
+    if constexpr (ID == F_SIMPLEPOT_HM1) out[0] = mk((e.re - 1.) * ir, e.im * ir);
+    if constexpr (ID == F_SIMPLEPOT_H) out[0] = mk(e.re * ir, e.im * ir);
+    if constexpr (ID == F_GRADSIMPLEPOT_H || GRAD) {
+        const double w = ir * ir * ir, ur = (-r * ph.k.im - 1.) * w, ui = r * ph.k.re * w;
+        const cplx z = mk(e.re * ur - e.im * ui, e.re * ui + e.im * ur);
+        cplx* o = GRAD ? grad : out;
+#pragma unroll
+        for (int i = 0; i < 3; i++) o[i] = mk(d[i] * z.re, d[i] * z.im);
+    }
+}
+
 // Calls f(y, weight) for this lane's nodes of the n x n split; triangles: weight 1
-// (the sum is scaled by area / n / n, cell_scale). Nodes as integral_quad / integral_tri.
+// (the sum is scaled by area / n / n, cell_scale). The nodes of integral_quad /
+// integral_tri with their divisions taken out: a quad's sub-cell centre is the
+// bilinear map X(p, q) = A + q B + p C + p q D at the middle of the sub-square, and
+// its weight |dX/dq x dX/dp| / n^2; a triangle's sub-centroid has barycentric
+// coordinates in thirds of 1 / n.
 template <int G, typename Fn>
 BIELCC_D void cell_nodes(const Lanes<G>& g, const DCell& c, int n, Fn f) {
-    double y[3], s;
+    const double h = 1.0 / n;
+    double B[3], C[3], D[3], y[3];
     if (c.nv == 4) {
-        for (int q = g.l; q < n * n; q += G) {
-            quad_node(c.v, q / n, q % n, n, y, &s);
-            f(y, s);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            B[k] = c.v[1][k] - c.v[0][k];
+            C[k] = c.v[3][k] - c.v[0][k];
+            D[k] = (c.v[2][k] - c.v[3][k]) - B[k];
+        }
+        auto node = [&](int i, int j) {
+            const double p = (i + 0.5) * h, q = (j + 0.5) * h;
+            double m1[3], m2[3], nr[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                m1[k] = fma(p, D[k], B[k]);
+                m2[k] = fma(q, D[k], C[k]);
+                y[k] = fma(q, m1[k], fma(p, C[k], c.v[0][k]));
+            }
+            cross3(m1, m2, nr);
+            double r, ir;
+            const double s = nr[0] * nr[0] + nr[1] * nr[1] + nr[2] * nr[2];
+            f(y, (root_and_inverse(s, &r, &ir) ? r : sqrt(s)) * (h * h));
+        };
+        if (G == 1) {
+            for (int i = 0; i < n; i++)
+                for (int j = 0; j < n; j++) node(i, j);
+        } else {
+            for (int q = g.l; q < n * n; q += G) {
+                const int i = q / n;
+                node(i, q - i * n);
+            }
         }
         return;
     }
-    double pv[3], qv[3], rv[3];
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-        pv[k] = (c.v[1][k] - c.v[0][k]) / n;
-        qv[k] = (c.v[2][k] - c.v[0][k]) / n;
-        rv[k] = (c.v[2][k] - c.v[1][k]) / n;
+        B[k] = c.v[1][k] - c.v[0][k];
+        C[k] = c.v[2][k] - c.v[0][k];
     }
     int i = 0, first = 0;  // row of the node (2 (n - i) - 1 of them) and its first node
     for (int q = g.l; q < n * n; q += G) {
@@ -734,10 +850,9 @@ BIELCC_D void cell_nodes(const Lanes<G>& g, const DCell& c, int n, Fn f) {
             i++;
         }
         const int j = (q - first) >> 1;
-        for (int k = 0; k < 3; k++) {
-            const double B = c.v[0][k] + (i + 1) * pv[k] + j * qv[k], A = B - pv[k];
-            y[k] = ((q - first) & 1) ? (B + (B + rv[k]) + (B + qv[k])) / 3.0 : (B + A + (A + qv[k])) / 3.0;
-        }
+        const double third = ((q - first) & 1) ? 2.0 / 3.0 : 1.0 / 3.0, s = (i + third) * h, t = (j + third) * h;
+#pragma unroll
+        for (int k = 0; k < 3; k++) y[k] = fma(t, C[k], fma(s, B[k], c.v[0][k]));
         f(y, 1.0);
     }
 }
@@ -746,14 +861,16 @@ BIELCC_D cplx cell_scale(cplx v, const DCell& c, double area, int n) {
 }
 
 // integral_cell over a group.
-template <int G>
-BIELCC_D void group_integral_cell(const Lanes<G>& g, int id, const double* x, const DCell& c, DKP& kp, int idim,
+template <int ID, int G>
+BIELCC_D void group_integral_cell(const Lanes<G>& g, const NearPhase& ph, const double* x, const DCell& c, DKP& kp,
                                   int n_start, int p_max, double eps, cplx* res) {
+    constexpr int idim = ID == F_GRADSIMPLEPOT_H ? 3 : 1;
     const double area = c.nv == 3 ? tri_area(c.v[0], c.v[1], c.v[2]) : 0.;
     adaptive<cplx>(n_start, p_max, eps, idim, kp, res, [&](int n, cplx* acc) {
         cplx ff[3], sum[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
         cell_nodes<G>(g, c, n, [&](const double* y, double w) {
-            eval_cplx(id, x, y, kp, ff);
+            near_eval<ID>(ph, x, y, kp, ff);
+#pragma unroll
             for (int q = 0; q < idim; q++) sum[q] = madd(sum[q], ff[q], w);
         });
         for (int q = 0; q < idim; q++) acc[q] = cell_scale(g.sum(sum[q]), c, area, n);
@@ -761,9 +878,9 @@ BIELCC_D void group_integral_cell(const Lanes<G>& g, int id, const double* x, co
 }
 
 // integral_seg over a group.
-template <int G>
-BIELCC_D void group_integral_seg(const Lanes<G>& g, int id, const double* a, const double* b, const double* x, DKP& kp,
-                                 int n_start, int p_max, double eps, cplx* res) {
+template <int ID, int G>
+BIELCC_D void group_integral_seg(const Lanes<G>& g, const NearPhase& ph, const double* a, const double* b,
+                                 const double* x, DKP& kp, int n_start, int p_max, double eps, cplx* res) {
     adaptive<cplx>(n_start, p_max, eps, 3, kp, res, [&](int n, cplx* acc) {
         double d[3], y[3];
         for (int k = 0; k < 3; k++) d[k] = (b[k] - a[k]) / n;
@@ -771,7 +888,7 @@ BIELCC_D void group_integral_seg(const Lanes<G>& g, int id, const double* a, con
         cplx ff[3], sum[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
         for (int i = g.l; i < n; i += G) {
             for (int k = 0; k < 3; k++) y[k] = a[k] + (i + 0.5) * d[k];
-            eval_cplx(id, x, y, kp, ff);
+            near_eval<ID>(ph, x, y, kp, ff);
             for (int q = 0; q < 3; q++) sum[q] = madd(sum[q], ff[q], dl);
         }
         for (int q = 0; q < 3; q++) acc[q] = g.sum(sum[q]);
@@ -783,8 +900,8 @@ BIELCC_D void group_integral_seg(const Lanes<G>& g, int id, const double* a, con
 // lanes each, every lane with the radius its edge starts from (shrunk per edge as
 // `adaptive` shrinks it); else edge after edge.
 template <int G>
-BIELCC_D void group_K0_matrix(const Lanes<G>& g, const double* x, const DCell& c, DKP& kp, int n_seg, int p_seg,
-                              double eps, cplx (*mat)[3]) {
+BIELCC_D void group_K0_matrix(const Lanes<G>& g, const NearPhase& ph, const double* x, const DCell& c, DKP& kp,
+                              int n_seg, int p_seg, double eps, cplx (*mat)[3]) {
     double nrm[3], nu[3];
     cell_normal(c, nrm);
     for (int p = 0; p < 3; p++)
@@ -806,7 +923,7 @@ BIELCC_D void group_K0_matrix(const Lanes<G>& g, const double* x, const DCell& c
             cplx ff[3], sum[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
             for (int i = g.l & (L - 1); i < n_seg; i += L) {
                 for (int k = 0; k < 3; k++) y[k] = A[k] + (i + 0.5) * d[k];
-                eval_cplx(F_GRADSIMPLEPOT_H, x, y, kp, ff);
+                near_eval<F_GRADSIMPLEPOT_H>(ph, x, y, kp, ff);
                 for (int q = 0; q < 3; q++) sum[q] = madd(sum[q], ff[q], dl);
             }
             for (int p = 0; p < 3; p++)
@@ -821,7 +938,7 @@ BIELCC_D void group_K0_matrix(const Lanes<G>& g, const double* x, const DCell& c
         const double* A = c.v[e];
         const double* B = c.v[e + 1 == c.nv ? 0 : e + 1];
         cplx ks[3];
-        group_integral_seg<G>(g, F_GRADSIMPLEPOT_H, A, B, x, kp, n_seg, p_seg, eps, ks);
+        group_integral_seg<F_GRADSIMPLEPOT_H>(g, ph, A, B, x, kp, n_seg, p_seg, eps, ks);
         edge_nu(A, B, nrm, nu);
         for (int p = 0; p < 3; p++)
             for (int q = 0; q < 3; q++) mat[p][q] += ks[p] * (-nu[q]);
@@ -836,6 +953,7 @@ BIELCC_D void group_K0_matrix(const Lanes<G>& g, const double* x, const DCell& c
 template <int G>
 BIELCC_D void near_pair_moments(const Lanes<G>& g, const double* x, const DCell& cl, cplx k, const DNP& np, cplx* o) {
     const double dm = cell_diam(cl);
+    const NearPhase ph = NearPhase::make(x, cl, k);
     cplx sF[1], gr[3], M[3][3];
     if (np.p_max == 1) {
         // one quadrature pass for both surface integrals: K_RotRot_Near_Smooth's
@@ -849,7 +967,7 @@ BIELCC_D void near_pair_moments(const Lanes<G>& g, const double* x, const DCell&
         sF[0] = gr[0] = gr[1] = gr[2] = mk(0, 0);
         cell_nodes<G>(g, cl, np.n_start, [&](const double* y, double w) {
             cplx f[1], gg[3];
-            eval_pot_and_grad(x, y, pS, f, gg);
+            near_eval<F_SIMPLEPOT_H, true>(ph, x, y, pS, f, gg);
             sF[0] = madd(sF[0], f[0], w);
             for (int q = 0; q < 3; q++) gr[q] = madd(gr[q], gg[q], w);
         });
@@ -865,8 +983,8 @@ BIELCC_D void near_pair_moments(const Lanes<G>& g, const double* x, const DCell&
         pF.smoothRMin = np.eps;    // K_RotRot_Near_Smooth's surface part (K.h:51-67)
         pR.smoothRMin = dm / 100.;  // R_Rot_Smooth (R.h:46-61)
         pF.k = pR.k = k;
-        group_integral_cell<G>(g, F_SIMPLEPOT_H, x, cl, pF, 1, np.n_start, np.p_max, np.eps, sF);
-        group_integral_cell<G>(g, F_GRADSIMPLEPOT_H, x, cl, pR, 3, np.n_start, np.p_max, np.eps, gr);
+        group_integral_cell<F_SIMPLEPOT_H>(g, ph, x, cl, pF, np.n_start, np.p_max, np.eps, sF);
+        group_integral_cell<F_GRADSIMPLEPOT_H>(g, ph, x, cl, pR, np.n_start, np.p_max, np.eps, gr);
     }
     // contour part (K.h:56-72): K0 with the shared, shrinking segment radius
     DKP pG;
@@ -874,7 +992,7 @@ BIELCC_D void near_pair_moments(const Lanes<G>& g, const double* x, const DCell&
     pG.smoothR = np.rs_seg * dm / np.n_start_seg;
     pG.smoothRMin = np.eps;
     pG.k = k;
-    group_K0_matrix<G>(g, x, cl, pG, np.n_start_seg, np.p_max_seg, np.eps, M);
+    group_K0_matrix<G>(g, ph, x, cl, pG, np.n_start_seg, np.p_max_seg, np.eps, M);
     auto put = [&](int q, cplx v) {
         if (g.l == (q & (G - 1))) o[q] = v;
     };
@@ -910,15 +1028,16 @@ BIELCC_D void group_hs_colloc(const Lanes<G>& g, const double* x, const DCell& c
     } else {
         a = integral_1divr_dev(c, x);
     }
+    const NearPhase ph = NearPhase::make(x, c, k);
     DKP kp, ps;
     dkp_zero(kp);
     kp.smoothR = kp.smoothRMin = kMachineZero;
     kp.k = k;
     ps = kp;
     cplx I[1];
-    group_integral_cell<G>(g, F_SIMPLEPOT_HM1, x, c, kp, 1, np.n_start, np.p_max, np.eps, I);
+    group_integral_cell<F_SIMPLEPOT_HM1>(g, ph, x, c, kp, np.n_start, np.p_max, np.eps, I);
     const cplx s = mk(a + I[0].re, I[0].im) * k * k / kFourPi;
-    group_K0_matrix<G>(g, x, c, ps, np.n_start_seg, np.p_max_seg, np.eps, mat);
+    group_K0_matrix<G>(g, ph, x, c, ps, np.n_start_seg, np.p_max_seg, np.eps, mat);
     for (int p = 0; p < 3; p++)
         for (int q = 0; q < 3; q++) {
             mat[p][q] = mat[p][q] / kFourPi;

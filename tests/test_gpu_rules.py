@@ -3,7 +3,7 @@ rule that a distance, cell and k allow equals the oracle's full n x n sum, over
 the splits where levels appear, and on cells where the Jacobian is no polynomial
 (twisted, reversed corner), vanishes (collapsed edge) or is strongly graded.
 
-Tolerances: a pair's truncation is at most 3e-17 (FP64) / 4e-9 (mixed) of
+Tolerances: a pair's truncation is at most 3e-17 (FP64) / 1e-8 (mixed) of
 sum w |F|; what remains is rounding, an ulp or so per operation: 1e-14 for
 the few cells summed here in FP64, plus the rounding of the phase, k r ulps on
 either side, and 1.5e-7 rms per pair in FP32."""
@@ -104,4 +104,33 @@ def test_non_finite_points_reach_the_result(gctx, precision):
     keep = ~bad
     Eo, _ = oracle.field_EH(cells, J, 2.0, pts[keep])
     assert rel_l2(E[0][keep], Eo[0]) < (1e-12 if precision == "fp64" else 1e-6)
+    m.close()
+
+
+@pytest.mark.parametrize("p_max", [1, 2])
+@pytest.mark.parametrize("nv", [3, 4])
+@pytest.mark.parametrize("n_start,k", [(3, 0.5), (8, 0.5), (8, 5.0), (7, 60.0), (8, 5.0 + 2.0j), (5, 0.3 + 0.1j), (8, 0.0)])
+def test_near_pairs_all_phase_forms(gctx, n_start, k, nv, p_max):
+    """Near pairs where |k| r, only |k| (r - r0) or neither stays below 1/2, inside and
+    outside the smoothing radius. Points lie within a diameter of every cell, at least
+    h = 0.01 off its nodes, whose positions (|y| < 4) carry 2 ulps on either side: 3 of
+    that over h for the 1/r^3 terms, and an ulp or so per operation."""
+    cells = _cells(nv)
+    n, h = len(cells), 0.01
+    rng = np.random.default_rng(11)
+    J = rng.standard_normal((1, n, 3)) + 1j * rng.standard_normal((1, n, 3))
+    ctr = cells.mean(axis=1)
+    nrm = np.cross(cells[:, 1] - cells[:, 0], cells[:, 2] - cells[:, 0])
+    nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
+    pts = np.concatenate([ctr + s * nrm for s in (0.05, 0.02 + h, 0.11)])
+    npm = abi.NumParam.default(n_start=n_start, p_max=p_max)
+    m = gctx.mesh(cells)
+    E, H, rep = gctx.field_EH(m, J, k, pts, numparam=npm, precision="fp64")
+    assert rep.n_near_pairs >= n
+    Eo, Ho = oracle.field_EH(cells, J, k, pts, npm)
+    tol = 3 * 4 * 2.0 ** -52 * 4 / h + 2e-14
+    assert rel_l2(E, Eo) < tol and rel_l2(H, Ho) < tol
+    if k != 0.0:
+        A, _ = gctx.assemble_K(m, k, numparam=npm, layout=abi.LAYOUT_FULL3)
+        assert rel_l2(A, oracle.assemble_K(cells, k, npm, layout=abi.LAYOUT_FULL3)) < tol
     m.close()
