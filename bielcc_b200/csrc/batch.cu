@@ -770,8 +770,12 @@ constexpr int kConCells = 16;
 #ifndef BIELCC_CON_R
 #define BIELCC_CON_R 4
 #endif
+// Resident CTAs per SM asked of it: 2 leaves the compiler 166 registers (three CTAs
+// fit), so that a cell's moments and currents load ahead of the multiply-adds. Replay
+// of 6 meshes x 2000 points x 1 - 64 currents 3.09 ms; 3 (156 registers) 3.14; 4 (128)
+// 3.51; 8 right-hand sides per thread 3.4 - 3.8.
 #ifndef BIELCC_CON_MINB
-#define BIELCC_CON_MINB 4
+#define BIELCC_CON_MINB 2
 #endif
 constexpr int kConR = BIELCC_CON_R;
 constexpr int kConSP = kBW * kConR * (kSP / (kBW * BatchCfg<true>::R) > 1 ? kSP / (kBW * BatchCfg<true>::R) : 1);
