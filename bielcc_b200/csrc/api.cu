@@ -346,7 +346,22 @@ int field_device_batched(bielcc_ctx ctx, const FieldArgs& a, cudaStream_t s, bie
     const int S = a.n_rhs;
     const double single = (S / 4) * 1.1 + (S % 4) / 2 + (S % 2);  // single-job launches, in quadratures
     if (single * busy <= 1.05) return BIELCC_OK;
-    TRY(w.ws->ensure(bp.ws_bytes));
+    // Still fewer than two items per resident CTA: up to kBatchRangesAlone ranges, as
+    // far as the partial sums stay small beside the L2 (4050 cells x 2000 points x 24
+    // currents: 378 items on 444 CTAs 1.61 ms, 882 items 1.42).
+    const int tiles = (a.n_pts + 31) / 32, ranges = (2 * bp.workers() + tiles - 1) / tiles;
+    bool sized = false;
+    if (ranges > bp.jobs[0].ranges && ranges > kBatchRanges) {
+        const int mr = std::min(ranges, kBatchRangesAlone);
+        BatchPlan fine;
+        plan_batch(fine, std::vector<JobDev>{d}, far_split_n(a.np), mixed, 1.0e5, ctx->batch_tc, split, mr);
+        if (fine.items.size() > bp.items.size() && fine.ws_bytes <= ((size_t)256 << 20) &&
+            w.ws->ensure(fine.ws_bytes) == BIELCC_OK) {
+            bp = std::move(fine);
+            sized = true;
+        }
+    }
+    if (!sized) TRY(w.ws->ensure(bp.ws_bytes));
     BatchDevPtrs dp;
     int l1 = 0, l2 = 0;
     TRY_CUDA(batch_stage1(bp, w.ws->p, a.np.analytic_calc, far_split_n(a.np), a.k.im != 0., s, &dp, &l1));

@@ -1517,17 +1517,16 @@ void split_grids(int& grid_mom, int& grid_con) {
 // evaluations per item, a per-context autotuned constant), never on the other
 // jobs of the batch, so a job's summation order - and its result - is the same
 // alone and in any mix. Ranges are multiples of 32 cells (near-mask words).
-int batch_cells_per_range(int n_cells, int n_rhs, int n_start, double item_cost) {
+int batch_cells_per_range(int n_cells, int n_rhs, int n_start, double item_cost, int max_ranges) {
     const double per_cell = (double)kBP * ((double)n_start * n_start + 1.2 * n_rhs);
-    // at most kMaxRanges ranges per job: bounds the partial sums to kMaxRanges x (S x 12 x P) doubles
-    constexpr int kMaxRanges = 6;
+    // max_ranges bounds the partial sums to that many times S x 12 x P doubles
     int cpr = (int)std::min<double>(n_cells, std::max(32.0, item_cost / per_cell));
-    cpr = std::max(cpr, (n_cells + kMaxRanges - 1) / kMaxRanges);
+    cpr = std::max(cpr, (n_cells + max_ranges - 1) / max_ranges);
     return (cpr + 31) / 32 * 32;
 }
 
 void plan_batch(BatchPlan& bp, const std::vector<JobDev>& jobs_in, int n_start, bool mixed, double item_cost,
-                bool allow_tc, size_t split_cap) {
+                bool allow_tc, size_t split_cap, int max_ranges) {
     bp.jobs = jobs_in;
     bp.mixed = mixed;
     bp.tc = mixed && allow_tc && n_start <= 8;
@@ -1545,7 +1544,7 @@ void plan_batch(BatchPlan& bp, const std::vector<JobDev>& jobs_in, int n_start, 
         pt_off += j.n_pts;
         for (int p = 0; p < j.n_pts; p++) bp.pt_job.push_back((int)ji);
         const double per_cell = (double)kBP * (nodes + 1.2 * j.n_rhs);
-        const int cpr = batch_cells_per_range(j.n_cells, j.n_rhs, n_start, item_cost);
+        const int cpr = batch_cells_per_range(j.n_cells, j.n_rhs, n_start, item_cost, max_ranges);
         j.cells_per_range = cpr;
         j.ranges = (j.n_cells + cpr - 1) / cpr;
         j.n_words = (j.n_cells + 31) / 32;

@@ -286,16 +286,18 @@ struct BatchDevPtrs {
 cudaError_t batch_status_to_host(const BatchDevPtrs& d, long long* h, cudaStream_t s);
 inline bool batch_timed_out(const long long* h) { return h[3] != 0; }
 
-// Cells per item of one job (a multiple of 32; at most 6 ranges per job);
-// depends on the job and item_cost only.
-int batch_cells_per_range(int n_cells, int n_rhs, int n_start, double item_cost);
+// Cells per item of one job (a multiple of 32; at most max_ranges ranges per job);
+// depends on the job, item_cost and max_ranges only. Batches take kBatchRanges; a job
+// that runs alone and leaves CTAs idle up to kBatchRangesAlone.
+constexpr int kBatchRanges = 6, kBatchRangesAlone = 24;
+int batch_cells_per_range(int n_cells, int n_rhs, int n_start, double item_cost, int max_ranges = kBatchRanges);
 // allow_tc: mixed batches that qualify run the tensor-core contraction
 // (bielcc_ctx_set_batch_tensor_cores); otherwise the CUDA-core kernel.
 // split_cap > 0: mixed batches with n_start <= 8 run the split pipeline with
 // a moments buffer of at most split_cap bytes (waves of items); 0: the fused
 // kernel.
 void plan_batch(BatchPlan& bp, const std::vector<JobDev>& jobs, int n_start, bool mixed, double item_cost,
-                bool allow_tc = true, size_t split_cap = 0);
+                bool allow_tc = true, size_t split_cap = 0, int max_ranges = kBatchRanges);
 // bytes of one moments block of the split pipeline (8 cells x 20 moments x 32 points, FP32)
 size_t moments_block_bytes();
 cudaError_t batch_stage1(BatchPlan& bp, void* ws, double analytic_calc, int n_start, bool ck, cudaStream_t s,
