@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
         for (int q = threadIdx.x; q < nc; q += kAsmThreads) {
             s_cell[q] = near_cell(a.geo[c0 + q], a.analytic_calc);
             if constexpr (MIXED) s_mode[q] = phase_mode((float)fabs(a.k.re) * a.rho32[c0 + q]);
-            else s_mode[q] = !CK && fabs(a.k.re) * (double)a.rho32[c0 + q] * (1.0 + 1e-6) <= 0.5;
+            else s_mode[q] = phase_range64(a.k, (double)a.rho32[c0 + q]) <= 0.5;
         }
         {
             const float kabs = rule_kabs(a.k);
@@ -309,7 +309,14 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
                     turn_f32(d * (a.k.re * kInvTwoPi), CK ? exp(-a.k.im * d) * kInvFourPi : kInvFourPi, &phr, &phi);
                 } else {
                     mm.zero();
-                    if (mode) sincos(a.k.re * d, &P0i, &P0r);
+                    if (mode) {
+                        sincos(a.k.re * d, &P0i, &P0r);
+                        if (CK) {
+                            const double am = exp(-a.k.im * d);
+                            P0r *= am;
+                            P0i *= am;
+                        }
+                    }
                 }
                 for (int k0 = 0; k0 < cnt; k0 += kRowChunk) {
                     const int kc = min(kRowChunk, cnt - k0);

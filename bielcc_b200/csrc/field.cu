@@ -264,8 +264,8 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
             if constexpr (MIXED) {
                 s_mode[i] = phase_mode((float)fabs(a.k.re) * a.rho32[c0 + i]);
             } else {  // FP64 phase split when the cell's phase range is small (farnode.cuh sincos_taylor64)
-                const double th = fabs(a.k.re) * (double)a.rho32[c0 + i] * (1.0 + 1e-6);
-                s_mode[i] = CK || !(th <= 0.5) ? -1 : (th <= 0.125 ? 2 : (th <= 0.25 ? 1 : 0));
+                const double th = phase_range64(a.k, (double)a.rho32[c0 + i]);
+                s_mode[i] = !(th <= 0.5) ? -1 : (th <= 0.125 ? 2 : (th <= 0.25 ? 1 : 0));
             }
         }
         {
@@ -320,6 +320,11 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
                 turn_f32(d * kturn, CK ? exp(-a.k.im * d) : 1.0, &P0r, &P0i);
             } else if (mode >= 0) {
                 sincos(a.k.re * d, &P0i, &P0r);
+                if (CK) {
+                    const double am = exp(-a.k.im * d);
+                    P0r *= am;
+                    P0i *= am;
+                }
             }
             for (int k0 = 0; k0 < cnt; k0 += kRowChunk) {
                 const int kc = min(kRowChunk, cnt - k0);
