@@ -296,7 +296,7 @@ struct FieldArgs {
 // each. The job runs as a one-job batch when the single-job launches (about
 // one quadrature each, 1.1 for a 4-RHS launch) outweigh the batched kernel's
 // idle SMs on a small point set (its work items over its resident CTAs).
-// Measured on 8192 cells x 20,000 points (mixed): S = 2 28.4 ms single-job
+// Measured on 8192 cells x 20,000 points (mixed, 64-node rows): S = 2 28.4 ms single-job
 // against 31.6 batched, S = 3 53.8 against 31.9, S = 4 34.9 against 32.0.
 // Returns false when the call is left to the single-job path.
 int field_device_batched(bielcc_ctx ctx, const FieldArgs& a, cudaStream_t s, bielcc_report* rep,

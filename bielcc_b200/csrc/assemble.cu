@@ -186,7 +186,7 @@ BIELCC_D void write_block(const AsmArgs& a, int i, int j, const double (&Kr)[3][
 
 // Minimum resident CTAs per SM asked of the real-k mixed far kernel (0: the
 // compiler's own register choice, which the other variants keep). 5 gives 96
-// registers without spills (20,480 triangles: 65.0 -> 62.4 ms).
+// registers without spills (20,480 triangles 20.0 ms; 4: 20.1; 6: 20.6).
 #ifndef BIELCC_ASM_MINB
 #define BIELCC_ASM_MINB 5
 #endif
@@ -201,8 +201,10 @@ BIELCC_D void write_block(const AsmArgs& a, int i, int j, const double (&Kr)[3][
 // (complex128: four) columns at a time in whole lines; near blocks are written
 // too (as zeros) and overwritten by asm_near_kernel, which always follows.
 // 20,480 triangles, mixed, complex64, whole call: 65.6 ms with all 64 nodes and
-// direct writes, 28.2 with the rules, 23.3 with rows staged per warp and whole-line
-// writes (this kernel 17.1 of it; bound by issue slots, 13.4 GB written).
+// direct writes, 28.2 with the rules, 20.0 with rows staged per warp and whole-line
+// writes (this kernel 16 of it: node loops 8, the pairs' set-up and projection 6,
+// writes 1; bound by issue slots, 72 % active; 13.4 GB written). Now 18.7 with the
+// near blocks' short forms.
 // ways = 4: 80 triangles, FP64, 0.70 -> 0.28 ms.
 template <bool CK, bool MIXED, bool MARKS = false, bool STAGE = false>
 __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB : 0)

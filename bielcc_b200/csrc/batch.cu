@@ -6,14 +6,14 @@
 // next item from a device counter. An item walks its cell range in chunks:
 //   phase A — warp w evaluates the far-field moments (A1, T, G: 20 values,
 //             farnode.cuh) of cells w, w+4, ... of the chunk for its 32 points
-//             and stores them in shared memory (node tiles staged with 128-bit
-//             loads, one observation point per lane);
+//             and stores them in shared memory (one observation point per lane,
+//             the shortest row of nodes the cells allow, rules.cu);
 //   phase B — the same threads contract the chunk's moments with the
 //             right-hand sides, staged in shared memory a pass of kSP at a time
 //             (the moments stay), R RHS per thread held in registers, and add
 //             the result into the job's partial sums.
 // Extra right-hand sides therefore cost ~72 FP32 operations per pair instead
-// of the 64-node integrand. Near cells (get_field.h:58) are flagged in the
+// of a quadrature. Near cells (get_field.h:58) are flagged in the
 // job's near mask and handled by the FP64 near-pair path afterwards, exactly
 // as in the single-job pipeline. Summation order depends only on the job
 // itself (its ranges and chunks), never on the other jobs of the batch.
@@ -37,10 +37,9 @@ constexpr int kBW = 4;    // warps
 // Mixed form: cells per chunk at n_start <= 8 (CH32), right-hand sides staged
 // per pass (SP; a chunk's moments are computed once and contracted pass by
 // pass), and resident CTAs per SM the kernel is compiled for (MINB).
-// Measured on the 256-mesh batch (B200), cells / RHS per pass / CTAs per SM:
-// 16 / 16 / 3 (168 registers, 73 KB smem) 680 ms; 12 / 16 / 3 709 ms;
-// 16 / 64 / 2 (234 registers, 109 KB) 760 ms; 12 / 16 / 4 787 ms;
-// 8 / 16 / 4 (128 registers) 888 ms.
+// Measured on 12 meshes x 2000 points x 1 - 64 RHS, cells / RHS per pass / CTAs per SM:
+// 16 / 16 / 3 (168 registers) 13.5 ms; 16 / 16 / 4 (128 registers) 14.3; 24 / 16 / 3
+// 15.1; 16 / 32 / 3 13.9; 16 / 64 / 3 17.2; 16 / 32 / 2 with 8 RHS per thread 17.4.
 #ifndef BIELCC_BATCH_CH32
 #define BIELCC_BATCH_CH32 16
 #endif
@@ -51,11 +50,8 @@ constexpr int kBW = 4;    // warps
 #define BIELCC_BATCH_MINB 3
 #endif
 // Mixed form: phase A two cells per warp at a time (TWO = 1) or one; RHS per
-// thread in phase B (R; SP a multiple of 4 R). Measured on the 256-mesh batch
-// (cells / SP / CTAs per SM / TWO / R): 16 / 16 / 3 / 1 / 4 (164 registers)
-// 659 ms; 16 / 16 / 3 / 0 / 4 707 ms; 12 / 8 / 4 / 0 / 2 (128 registers)
-// 705 ms; 8 / 8 / 4 / 1 / 2 734 ms; 8 / 8 / 5 / 0 / 2 (96 registers, 20 warps
-// per SM) 865 ms: the two-cell node loop's second dependency chain is worth
+// thread in phase B (R; SP a multiple of 4 R). One cell at a time at 4 CTAs per SM:
+// 16.5 ms against 13.5: the two-cell node loop's second dependency chain is worth
 // more than extra warps.
 #ifndef BIELCC_BATCH_TWO
 #define BIELCC_BATCH_TWO 1
@@ -67,7 +63,7 @@ constexpr int kSP = BIELCC_BATCH_SP;  // right-hand sides staged per pass (a mul
 // Unrolling of the one-cell and two-cell phase-A node loops. Three CTAs of
 // different jobs (different phase polynomials) share an SM's instruction
 // cache: the two-cell loop, already two dependency chains wide, is not
-// unrolled (256-mesh batch: 681 ms unrolled x2, 661 ms not unrolled).
+// unrolled (13.8 ms unrolled x2, 13.5 not unrolled).
 #ifndef BIELCC_BATCH_U1
 #define BIELCC_BATCH_U1 4
 #endif
@@ -75,7 +71,7 @@ constexpr int kSP = BIELCC_BATCH_SP;  // right-hand sides staged per pass (a mul
 #define BIELCC_BATCH_U2 1
 #endif
 // FP64 form: unrolling of the node loop and resident CTAs per SM asked of the
-// kernel. Measured on 64 meshes of the batched workload (unroll / CTAs per SM):
+// kernel. Measured with 64-node rows on 64 meshes (unroll / CTAs per SM):
 // 1 / 3 (168 registers, no spills) 284 ms; 2 / 3 284 ms; 4 / 3 322-327 ms;
 // 1 / 2 (206 registers) 338 ms; 8 / 2 388 ms; 8 / 3 436 ms; 16 / 3 491 ms.
 // Unrolling costs instruction-cache misses (CTAs of different jobs share an
