@@ -33,16 +33,24 @@ sys.path.insert(0, ROOT)
 
 METRIC = "E+H cell*point evals/s (mixed, <=1e-6 rel-L2 vs FP64)"
 UNIT = "pairs/s"
-# Algorithmic flops of one far pair with the default 8 x 8 split: 64 nodes x
-# 130 real flops for the fused K (F_RotRotSimplePot_H) + R (F_GradSimplePot_H)
-# integrand, transcendentals (sqrt, 1/r, sincos) not counted.
+# Flops of one far pair: its row's nodes x 130 real flops for the fused K
+# (F_RotRotSimplePot_H) + R (F_GradSimplePot_H) integrand, transcendentals (sqrt,
+# 1/r, sincos) not counted. The far kernels stand rows of 7-36 nodes in for the
+# 8 x 8 split's 64 (csrc/rules.cu); the mean row length per far pair was counted
+# on the default workload in the mixed and the FP64 form and on 64 of the batch's
+# 256 meshes.
 FLOPS_PER_NODE = 130
-NODES_PER_PAIR = 64
-FLOPS_PER_FAR_PAIR = FLOPS_PER_NODE * NODES_PER_PAIR
+NODES_MIXED, NODES_FP64, NODES_BATCH = 9.0, 30.5, 10.3
 # Algorithmic flops of one moment contraction per (point, cell, RHS) in the
 # batched kernel: (A1 I + T) J is 9 complex multiply-adds (72 flops), G x J
 # three components of two complex products and a difference (42 flops).
 FLOPS_PER_RHS_CONTRACTION = 114
+
+
+def far_pair_flops(nodes, rhs=1):
+    return FLOPS_PER_NODE * nodes + FLOPS_PER_RHS_CONTRACTION * rhs
+
+
 # moments buffer of the split batched pipeline (the library's default)
 SPLIT_MOMENTS_BYTES = 16 << 30
 
@@ -341,8 +349,8 @@ def run_batched(args, ctx, torch, dev, stream, flush, fp64_single_rhs_value, pea
     for m, _, _ in keep:
         m.close()
     value = rhs_pairs / (ms * 1e-3)
-    # Roofline of the whole launch against the measured FP32 FMA peak: 8320
-    # flops per (point, cell) quadrature (the moments) plus 114 per (point,
+    # Roofline of the whole launch against the measured FP32 FMA peak: the mean
+    # row's flops per (point, cell) quadrature (the moments) plus 114 per (point,
     # cell, RHS) for the contraction on the CUDA cores. The tensor-core form
     # runs the moments on the FP32 pipe and the contraction as 2 M = 128 MMAs
     # of K = 6 and N = 2 min(16, S8 - 16 g) (S8 = S rounded up to 8) per 32-point
@@ -364,8 +372,8 @@ def run_batched(args, ctx, torch, dev, stream, flush, fp64_single_rhs_value, pea
         peak_tf32 = mp["bf16_tflops"] / 2.0
     except Exception:
         pass
-    cc_achieved = (geo_pairs * FLOPS_PER_FAR_PAIR + rhs_pairs * FLOPS_PER_RHS_CONTRACTION) / (ms_cc * 1e-3) / 1e12
-    tc_moments = geo_pairs * FLOPS_PER_FAR_PAIR / (ms_tc * 1e-3) / 1e12
+    cc_achieved = (geo_pairs * far_pair_flops(NODES_BATCH, 0) + rhs_pairs * FLOPS_PER_RHS_CONTRACTION) / (ms_cc * 1e-3) / 1e12
+    tc_moments = geo_pairs * far_pair_flops(NODES_BATCH, 0) / (ms_tc * 1e-3) / 1e12
     tc_achieved = tc_flops / (ms_tc * 1e-3) / 1e12
 
     def rel_vs_fp64(outs_m):
@@ -379,7 +387,7 @@ def run_batched(args, ctx, torch, dev, stream, flush, fp64_single_rhs_value, pea
                 else "batch_far_kernel<MIXED=1> (whole batch, one launch)",
                 "achieved": tc_moments if args.tensor_cores else cc_achieved, "peak": peak32, "unit": "TFLOP/s",
                 "frac": (tc_moments if args.tensor_cores else cc_achieved) / peak32,
-                "flops": f"{FLOPS_PER_FAR_PAIR} per (point, cell) quadrature" + (
+                "flops": f"{far_pair_flops(NODES_BATCH, 0):.0f} per (point, cell) quadrature (mean row of {NODES_BATCH} nodes)" + (
                     "" if args.tensor_cores else f" + {FLOPS_PER_RHS_CONTRACTION} per (point, cell, RHS)"),
                 "peak_source": "measured FMA loop (bielcc_measure_fma_peak)"}
     forms = {"cuda_cores": {"ms": ms_cc, "ctas": ctas_cc, "rel_l2_vs_fp64": rel_vs_fp64(out_cc),
@@ -947,10 +955,10 @@ def run_ours(args, ws, rank, local):
     peak32 = ctx.measure_fma_peak(False)
     peak64 = ctx.measure_fma_peak(True)
     far_ms = st["far_ms"] / max(1, st["far_launches"])
-    far_flops = FLOPS_PER_FAR_PAIR * st["far_pairs"] / max(1, st["far_launches"])
+    far_flops = far_pair_flops(NODES_MIXED) * st["far_pairs"] / max(1, st["far_launches"])
     achieved = far_flops / (far_ms * 1e-3) / 1e12
     far64_ms = st64["far_ms"] / max(1, st64["far_launches"])
-    achieved64 = FLOPS_PER_FAR_PAIR * st64["far_pairs"] / max(1, st64["far_launches"]) / (far64_ms * 1e-3) / 1e12
+    achieved64 = far_pair_flops(NODES_FP64) * st64["far_pairs"] / max(1, st64["far_launches"]) / (far64_ms * 1e-3) / 1e12
     # DRAM bytes per far-kernel launch: a constant read from the ncu capture
     # summarised in profiles/ (ncu does not run inside the bench)
     traffic = None
@@ -1009,7 +1017,7 @@ def run_ours(args, ws, rank, local):
                      "traffic_source": "one-pass ncu capture of the same full-size launch summarised in "
                                        "profiles/far_kernel_traffic_sphere8192.md (a constant from that capture, "
                                        "not measured in this run)",
-                     "algorithmic_flops_per_launch": far_flops, "far_ms_per_launch": far_ms,
+                     "algorithmic_flops_per_launch": far_flops, "nodes_per_far_pair": NODES_MIXED, "far_ms_per_launch": far_ms,
                      "peak_source": "measured FMA loop (bielcc_measure_fma_peak); MEASURED_PEAKS.json has no FP32 "
                                     "CUDA-core figure"},
         "cpu_baseline": cpu,
