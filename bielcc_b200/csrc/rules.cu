@@ -583,7 +583,9 @@ __global__ void rule_limits_quad_kernel(const __grid_constant__ RuleHost h, cons
                 buf[lane] = make_double4(y[0], y[1], y[2], w);
             }
             __syncwarp();
-            for (int q = 0; q < min(32, count - q0); q++) {
+            const int m32 = min(32, count - q0);
+#pragma unroll 4
+            for (int q = 0; q < m32; q++) {
                 const double4 b = buf[q];
                 add(m, cc, b.w, (b.x * e[0] + b.y * e[1] + b.z * e[2]) * ir);
             }
@@ -627,7 +629,7 @@ __global__ void rule_limits_quad_kernel(const __grid_constant__ RuleHost h, cons
 #pragma unroll
                 for (int d = 0; d < kRuleDeg; d++) {
                     s += p * dm[d];
-                    p *= ka / (d + 1);
+                    p *= ka * (1.0 / (d + 1));
                 }
                 return 1.5 * s <= tol[g];
             };
