@@ -169,13 +169,18 @@ void free_mesh(MeshDev* m) {
 }
 
 // The compressed rules of an n-split table (rules.cu), in an allocation of their
-// own; without room for it the far pass runs on the full rows.
+// own; without room for it the far pass runs on the full rows. At most an eighth of
+// the free memory: the tables, workspaces and matrices that follow come first.
 int build_rules(MeshDev* m, int n, void** mem, FarRules* out, cudaStream_t s) {
     cudaFree(*mem);
     *mem = nullptr;
     *out = FarRules();
     const size_t b = rules_bytes(m->nv, n, m->n_cells);
-    if (!b) return BIELCC_OK;
+    size_t free_b = 0, total_b = 0;
+    if (!b || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || b > free_b / 8) {
+        cudaGetLastError();
+        return BIELCC_OK;
+    }
     if (cudaMalloc(mem, b) != cudaSuccess) {
         cudaGetLastError();
         *mem = nullptr;
