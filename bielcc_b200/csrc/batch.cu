@@ -384,7 +384,7 @@ BIELCC_D bool batch_two_cells(const RuleTab<float4>& tab, RowBuf<float4>* rb, co
     for (int q = 0; q < 20; q++) moa[q] = mob[q] = 0.f;
     const float ka = warp_min_pos(rule_key(fa, da.d)), kb = warp_min_pos(rule_key(fb, db.d));
     if (!(fminf(ka, kb) < __int_as_float(0x7f800000))) return two;  // no lane is far from either
-    const int l = max(rule_level(s_rmin[cc], tab.n_lev, ka), rule_level(s_rmin[c2], tab.n_lev, kb)), nn = tab.cnt[l];
+    const int l = rule_level2(s_rmin[cc], ka, s_rmin[c2], kb, tab.n_lev), nn = tab.cnt[l];
     const float4 *rowa = tab.base[l] + (size_t)(c0 + cc) * nn, *rowb = tab.base[l] + (size_t)(c0 + c2) * nn;
     if (k.im != 0.0)
         batch_moments2<true>(rb, rowa, rowb, nn, lane, fa || fb, da, s_rho[cc], db, s_rho[c2], k, moa, mob);

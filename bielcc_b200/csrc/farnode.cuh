@@ -124,10 +124,21 @@ BIELCC_D float rule_key(bool far, double d) {
     return far ? fminf(fmaxf((float)d, 0.f), 3e38f) : __int_as_float(0x7f800000);
 }
 // Shortest row usable from distance r (a warp's smallest, so the level is
-// uniform over the warp): rmin[l], l < n_lev, decreases with l.
+// uniform over the warp): the first l < n_lev with r >= rmin[l], else the whole
+// table (n_lev). A longer level need not reach nearer: on distorted cells the
+// total-degree rules' limits fall behind those of shorter tensor rules, and a
+// level that a cell cannot use at all has rmin = infinity.
 BIELCC_D int rule_level(const float* rmin, int n_lev, float r) {
     int l = 0;
     while (l < n_lev && !(r >= rmin[l])) l++;
+    return l;
+}
+// The same for two cells that take rows of one level: the first that both allow
+// (a level that only one of them allows may be one that the other cannot use).
+// An infinite distance (no lane far from that cell) allows every level.
+BIELCC_D int rule_level2(const float* rmin_a, float ra, const float* rmin_b, float rb, int n_lev) {
+    int l = 0;
+    while (l < n_lev && !(ra >= rmin_a[l] && rb >= rmin_b[l])) l++;
     return l;
 }
 

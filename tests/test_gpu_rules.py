@@ -134,3 +134,71 @@ def test_near_pairs_all_phase_forms(gctx, n_start, k, nv, p_max):
         A, _ = gctx.assemble_K(m, k, numparam=npm, layout=abi.LAYOUT_FULL3)
         assert rel_l2(A, oracle.assemble_K(cells, k, npm, layout=abi.LAYOUT_FULL3)) < tol
     m.close()
+
+
+# Truncation seen apart from rounding: the errors of a cluster of points share the
+# truncation of one row (they lie within 1 % of each other's distance and direction)
+# while their rounding is independent, so the cluster's mean keeps the first and
+# loses the second: m points leave 1.5e-7 (mixed; FP64: an ulp of the phase |k| r
+# on either side) / sqrt(m) of it.
+def _clusters(r, n_dirs, m, rng):
+    d = rng.standard_normal((n_dirs, 1, 3))
+    d = d / np.linalg.norm(d, axis=2, keepdims=True) + 0.005 * rng.uniform(-1, 1, (n_dirs, m, 3))
+    d /= np.linalg.norm(d, axis=2, keepdims=True)
+    return (d * r * rng.uniform(0.995, 1.005, (n_dirs, m, 1))).reshape(-1, 3)
+
+
+def _cluster_rms(a, ref, m):
+    """Per-cluster |mean relative error|, rms over clusters; rows of a, ref: points."""
+    e = (a - ref) / np.linalg.norm(ref, axis=-1, keepdims=True)
+    e = e.reshape(e.shape[:-2] + (-1, m, 3)).mean(axis=-2)
+    return np.sqrt((np.abs(e) ** 2).sum(-1).mean())
+
+
+def _unit_cells(shape):
+    """Centred on the vertex mean, largest vertex distance 1."""
+    c = np.array(shape, dtype=float)
+    c -= c.mean(axis=0)
+    return c / np.linalg.norm(c, axis=1).max()
+
+
+@pytest.mark.parametrize("form", ["fused", "split", "tensor"])
+def test_batch_pairs_take_a_row_both_cells_allow(gctx, form):
+    """A collapsed quad (as at a sphere's pole) allows 16 nodes here but not the next
+    level's 20, which its partner, a square, needs: the pair takes the first row that
+    both allow. With 20 nodes the collapsed quads' truncation is up to 2.2e-7. One
+    right-hand side per cell; tolerance: 1.5e-7 / sqrt(32) of rounding (2.7e-8), the
+    allowed truncation 1e-8 and half of their sum again for the spread of 64 clusters."""
+    torch = pytest.importorskip("torch")
+    k, r, m = 0.96, 13.4, 32
+    pole = _unit_cells([[-3.5, -1, 0], [3.5, -1, 0], [0.59, 1, 0], [0.59, 1, 0]])
+    square = 1.4 * _unit_cells([[0, 0, 0], [1, 0, 0], [1, 1, 0], [0, 1, 0]])
+    cells = np.stack([pole] * 4 + [square] * 4)
+    J = np.zeros((8, 8, 3), np.complex128)
+    for c in range(8):
+        J[c, c, c % 2] = 1.0  # in the cells' plane
+    pts = _clusters(r, 64, m, np.random.default_rng(3))
+    Eo, Ho = oracle.field_EH(cells, J, k, pts)
+    mesh = gctx.mesh(cells)
+    dev = [torch.from_numpy(a).cuda() for a in (J, pts)]
+    E, H = (torch.zeros((8, len(pts), 3), dtype=torch.complex128, device="cuda") for _ in range(2))
+    jobs = gctx.make_jobs([dict(mesh=mesh, n_rhs=8, n_pts=len(pts), J=dev[0].data_ptr(), pts=dev[1].data_ptr(),
+                                E=E.data_ptr(), H=H.data_ptr(), k=k)])
+    if form == "tensor":
+        gctx.set_batch_tensor_cores(True)
+    try:
+        if form == "split":
+            plan = gctx.batch_plan(jobs, precision="mixed", stream=0)
+            plan.launch(stream=0)
+            torch.cuda.synchronize()
+            plan.close()
+        else:
+            gctx.field_EH_batch(jobs, precision="mixed", stream=0)
+    finally:
+        gctx.set_batch_tensor_cores(False)
+    torch.cuda.synchronize()
+    tol = 1.5 * (1.5e-7 / np.sqrt(m) + 1e-8)
+    for c in range(8):
+        assert _cluster_rms(E[c].cpu().numpy(), Eo[c], m) < tol, c
+        assert _cluster_rms(H[c].cpu().numpy(), Ho[c], m) < tol, c
+    mesh.close()
