@@ -267,10 +267,10 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
             else s_mode[q] = phase_range64(a.k, (double)a.rho32[c0 + q]) <= 0.5;
         }
         {
-            const float kabs = rule_kabs(a.k);
+            const RuleK rk = rule_k(a.k);
             const float2* lim = rule_limits(a.rules, NodeT()) + (size_t)c0 * n_lev;
             for (int q = threadIdx.x; q < nc * n_lev; q += kAsmThreads)
-                s_rmin[q / n_lev][q % n_lev] = rule_rmin(lim[q], kabs);
+                s_rmin[q / n_lev][q % n_lev] = rule_rmin(lim[q], rk);
         }
         __syncthreads();
         for (int cc = split_cols ? warp : 0; cc < nc; cc += split_cols ? kWarps : 1) {
@@ -526,12 +526,12 @@ __global__ void asm_refine_decide_kernel(const __grid_constant__ AsmArgs a, cons
     for (int j = cb; j < ce; j++) {
         if ((j & 31) == 0) {
             const int nc = min(kAsmStageCells, ce - j);
-            const float kabs = rule_kabs(a.k);
+            const RuleK rk = rule_k(a.k);
             __syncthreads();  // the previous columns' limits are no longer read
             for (int q = threadIdx.x; q < nc * nlo; q += kAsmThreads)
-                s_rmin[0][q / nlo][q % nlo] = rule_rmin(rules_lo.thr64[(size_t)j * nlo + q], kabs);
+                s_rmin[0][q / nlo][q % nlo] = rule_rmin(rules_lo.thr64[(size_t)j * nlo + q], rk);
             for (int q = threadIdx.x; q < nc * nhi; q += kAsmThreads)
-                s_rmin[1][q / nhi][q % nhi] = rule_rmin(a.rules.thr64[(size_t)j * nhi + q], kabs);
+                s_rmin[1][q / nhi][q % nhi] = rule_rmin(a.rules.thr64[(size_t)j * nhi + q], rk);
             __syncthreads();
         }
         const CellGeo& gj = a.geo[j];
@@ -758,7 +758,7 @@ __global__ void asm_error_sample_kernel(AsmArgs a, const double* __restrict__ ve
             // 2.46 ms with K_far_dev per column
             const int nl = a.rules.n_lev;
             float rmin[kMaxRules];
-            for (int l = 0; l < nl; l++) rmin[l] = rule_rmin(a.rules.thr64[(size_t)j * nl + l], rule_kabs(a.k));
+            for (int l = 0; l < nl; l++) rmin[l] = rule_rmin(a.rules.thr64[(size_t)j * nl + l], rule_k(a.k));
             const int l = rule_level(rmin, nl, rule_key(true, d));
             const int cnt = l < nl ? a.rules.cnt[l] : a.nn;
             const double4* row = (l < nl ? a.rules.n64 + (size_t)a.rules.off[l] * N : a.nodes64) + (size_t)j * cnt;

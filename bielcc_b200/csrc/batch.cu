@@ -508,13 +508,13 @@ BIELCC_D void batch_fill_tab(RuleTab<float4>& t, const JobDev& jb, int nn, bool 
 BIELCC_D void batch_fill_tab(RuleTab<double4>& t, const JobDev& jb, int nn, bool who) {
     if (who) t.fill(jb.rules, jb.rules.n64, jb.nodes64, nn, jb.n_cells);
 }
-// Smallest distances of the levels of cells c0 .. c0 + nc - 1 at |k| = kabs.
+// Smallest distances of the levels of cells c0 .. c0 + nc - 1 at the wave number rk.
 template <typename NodeT>
-BIELCC_D void batch_stage_limits(float (*s_rmin)[kMaxRules], const JobDev& jb, int c0, int nc, float kabs, int tid,
+BIELCC_D void batch_stage_limits(float (*s_rmin)[kMaxRules], const JobDev& jb, int c0, int nc, RuleK rk, int tid,
                                  int threads) {
     const int n_lev = jb.rules.n_lev;
     const float2* lim = rule_limits(jb.rules, NodeT()) + (size_t)c0 * n_lev;
-    for (int i = tid; i < nc * n_lev; i += threads) s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], kabs);
+    for (int i = tid; i < nc * n_lev; i += threads) s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], rk);
 }
 
 // Stages the currents of RHS s0 .. s0 + sp - 1 of cells c0 .. c0 + nc - 1
@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(kBT, MIXED ? BIELCC_BATCH_MINB : BIELCC_BATCH6
         const int ce = min(N, cb + jb.cells_per_range);
         const cplx k = jb.k;
         const double k2r = k.re * k.re - k.im * k.im, k2i = 2.0 * k.re * k.im;
-        const float kabs = rule_kabs(k);
+        const RuleK rk = rule_k(k);
         batch_fill_tab(s_tab, jb, nn, threadIdx.x == 0);
         unsigned nbits = 0;
 
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kBT, MIXED ? BIELCC_BATCH_MINB : BIELCC_BATCH6
             auto stage_j = [&](int s0, int sp) { batch_stage_j<MIXED>(s_j, jb, c0, nc, s0, sp, threadIdx.x); };
             __syncthreads();
             // stage cell rows, limits and the first RHS pass's currents
-            batch_stage_limits<NodeT>(s_rmin, jb, c0, nc, kabs, threadIdx.x, kBT);
+            batch_stage_limits<NodeT>(s_rmin, jb, c0, nc, rk, threadIdx.x, kBT);
             for (int i = threadIdx.x; i < nc; i += kBT) {
                 s_cell[i] = near_cell(jb.geo[c0 + i], analytic_calc);
                 s_rho[i] = (double)jb.rho32[c0 + i];
@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(kBT, BIELCC_MOM_MINB)
         const int cb = bi.range * jb.cells_per_range;
         const int ce = min(N, cb + jb.cells_per_range);
         const cplx k = jb.k;
-        const float kabs = rule_kabs(k);
+        const RuleK rk = rule_k(k);
         batch_fill_tab(s_tab, jb, nn, threadIdx.x == 0);
         float* mo = mom + (size_t)bi.pad * kMomBlock;  // the item's blocks, in cell order
         unsigned nbits = 0;
@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(kBT, BIELCC_MOM_MINB)
             const int nc = min(kMomCells, ce - c0);
             __syncthreads();  // the previous chunk's reads of the staged rows are done
             {
-                batch_stage_limits<float4>(s_rmin, jb, c0, nc, kabs, threadIdx.x, kBT);
+                batch_stage_limits<float4>(s_rmin, jb, c0, nc, rk, threadIdx.x, kBT);
                 for (int i = threadIdx.x; i < nc; i += kBT) {
                     s_cell[i] = near_cell(jb.geo[c0 + i], analytic_calc);
                     s_rho[i] = (double)jb.rho32[c0 + i];
@@ -1098,7 +1098,7 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
         const double k2r = k.re * k.re - k.im * k.im, k2i = 2.0 * k.re * k.im;
         const bool ck = k.im != 0.0;
         const float* mo = BUF ? mom + (size_t)bi.pad * kMomBlock : nullptr;
-        const float kabs = rule_kabs(k);
+        const RuleK rk = rule_k(k);
         if constexpr (!BUF) batch_fill_tab(s_tab, jb, nn, gt == 0);
         const int G = (S + tcb::kG - 1) / tcb::kG;
         const int Spad = (S + 7) & ~7;
@@ -1141,7 +1141,7 @@ __global__ void __launch_bounds__(tcb::kThreads, 1)
                 if (nc <= 0) break;
                 if constexpr (!BUF) {
                     group_sync(bar_id);  // the previous round's reads of the staged rows are done
-                    batch_stage_limits<float4>(s_rmin, jb, rc0, nc, kabs, gt, tcb::kGroupThreads);
+                    batch_stage_limits<float4>(s_rmin, jb, rc0, nc, rk, gt, tcb::kGroupThreads);
                     for (int i = gt; i < nc; i += tcb::kGroupThreads) {
                         s_cell[i] = near_cell(jb.geo[rc0 + i], analytic_calc);
                         s_rho[i] = (double)jb.rho32[rc0 + i];

@@ -111,9 +111,21 @@ BIELCC_D double4 ldg_node(const double4* p) {
     const double2 a = __ldg(q), b = __ldg(q + 1);
     return make_double4(a.x, a.y, b.x, b.y);
 }
-// |k| as the limits take it, and a limit's smallest distance at that |k|.
-BIELCC_D float rule_kabs(cplx k) { return (float)(sqrt(cabs2(k)) * (1.0 + 1e-6)); }
-BIELCC_D float rule_rmin(float2 lim, float kabs) { return kabs <= lim.y ? lim.x : __int_as_float(0x7f800000); }
+// |k| and |Im k| as the limits take them, and a limit's smallest distance at that k.
+// A limit holds theta = rho / r0 and kappa = |k| rho each at its own largest value.
+// For real k both may be at it. Growth or decay adds the mixed terms of the product
+// of the two series (rules.cu), which the sum of the two fractions bounds: theta /
+// theta_max + |Im k| / kmax <= 1.
+struct RuleK {
+    float abs, im;
+};
+BIELCC_D RuleK rule_k(cplx k) {
+    return {(float)(sqrt(cabs2(k)) * (1.0 + 1e-6)), (float)(fabs(k.im) * (1.0 + 1e-6))};
+}
+BIELCC_D float rule_rmin(float2 lim, RuleK k) {
+    if (!(k.abs <= lim.y)) return __int_as_float(0x7f800000);
+    return k.im > 0.f ? lim.x / fmaxf(1.f - k.im / lim.y, 0.f) : lim.x;
+}
 
 // Smallest of the warp's values (all >= 0): every lane calls.
 BIELCC_D float warp_min_pos(float v) { return __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(v))); }

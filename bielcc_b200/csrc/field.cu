@@ -269,10 +269,10 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
             }
         }
         {
-            const float kabs = rule_kabs(a.k);
+            const RuleK rk = rule_k(a.k);
             const float2* lim = rule_limits(a.rules, NodeT()) + (size_t)c0 * n_lev;
             for (int i = threadIdx.x; i < nc * n_lev; i += kFarThreads)
-                s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], kabs);
+                s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], rk);
         }
         for (int i = threadIdx.x; i < nc * NRHS * 6; i += kFarThreads) {
             const int cc = i / (NRHS * 6), rem = i - cc * NRHS * 6, rr = rem / 6, g = rem - rr * 6;
@@ -512,12 +512,12 @@ __global__ void far_refine_decide_kernel(const __grid_constant__ FarArgs a, cons
     for (int c = cb; c < ce; c++) {
         if ((c & 31) == 0) {
             const int nc = min(kStageCells, ce - c);
-            const float kabs = rule_kabs(a.k);
+            const RuleK rk = rule_k(a.k);
             __syncthreads();  // the previous cells' limits are no longer read
             for (int i = threadIdx.x; i < nc * nlo; i += kFarThreads)
-                s_rmin[0][i / nlo][i % nlo] = rule_rmin(rules_lo.thr64[(size_t)c * nlo + i], kabs);
+                s_rmin[0][i / nlo][i % nlo] = rule_rmin(rules_lo.thr64[(size_t)c * nlo + i], rk);
             for (int i = threadIdx.x; i < nc * nhi; i += kFarThreads)
-                s_rmin[1][i / nhi][i % nhi] = rule_rmin(a.rules.thr64[(size_t)c * nhi + i], kabs);
+                s_rmin[1][i / nhi][i % nhi] = rule_rmin(a.rules.thr64[(size_t)c * nhi + i], rk);
             __syncthreads();
         }
         const CellGeo& gg = a.geo[c];

@@ -42,9 +42,10 @@ inline bool far_third_pass(const NumParamH& np) { return np.p_max == 3; }
 
 // Compressed rules of one node table (rules.cu): levels of increasing length;
 // cell c's row of level l is cnt[l] nodes at off[l] * n_cells + c * cnt[l]. A
-// row may stand in for the n^2-node row at distance r0 and wave number k when
-// r0 >= thr.x and |k| <= thr.y of (cell, level): thr32 for FP32 sums, thr64 for
-// FP64 ones, [N][n_lev] each. n_lev = 0: no rules, the full rows are used.
+// row may stand in for the n^2-node row at distance r0 and real wave number k when
+// r0 >= thr.x and k <= thr.y of (cell, level); rule_rmin (farnode.cuh) has complex k.
+// thr32 for FP32 sums, thr64 for FP64 ones, [N][n_lev] each. n_lev = 0: no rules, the
+// full rows are used.
 constexpr int kMaxRules = 8;
 struct FarRules {
     int n_lev = 0;

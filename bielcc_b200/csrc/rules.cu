@@ -28,16 +28,27 @@
 // distance rmin and a wave number kmax. With theta = rho / r0 (rho: largest
 // node distance from the centre, r0: distance of the point) and kappa = |k| rho,
 // the error relative to sum w |F| is bounded by
-//   sum_d C_d theta^d D_d + sum_d kappa^d / d! D_d,   C_d = (d+1)(d+2)/2,
+//   sum_d D_d sum_{a + b = d} C_a theta^a kappa^b / b!,   C_a = (a+1)(a+2)/2,
 // D_d the rule's error in the cell's own d-th moments (the largest over 32
 // directions, measured per quad: it covers distorted, degenerate and
-// non-planar cells, whose Jacobian is no polynomial). C_d is the growth of the
-// Taylor coefficients of 1/r^3. Compared with the true error over shapes (squares,
-// rectangles to 6:1, trapezoids to triangles, twisted and skew cells), directions
-// and distances the theta part is 0.79 - 2 times it for the tensor rules (taken
-// 1.6 times); for the total-degree rules, whose error is one angular harmonic that
-// real directions see only in part, up to 2.1, 16, 8 and 140 times too small
-// (taken 2.6, 20, 10 and 175 times). The kappa part (real directions) is 0.98 - 4
+// non-planar cells, whose Jacobian is no polynomial). C_a is the growth of the
+// Taylor coefficients of 1/r^3. rmin and kmax are where the terms of theta alone
+// (b = 0) and of kappa alone (a = 0) reach the tolerance.
+//   Real k: both may be at their limit; e^{ikr} turns the terms of different b
+//   against each other. Measured there, over shapes (squares, rectangles to 6:1,
+//   trapezoids to triangles, twisted and skew cells, triangles to needles) and
+//   directions: at most 0.7 of the FP32 tolerance and 1.5 of the FP64 one.
+//   Complex k: e^{-Im k r} makes them add. With both at their limit the error was up
+//   to 34 (FP32) and 67 (FP64) times the tolerance, so the limits share it:
+//   theta / theta_max + |Im k| / kmax <= 1. Because (C_a a!)^(1/a) grows with a, the
+//   terms of each degree are then below those of a binomial (x + y)^d whose ends are
+//   the two parts, hence below the part of them that the fractions take. Measured: 1.03
+//   and 1.8.
+// Moment differences below kRuleFloor count as none, so that much (an ulp or two) can
+// come on top in FP64. Compared with the true error the theta part is 0.79 - 2 times it
+// for the tensor rules (taken 1.6 times); for the total-degree rules, whose error is one
+// angular harmonic that real directions see only in part, up to 2.1, 16, 8 and 140 times
+// too small (taken 2.6, 20, 10 and 175 times). The kappa part (real directions) is 0.98 - 4
 // times the error, taken 1.5 times. An affine triangle needs no measurement: its error is
 // (alpha theta)^(D+1) and (beta kappa)^(D+1) with alpha, beta the largest over
 // shapes (equilateral to needles of height 0.02) and directions.

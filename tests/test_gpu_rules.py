@@ -202,3 +202,40 @@ def test_batch_pairs_take_a_row_both_cells_allow(gctx, form):
         assert _cluster_rms(E[c].cpu().numpy(), Eo[c], m) < tol, c
         assert _cluster_rms(H[c].cpu().numpy(), Ho[c], m) < tol, c
     mesh.close()
+
+
+@pytest.mark.parametrize("arg", [0.0, 0.25, 0.5])  # of k, in half turns
+@pytest.mark.parametrize("precision,shape,kappa,theta", [
+    ("fp64", QUADS[0], 0.472, 0.0408),  # the limits of 28 nodes
+    ("fp64", QUADS[0], 0.400, 0.0400),
+    ("fp64", TRIS[0], 0.760, 0.0820),   # of 33 nodes
+    ("fp64", TRIS[0], 0.394, 0.0490),   # of 25
+    ("mixed", TRIS[0], 1.285, 0.1640),  # of 16
+    ("mixed", QUADS[0], 0.788, 0.0935)])  # of 12
+def test_truncation_with_loss_at_the_limits(gctx, precision, shape, kappa, theta, arg):
+    """A cell at a distance and |k| where both limits of a level for real k are reached:
+    with Im k the level is not allowed there (its error was up to 1.7e-15 in FP64 and
+    2.5e-7 in the mixed form). Copies of the problem at several scales, k scaled along,
+    share the truncation and not the FP32 rounding, which points at one distance have in
+    common. Tolerance: the allowed truncation (1.8 times 3e-17; 1e-8) and 1.5 times what
+    the averages leave of the rounding: FP64, the exponent's |k| r ulps on either side
+    and a few of the sums over 128 points; mixed, 1.5e-7 per pair over 16 scales."""
+    m, dirs, n_scales = 128, 16, 1 if precision == "fp64" else 16
+    rho = 1 - 1 / 8  # of the nodes of the 8-split of a square or triangle of radius 1
+    k = kappa / rho * np.exp(1j * np.pi * arg)
+    cell = _unit_cells(shape)[None]
+    J = np.zeros((2, 1, 3), np.complex128)
+    J[0, 0, 0] = J[1, 0, 1] = 1.0
+    pts = _clusters(rho / theta, dirs, m, np.random.default_rng(5))
+    err = []
+    for scale in np.geomspace(1, 4, n_scales, endpoint=False):
+        mesh = gctx.mesh(scale * cell)
+        out = gctx.field_EH(mesh, J, k / scale, scale * pts, precision=precision)[:2]
+        ref = oracle.field_EH(scale * cell, J, k / scale, scale * pts)
+        mesh.close()
+        err.append([((a - b) / np.linalg.norm(b, axis=-1, keepdims=True)).reshape(2, dirs, m, 3).mean(axis=2)
+                    for a, b in zip(out, ref)])
+    tol = (5.4e-17 + 1.5 * (kappa / theta + 4) * 2.0 ** -53 / np.sqrt(m) if precision == "fp64"
+           else 1e-8 + 1.5 * 1.5e-7 / np.sqrt(n_scales))
+    e = np.mean(err, axis=0)  # [E, H][right-hand side][cluster][3]
+    assert np.sqrt((np.abs(e) ** 2).sum(-1).mean(axis=(1, 2))).max() < tol
