@@ -186,7 +186,7 @@ int build_rules(MeshDev* m, int n, void** mem, FarRules* out, cudaStream_t s) {
         *mem = nullptr;
         return BIELCC_OK;
     }
-    TRY_CUDA(launch_rules(m->verts, m->geo, m->rho32, m->nv, m->n_cells, n, *mem, out, s));
+    TRY_CUDA(launch_rules(m->verts, m->geo, m->nv, m->n_cells, n, *mem, out, s));
     return BIELCC_OK;
 }
 

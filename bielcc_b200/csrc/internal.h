@@ -97,14 +97,14 @@ cudaError_t launch_node_tables(const double* verts, const CellGeo* geo, int nv, 
                                float4* nodes32, float* rho32, cudaStream_t s);
 
 // ---- rules.cu: device bytes of the rules of an n-split table (0: none) and
-// their construction in `mem` (rho32: the table's node radii)
+// their construction in `mem`
 size_t rules_bytes(int nv, int n, int n_cells);
-cudaError_t launch_rules(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
+cudaError_t launch_rules(const double* verts, const CellGeo* geo, int nv, int n_cells, int n,
                          void* mem, FarRules* out, cudaStream_t s);
 
 // The same for one precision, with only the shortest levels that fit in `bytes`
 // (none, if none does).
-cudaError_t launch_rules_within(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
+cudaError_t launch_rules_within(const double* verts, const CellGeo* geo, int nv, int n_cells, int n,
                                 bool mixed, void* mem, size_t bytes, FarRules* out, cudaStream_t s);
 
 // ---- field.cu

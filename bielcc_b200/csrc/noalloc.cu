@@ -174,7 +174,7 @@ extern "C" int bielcc_field_EH_noalloc(int n_vert, int n_cells, const double* ce
     // 8192 quads x 5000 points, mixed: 7.0 ms without, 2.2 with; 8192 x 2000, FP64:
     // 6.1 without, 3.6 with; 2048 x 1000, p_max 2, mixed: 1.50 without, 0.55 with.
     if (e == cudaSuccess && (long long)n_pts * n_rhs * far_split_n(n) * far_split_n(n) >= 65536 && !far_adaptive(n))
-        e = launch_rules_within(m.verts, m.geo, m.rho32, n_vert, n_cells, far_split_n(n), precision == BIELCC_PREC_MIXED,
+        e = launch_rules_within(m.verts, m.geo, n_vert, n_cells, far_split_n(n), precision == BIELCC_PREC_MIXED,
                                 sp + off, BIELCC_NOALLOC_SCRATCH_BYTES - off, &m.rules, s);
     int l1 = 0, lf = 0, l2 = 0;
     if (e == cudaSuccess) e = field_stage1(f, ws, splits, d_total, s, &l1, nullptr, nullptr, &lf);

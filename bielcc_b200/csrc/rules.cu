@@ -516,12 +516,13 @@ __global__ void rule_weights_kernel(const __grid_constant__ RuleHost h, const do
     }
 }
 
-// Triangles: the limits are the same for every cell up to its radius rho.
-__global__ void rule_limits_tri_kernel(const __grid_constant__ RuleHost h, const float* __restrict__ rho, int n_cells,
-                                       float2* __restrict__ thr) {
+// Triangles: the limits are the same for every cell up to its node radius. The node
+// nearest a vertex is the centroid of a sub-triangle 1/n the size with that vertex.
+__global__ void rule_limits_tri_kernel(const __grid_constant__ RuleHost h, const CellGeo* __restrict__ geo, int n_cells,
+                                       int n, float2* __restrict__ thr) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n_cells) return;
-    const double r = (double)rho[c] * (1.0 + 1e-6);
+    const double r = geo[c].rho * (1.0 - 1.0 / n) * (1.0 + 1e-6);
     for (int g = 0; g < 2; g++)
         for (int l = 0; l < h.n_lev; l++)
             thr[((size_t)g * n_cells + c) * h.n_lev + l] =
@@ -684,7 +685,7 @@ size_t rules_bytes(int nv, int n, int n_cells) {
 }
 
 // Builds the levels of h in `mem` ([FP64 rows][FP32 rows][limits]).
-static cudaError_t build_levels(const RuleHost& h, const double* verts, const CellGeo* geo, const float* rho32, int nv,
+static cudaError_t build_levels(const RuleHost& h, const double* verts, const CellGeo* geo, int nv,
                                 int n_cells, int n, bool f64, bool f32, void* mem, FarRules* out, cudaStream_t s) {
     double4* n64 = f64 ? (double4*)mem : nullptr;
     char* end = (char*)mem + (f64 ? (size_t)h.total * n_cells * sizeof(double4) : 0);
@@ -696,7 +697,7 @@ static cudaError_t build_levels(const RuleHost& h, const double* verts, const Ce
         rule_weights_kernel<<<(unsigned)(((size_t)n_cells * h.n_lev + 127) / 128), 128, 0, s>>>(h, verts, nv, n_cells,
                                                                                                 n32);
     if (nv == 4) rule_limits_quad_kernel<<<(n_cells + 3) / 4, 128, 0, s>>>(h, verts, geo, n_cells, n, thr);
-    else rule_limits_tri_kernel<<<(n_cells + 127) / 128, 128, 0, s>>>(h, rho32, n_cells, thr);
+    else rule_limits_tri_kernel<<<(n_cells + 127) / 128, 128, 0, s>>>(h, geo, n_cells, n, thr);
     out->n_lev = h.n_lev;
     for (int l = 0; l < h.n_lev; l++) {
         out->cnt[l] = h.cnt[l];
@@ -709,15 +710,15 @@ static cudaError_t build_levels(const RuleHost& h, const double* verts, const Ce
     return cudaGetLastError();
 }
 
-cudaError_t launch_rules(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
+cudaError_t launch_rules(const double* verts, const CellGeo* geo, int nv, int n_cells, int n,
                          void* mem, FarRules* out, cudaStream_t s) {
     *out = FarRules();
     const RuleHost& h = rules_for(nv, n);
     if (!h.n_lev || n_cells <= 0) return cudaSuccess;
-    return build_levels(h, verts, geo, rho32, nv, n_cells, n, true, true, mem, out, s);
+    return build_levels(h, verts, geo, nv, n_cells, n, true, true, mem, out, s);
 }
 
-cudaError_t launch_rules_within(const double* verts, const CellGeo* geo, const float* rho32, int nv, int n_cells, int n,
+cudaError_t launch_rules_within(const double* verts, const CellGeo* geo, int nv, int n_cells, int n,
                                 bool mixed, void* mem, size_t bytes, FarRules* out, cudaStream_t s) {
     *out = FarRules();
     RuleHost h = rules_for(nv, n);
@@ -726,7 +727,7 @@ cudaError_t launch_rules_within(const double* verts, const CellGeo* geo, const f
         h.total = h.off[h.n_lev];
     }
     if (!h.n_lev || n_cells <= 0) return cudaSuccess;
-    return build_levels(h, verts, geo, rho32, nv, n_cells, n, !mixed, mixed, mem, out, s);
+    return build_levels(h, verts, geo, nv, n_cells, n, !mixed, mixed, mem, out, s);
 }
 
 }  // namespace bielcc_gpu
