@@ -89,6 +89,7 @@ struct bielcc_ctx_s {
     std::mutex mu;
     std::map<int, MeshDev*> meshes;
     int next_mesh = 1;
+    size_t rules_total = 0, rules_cap = 0;  // device memory of the meshes' compressed rules, and its limit
     DevBuf ws, pair_ws, io, scratch_small;
     DevBuf full;  // [j_E; j_M] and the 2S-RHS outputs of bielcc_field_EH_full
     long long* h_total = nullptr;  // pinned
@@ -152,97 +153,137 @@ int get_mesh(bielcc_ctx ctx, bielcc_mesh id, MeshDev** out) {
     return BIELCC_OK;
 }
 
+// A node table of a mesh: the far pass's, the one at n_start and the one at 4 n_start
+// (MeshDev). lo holds FP64 nodes only.
+enum TableId { kFarTable, kLoTable, kHiTable };
+struct TableRef {
+    int* n;
+    double4** n64;
+    float4** n32;
+    float** rho32;
+    FarRules* rules;
+};
+TableRef table_of(MeshDev* m, TableId id) {
+    if (id == kFarTable) return {&m->table_n, &m->nodes64, &m->nodes32, &m->rho32, &m->rules};
+    if (id == kLoTable) return {&m->table_lo_n, &m->nodes64_lo, nullptr, nullptr, &m->rules_lo};
+    return {&m->table_hi_n, &m->nodes64_hi, &m->nodes32_hi, &m->rho32_hi, &m->rules_hi};
+}
+
+// Rows of the compressed rules that a call reads.
+enum : unsigned { kRows64 = 1, kRows32 = 2, kRowsBoth = 3 };
+unsigned rows_of(int precision) { return precision == BIELCC_PREC_MIXED ? kRows32 : kRows64; }
+
+// Frees a table and its rules.
+void free_table(MeshDev* m, TableId id) {
+    const TableRef t = table_of(m, id);
+    size_t b = 0;
+    const bool r64 = t.rules->n64, r32 = t.rules->n32;
+    if (r64 || r32) b = rules_bytes(m->nv, *t.n, m->n_cells, r64, r32, FarRules());
+    m->rules_bytes -= b;
+    if (m->rules_total) *m->rules_total -= b;
+    cudaFree(m->table_mem[id]);
+    for (void*& p : m->rules_mem[id]) {
+        cudaFree(p);
+        p = nullptr;
+    }
+    m->table_mem[id] = nullptr;
+    *t.rules = FarRules();
+    *t.n64 = nullptr;
+    if (t.n32) *t.n32 = nullptr;
+    if (t.rho32) *t.rho32 = nullptr;
+    *t.n = 0;
+    if (id == kFarTable) m->served = false;
+}
+
 void free_mesh(MeshDev* m) {
     cudaFree(m->verts);
     cudaFree(m->geo);
-    cudaFree(m->nodes64);
-    cudaFree(m->nodes32);
-    cudaFree(m->rho32);
-    cudaFree(m->nodes64_lo);
-    cudaFree(m->nodes64_hi);
-    cudaFree(m->nodes32_hi);
-    cudaFree(m->rho32_hi);
-    cudaFree(m->rules_mem);
-    cudaFree(m->rules_lo_mem);
-    cudaFree(m->rules_hi_mem);
+    for (TableId id : {kFarTable, kLoTable, kHiTable}) free_table(m, id);
     delete m;
 }
 
-// The compressed rules of an n-split table (rules.cu), in an allocation of their
-// own; without room for it the far pass runs on the full rows. At most an eighth of
-// the free memory: the tables, workspaces and matrices that follow come first.
-int build_rules(MeshDev* m, int n, void** mem, FarRules* out, cudaStream_t s) {
-    cudaFree(*mem);
-    *mem = nullptr;
-    *out = FarRules();
-    const size_t b = rules_bytes(m->nv, n, m->n_cells);
+// Device bytes for the rules of an n-split table, 0 where they are left out (the far
+// pass then runs on the full rows): the context's meshes take at most an eighth of the
+// device for theirs, and rules above 64 MiB at most an eighth of what is free, since
+// the tables, workspaces and matrices that follow come first.
+size_t rules_room(const MeshDev* m, int n, unsigned rows, const FarRules& have) {
+    const size_t b = rules_bytes(m->nv, n, m->n_cells, rows & kRows64, rows & kRows32, have);
+    if (!b || (m->rules_total && *m->rules_total + b > m->rules_cap)) return 0;
     size_t free_b = 0, total_b = 0;
-    if (!b || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || b > free_b / 8) {
+    if (b > ((size_t)64 << 20) && (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || b > free_b / 8)) {
         cudaGetLastError();
-        return BIELCC_OK;
+        return 0;
     }
-    if (cudaMalloc(mem, b) != cudaSuccess) {
-        cudaGetLastError();
-        *mem = nullptr;
-        return BIELCC_OK;
-    }
-    TRY_CUDA(launch_rules(m->verts, m->geo, m->nv, m->n_cells, n, *mem, out, s));
+    return b;
+}
+
+int build_rules(MeshDev* m, const TableRef& t, int n, unsigned rows, void* mem, size_t bytes, cudaStream_t s) {
+    m->rules_bytes += bytes;
+    if (m->rules_total) *m->rules_total += bytes;
+    TRY_CUDA(launch_rules(m->verts, m->geo, m->nv, m->n_cells, n, rows & kRows64, rows & kRows32, mem, t.rules, s));
     return BIELCC_OK;
 }
 
-// Node tables for split n, built on first use and cached on the mesh.
-int ensure_tables(MeshDev* m, int n, cudaStream_t s) {
-    if (m->table_n == n && m->nodes64) return BIELCC_OK;
-    cudaFree(m->nodes64);
-    cudaFree(m->nodes32);
-    cudaFree(m->rho32);
-    m->nodes64 = nullptr;
-    m->nodes32 = nullptr;
-    m->rho32 = nullptr;
-    m->table_n = 0;
-    size_t nn = (size_t)n * n * m->n_cells;
-    TRY_CUDA(cudaMalloc(&m->nodes64, nn * sizeof(double4) + 16));
-    TRY_CUDA(cudaMalloc(&m->nodes32, nn * sizeof(float4) + 16));
-    TRY_CUDA(cudaMalloc(&m->rho32, (size_t)m->n_cells * sizeof(float) + 16));
-    TRY_CUDA(launch_node_tables(m->verts, m->geo, m->nv, m->n_cells, n, m->nodes64, m->nodes32, m->rho32, s));
-    TRY(build_rules(m, n, &m->rules_mem, &m->rules, s));
-    m->table_n = n;
+// The rules of a finished table in the rows that a call reads and that it lacks: of
+// the other precision than its first call's, or left out then for want of memory.
+int add_rules(MeshDev* m, TableId id, unsigned rows, cudaStream_t s) {
+    const TableRef t = table_of(m, id);
+    if (id == kFarTable && m->served) return BIELCC_OK;
+    for (int g = 0; g < 2; g++) {
+        const unsigned want = rows & (g ? kRows32 : kRows64);
+        const size_t b = want ? rules_room(m, *t.n, want, *t.rules) : 0;
+        if (!b) continue;
+        if (cudaMalloc(&m->rules_mem[id][g], b) != cudaSuccess) {
+            cudaGetLastError();
+            m->rules_mem[id][g] = nullptr;
+            continue;
+        }
+        TRY(build_rules(m, t, *t.n, want, m->rules_mem[id][g], b, s));
+    }
     return BIELCC_OK;
 }
+
+// A node table for split n, built on first use and cached on the mesh, and the rules
+// in the rows that this call reads. One allocation: each of more than 1 MB costs 0.33
+// ms, as much as the kernels that fill it (1800 quads, n = 8: 0.16 ms). First FP64
+// assembly of 1800 quads on a new mesh: 2.63 ms with the rules of both precisions in
+// an allocation of their own, 2.19 so (2.26 without rules).
+int ensure_table(MeshDev* m, TableId id, int n, unsigned rows, cudaStream_t s) {
+    const TableRef t = table_of(m, id);
+    if (*t.n == n && *t.n64) return add_rules(m, id, rows, s);
+    free_table(m, id);
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t nn = (size_t)n * n * m->n_cells;
+    const size_t b64 = al(nn * sizeof(double4)), b32 = t.n32 ? al(nn * sizeof(float4)) : 0,
+                 b_rho = t.rho32 ? al((size_t)m->n_cells * sizeof(float)) : 0;
+    size_t b_rules = rules_room(m, n, rows, FarRules());
+    if (b_rules && cudaMalloc(&m->table_mem[id], b64 + b32 + b_rho + b_rules) != cudaSuccess) {
+        cudaGetLastError();
+        m->table_mem[id] = nullptr;
+        b_rules = 0;
+    }
+    if (!b_rules) TRY_CUDA(cudaMalloc(&m->table_mem[id], b64 + b32 + b_rho));
+    char* p = (char*)m->table_mem[id];
+    *t.n64 = (double4*)p;
+    if (t.n32) *t.n32 = (float4*)(p + b64);
+    if (t.rho32) *t.rho32 = (float*)(p + b64 + b32);
+    TRY_CUDA(launch_node_tables(m->verts, m->geo, m->nv, m->n_cells, n, *t.n64, t.n32 ? *t.n32 : nullptr,
+                                t.rho32 ? *t.rho32 : nullptr, s));
+    *t.n = n;
+    if (b_rules) TRY(build_rules(m, t, n, rows, p + b64 + b32 + b_rho, b_rules, s));
+    return BIELCC_OK;
+}
+
+int ensure_tables(MeshDev* m, int n, unsigned rows, cudaStream_t s) { return ensure_table(m, kFarTable, n, rows, s); }
 
 // The far pass's node tables (far_split_n) and, for p_max >= 3, the FP64
 // table at n_start that the convergence test compares against and, for
-// p_max = 3, the tables at 4 n_start of the third pass.
-int ensure_far_tables(MeshDev* m, const NumParamH& np, cudaStream_t s) {
-    TRY(ensure_tables(m, far_split_n(np), s));
-    if (far_adaptive(np) && (m->table_lo_n != np.n_start || !m->nodes64_lo)) {
-        cudaFree(m->nodes64_lo);
-        m->nodes64_lo = nullptr;
-        m->table_lo_n = 0;
-        TRY_CUDA(cudaMalloc(&m->nodes64_lo, (size_t)np.n_start * np.n_start * m->n_cells * sizeof(double4) + 16));
-        TRY_CUDA(launch_node_tables(m->verts, m->geo, m->nv, m->n_cells, np.n_start, m->nodes64_lo, nullptr, nullptr,
-                                    s));
-        TRY(build_rules(m, np.n_start, &m->rules_lo_mem, &m->rules_lo, s));
-        m->table_lo_n = np.n_start;
-    }
-    const int n3 = 4 * np.n_start;
-    if (far_third_pass(np) && (m->table_hi_n != n3 || !m->nodes64_hi)) {
-        cudaFree(m->nodes64_hi);
-        cudaFree(m->nodes32_hi);
-        cudaFree(m->rho32_hi);
-        m->nodes64_hi = nullptr;
-        m->nodes32_hi = nullptr;
-        m->rho32_hi = nullptr;
-        m->table_hi_n = 0;
-        const size_t nn = (size_t)n3 * n3 * m->n_cells;
-        TRY_CUDA(cudaMalloc(&m->nodes64_hi, nn * sizeof(double4) + 16));
-        TRY_CUDA(cudaMalloc(&m->nodes32_hi, nn * sizeof(float4) + 16));
-        TRY_CUDA(cudaMalloc(&m->rho32_hi, (size_t)m->n_cells * sizeof(float) + 16));
-        TRY_CUDA(launch_node_tables(m->verts, m->geo, m->nv, m->n_cells, n3, m->nodes64_hi, m->nodes32_hi,
-                                    m->rho32_hi, s));
-        TRY(build_rules(m, n3, &m->rules_hi_mem, &m->rules_hi, s));
-        m->table_hi_n = n3;
-    }
+// p_max = 3, the tables at 4 n_start of the third pass. The test reads FP64 rows
+// in either precision.
+int ensure_far_tables(MeshDev* m, const NumParamH& np, unsigned rows, cudaStream_t s) {
+    TRY(ensure_tables(m, far_split_n(np), far_adaptive(np) ? rows | kRows64 : rows, s));
+    if (far_adaptive(np)) TRY(ensure_table(m, kLoTable, np.n_start, kRows64, s));
+    if (far_third_pass(np)) TRY(ensure_table(m, kHiTable, 4 * np.n_start, rows, s));
     return BIELCC_OK;
 }
 
@@ -308,7 +349,7 @@ int field_device_batched(bielcc_ctx ctx, const FieldArgs& a, cudaStream_t s, bie
                          unsigned long long* d_nonfinite, bool* done, const WsSet& w) {
     *done = false;
     if (a.n_rhs <= 2 || far_adaptive(a.np) || far_split_n(a.np) > kBatchMaxNStart || a.n_pts == 0) return BIELCC_OK;
-    TRY(ensure_tables(a.m, far_split_n(a.np), s));
+    TRY(ensure_tables(a.m, far_split_n(a.np), rows_of(a.precision), s));
     JobDev d;
     memset(&d, 0, sizeof(d));
     d.geo = a.m->geo;
@@ -407,7 +448,7 @@ int field_begin(bielcc_ctx ctx, const FieldArgs& a, cudaStream_t s, bielcc_repor
     p->a = a;
     TRY(field_device_batched(ctx, a, s, rep, d_nonfinite, &p->batched, w));
     if (p->batched) return BIELCC_OK;
-    TRY(ensure_far_tables(a.m, a.np, s));
+    TRY(ensure_far_tables(a.m, a.np, rows_of(a.precision), s));
     FieldLaunch& f = p->f;
     f.mesh = a.m;
     f.pts = a.pts;
@@ -526,7 +567,7 @@ int est_single_begin(bielcc_ctx ctx, const FieldArgs& a, cudaStream_t s, SingleE
     j.H = H_out;
     j.Eq = e.full ? e.Ec : e.Eq;
     j.Hq = H_out ? (e.full ? e.Hc : e.Hq) : nullptr;
-    TRY(ensure_far_tables(a.m, a.np, s));
+    TRY(ensure_far_tables(a.m, a.np, kRowsBoth, s));  // the sample's FP64 rows and the call's
     TRY_CUDA(cudaEventRecord(ctx->side_in, s));  // inputs and node tables on the device
     TRY_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_in, 0));
     TRY_CUDA(cudaMemcpyAsync(e.d_job, &j, sizeof(j), cudaMemcpyHostToDevice, ctx->side));
@@ -601,7 +642,9 @@ int bielcc_ctx_create(int device, bielcc_ctx* out) {
     bielcc_ctx c = new (std::nothrow) bielcc_ctx_s;
     if (!c) return set_error(BIELCC_ERR_OOM, "host allocation failed");
     c->device = device;
+    size_t free_b = 0, total_b = 0;
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &total_b);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ws_done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_total, 64);
     if (e == cudaSuccess) e = cudaEventCreate(&c->far_begin);
@@ -624,6 +667,7 @@ int bielcc_ctx_create(int device, bielcc_ctx* out) {
         return cuda_status(e, "context set-up", __LINE__);
     }
     c->h_nonfinite = reinterpret_cast<unsigned long long*>(c->h_total + 1);
+    c->rules_cap = total_b / 8;
     TRY_CUDA(cudaEventRecord(c->ws_done, c->stream));
     *out = c;
     return BIELCC_OK;
@@ -704,9 +748,7 @@ int bielcc_ctx_mem_used(bielcc_ctx ctx, int64_t* bytes) {
         if (m->table_n) b += (int64_t)m->n_cells * m->table_n * m->table_n * (32 + 16) + 4 * m->n_cells;
         if (m->table_lo_n) b += (int64_t)m->n_cells * m->table_lo_n * m->table_lo_n * 32;
         if (m->table_hi_n) b += (int64_t)m->n_cells * m->table_hi_n * m->table_hi_n * (32 + 16) + 4 * m->n_cells;
-        if (m->rules_mem) b += rules_bytes(m->nv, m->table_n, m->n_cells);
-        if (m->rules_lo_mem) b += rules_bytes(m->nv, m->table_lo_n, m->n_cells);
-        if (m->rules_hi_mem) b += rules_bytes(m->nv, m->table_hi_n, m->n_cells);
+        b += m->rules_bytes;
     }
     *bytes = b;
     return BIELCC_OK;
@@ -722,6 +764,8 @@ int bielcc_mesh_create(bielcc_ctx ctx, int n_vert, int n_cells, const double* ce
     if (!m) return set_error(BIELCC_ERR_OOM, "host allocation failed");
     m->nv = n_vert;
     m->n_cells = n_cells;
+    m->rules_total = &ctx->rules_total;
+    m->rules_cap = ctx->rules_cap;
     size_t vb = (size_t)n_cells * n_vert * 3 * sizeof(double);
     cudaError_t e = cudaMalloc(&m->verts, vb);
     if (e == cudaSuccess) e = cudaMalloc(&m->geo, (size_t)n_cells * sizeof(CellGeo));
@@ -1004,14 +1048,14 @@ namespace {
 
 // bielcc_field_job records -> device job records (node tables built first).
 int jobs_to_dev(int n_jobs, const bielcc_field_job* jobs, const std::vector<MeshDev*>& meshes, const NumParamH& n,
-                cudaStream_t s, std::vector<JobDev>& jd, bool* ck, int64_t* pairs) {
+                unsigned rows, cudaStream_t s, std::vector<JobDev>& jd, bool* ck, int64_t* pairs) {
     jd.assign(n_jobs, JobDev{});
     *ck = false;
     *pairs = 0;
     for (int i = 0; i < n_jobs; i++) {
         const bielcc_field_job& j = jobs[i];
         MeshDev* m = meshes[i];
-        TRY(ensure_tables(m, far_split_n(n), s));
+        TRY(ensure_tables(m, far_split_n(n), rows, s));
         JobDev& d = jd[i];
         memset(&d, 0, sizeof(d));
         d.geo = m->geo;
@@ -1178,12 +1222,13 @@ int field_batch_locked(bielcc_ctx ctx, int n_jobs, const bielcc_field_job* jobs,
     std::vector<JobDev> jd;
     bool ck = false;
     int64_t pairs = 0;
-    TRY(jobs_to_dev(n_jobs, jobs, meshes, n, s, jd, &ck, &pairs));
     // mixed: the error sample, with a report or when a job asks for its estimate
     bool want_est = report != nullptr;
     for (int i = 0; i < n_jobs; i++) want_est = want_est || jobs[i].est_dev;
+    want_est = want_est && precision == BIELCC_PREC_MIXED && n_jobs > 0;
+    TRY(jobs_to_dev(n_jobs, jobs, meshes, n, want_est ? kRowsBoth : rows_of(precision), s, jd, &ck, &pairs));
     BatchEst es;
-    if (precision == BIELCC_PREC_MIXED && want_est && n_jobs > 0)
+    if (want_est)
         TRY(batch_est_begin(ctx, jd, jobs, n, ck, item_cost, s, es));
     BatchPlan bp;
     plan_batch(bp, jd, far_split_n(n), precision == BIELCC_PREC_MIXED, item_cost, ctx->batch_tc,
@@ -1294,7 +1339,7 @@ int bielcc_batch_plan_create(bielcc_ctx ctx, int n_jobs, const bielcc_field_job*
     p->n_start = n.n_start;
     std::vector<JobDev> jd;
     bool ck = false;
-    int rc = jobs_to_dev(n_jobs, jobs, meshes, n, s, jd, &ck, &p->pairs);
+    int rc = jobs_to_dev(n_jobs, jobs, meshes, n, rows_of(precision), s, jd, &ck, &p->pairs);
     cudaError_t e = cudaSuccess;
     int l1 = 0, l2 = 0;
     if (rc == BIELCC_OK) {
@@ -1680,7 +1725,7 @@ int bielcc_assemble_K_device(bielcc_ctx ctx, bielcc_mesh mesh, double k_re, doub
     if (!A_dev) return set_error(BIELCC_ERR_ARG, "null matrix");
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     TRY(ws_acquire(ctx, s));
-    TRY(ensure_far_tables(m, n, s));
+    TRY(ensure_far_tables(m, n, rows_of(precision), s));
     AssembleLaunch a{m, mk(k_re, k_im), n, layout, out_c64 ? 1 : 0, precision, A_dev};
     TRY(ctx->ws.ensure(assemble_ws_base_bytes(a)));
     TRY(ctx->scratch_small.ensure(256));
@@ -1798,15 +1843,17 @@ int bielcc_assemble_K(bielcc_ctx ctx, bielcc_mesh mesh, double k_re, double k_im
 namespace bielcc_gpu {
 
 // The server's view of a context's mesh: node tables built for `n_start`
-// (and finished) before the mesh joins a batch on another stream.
+// (and finished), with the rules of both precisions (a mixed batch samples its error
+// in FP64), before the mesh joins a batch on another stream.
 int server_mesh(bielcc_ctx ctx, bielcc_mesh id, int n_start, MeshDev** out) {
     TRY(enter(ctx));
     std::lock_guard<std::mutex> g(ctx->mu);
     MeshDev* m;
     TRY(get_mesh(ctx, id, &m));
-    if (m->table_n != n_start || !m->nodes64) {
-        TRY(ensure_tables(m, n_start, ctx->stream));
+    if (m->table_n != n_start || !m->nodes64 || !m->served) {
+        TRY(ensure_tables(m, n_start, kRowsBoth, ctx->stream));
         TRY_CUDA(cudaStreamSynchronize(ctx->stream));
+        m->served = true;
     }
     *out = m;
     return BIELCC_OK;

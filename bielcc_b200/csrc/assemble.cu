@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
     const int cb = blockIdx.y * a.cols_per_split;  // a multiple of 32
     const int ce = min(a.n_cells, cb + a.cols_per_split);
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
-    const int n_lev = a.rules.n_lev;
+    const int n_lev = rule_count(a.rules, NodeT());
     if (threadIdx.x == 0) {
         const NodeT* full;
         if constexpr (MIXED) full = a.nodes32;
@@ -517,7 +517,7 @@ __global__ void asm_refine_decide_kernel(const __grid_constant__ AsmArgs a, cons
     const bool ck = a.k.im != 0.0;
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
     const size_t plane = (size_t)((a.n_cells + 31) >> 5) * a.n_cells;
-    const int nlo = rules_lo.n_lev, nhi = a.rules.n_lev;
+    const int nlo = rule_count(rules_lo, double4()), nhi = rule_count(a.rules, double4());
     if (threadIdx.x == 0) {
         s_lo.fill(rules_lo, rules_lo.n64, lo, nn_lo, a.n_cells);
         s_hi.fill(a.rules, a.rules.n64, a.nodes64, a.nn, a.n_cells);
@@ -756,7 +756,7 @@ __global__ void asm_error_sample_kernel(AsmArgs a, const double* __restrict__ ve
             // one FP64 pass over the shortest row of the far pass's table that this pair
             // allows (p_max = 2: the pass at 2 n_start): 20,480 triangles, 16 rows,
             // 2.46 ms with K_far_dev per column
-            const int nl = a.rules.n_lev;
+            const int nl = rule_count(a.rules, double4());
             float rmin[kMaxRules];
             for (int l = 0; l < nl; l++) rmin[l] = rule_rmin(a.rules.thr64[(size_t)j * nl + l], rule_k(a.k));
             const int l = rule_level(rmin, nl, rule_key(true, d));

@@ -512,7 +512,7 @@ BIELCC_D void batch_fill_tab(RuleTab<double4>& t, const JobDev& jb, int nn, bool
 template <typename NodeT>
 BIELCC_D void batch_stage_limits(float (*s_rmin)[kMaxRules], const JobDev& jb, int c0, int nc, RuleK rk, int tid,
                                  int threads) {
-    const int n_lev = jb.rules.n_lev;
+    const int n_lev = rule_count(jb.rules, NodeT());
     const float2* lim = rule_limits(jb.rules, NodeT()) + (size_t)c0 * n_lev;
     for (int i = tid; i < nc * n_lev; i += threads) s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], rk);
 }

@@ -92,17 +92,19 @@ struct RuleTab {
     int n_lev;
     // one thread fills it; the caller synchronises
     BIELCC_D void fill(const FarRules& r, const NodeT* rows, const NodeT* full, int nn, int n_cells) {
-        n_lev = r.n_lev;
-        for (int l = 0; l < r.n_lev; l++) {
+        n_lev = rows ? r.n_lev : 0;
+        for (int l = 0; l < n_lev; l++) {
             base[l] = rows + (size_t)r.off[l] * n_cells;
             cnt[l] = r.cnt[l];
         }
-        base[r.n_lev] = full;
-        cnt[r.n_lev] = nn;
+        base[n_lev] = full;
+        cnt[n_lev] = nn;
     }
 };
 BIELCC_D const float4* rule_rows(const FarRules& r, float4) { return r.n32; }
 BIELCC_D const double4* rule_rows(const FarRules& r, double4) { return r.n64; }
+BIELCC_D int rule_count(const FarRules& r, float4) { return r.n32 ? r.n_lev : 0; }
+BIELCC_D int rule_count(const FarRules& r, double4) { return r.n64 ? r.n_lev : 0; }
 BIELCC_D const float2* rule_limits(const FarRules& r, float4) { return r.thr32; }
 BIELCC_D const float2* rule_limits(const FarRules& r, double4) { return r.thr64; }
 // A node of a row in global memory (the same address for the whole warp).

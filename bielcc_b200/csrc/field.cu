@@ -228,7 +228,7 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
     const int ce = min(a.n_cells, cb + a.cells_per_split);
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
     const double kturn = a.k.re * kInvTwoPi;
-    const int n_lev = a.rules.n_lev;
+    const int n_lev = rule_count(a.rules, NodeT());
     if (threadIdx.x == 0) {
         const NodeT* full;
         if constexpr (MIXED) full = a.nodes32;
@@ -503,7 +503,7 @@ __global__ void far_refine_decide_kernel(const __grid_constant__ FarArgs a, cons
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
     const int nw = (a.n_cells + 31) >> 5;
     const size_t P = a.n_pts;
-    const int nlo = rules_lo.n_lev, nhi = a.rules.n_lev;
+    const int nlo = rule_count(rules_lo, double4()), nhi = rule_count(a.rules, double4());
     if (threadIdx.x == 0) {
         s_lo.fill(rules_lo, rules_lo.n64, lo, nn_lo, a.n_cells);
         s_hi.fill(a.rules, a.rules.n64, a.nodes64, a.nn, a.n_cells);

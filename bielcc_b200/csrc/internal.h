@@ -51,8 +51,8 @@ struct FarRules {
     int n_lev = 0;
     int cnt[kMaxRules] = {0};
     int off[kMaxRules] = {0};
-    const double4* n64 = nullptr;  // (y, weight)
-    const float4* n32 = nullptr;   // (y - centre, weight)
+    const double4* n64 = nullptr;  // (y, weight); null: not built, FP64 sums take the full rows
+    const float4* n32 = nullptr;   // (y - centre, weight); null: not built, FP32 sums take the full rows
     const float2* thr32 = nullptr;
     const float2* thr64 = nullptr;
 };
@@ -77,11 +77,16 @@ struct MeshDev {
     double4* nodes64_hi = nullptr;
     float4* nodes32_hi = nullptr;
     float* rho32_hi = nullptr;
-    // compressed rules of the three tables, each in one allocation (null: none)
+    // compressed rules of the three tables
     FarRules rules, rules_lo, rules_hi;
-    void* rules_mem = nullptr;
-    void* rules_lo_mem = nullptr;
-    void* rules_hi_mem = nullptr;
+    // each table and the rules that its first call needed in one allocation; rules of
+    // the other precision (FP64, FP32) in their own when a later call needs them
+    void* table_mem[3] = {nullptr, nullptr, nullptr};
+    void* rules_mem[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
+    size_t rules_bytes = 0;         // device memory of the rules
+    size_t* rules_total = nullptr;  // the same of all meshes of the context, at most rules_cap
+    size_t rules_cap = 0;
+    bool served = false;            // the far table is read by a server's threads: no rules are added to it
     size_t bytes = 0;
 };
 
@@ -96,10 +101,12 @@ cudaError_t launch_cell_geometry(const double* verts, int nv, int n_cells, CellG
 cudaError_t launch_node_tables(const double* verts, const CellGeo* geo, int nv, int n_cells, int n, double4* nodes64,
                                float4* nodes32, float* rho32, cudaStream_t s);
 
-// ---- rules.cu: device bytes of the rules of an n-split table (0: none) and
-// their construction in `mem`
-size_t rules_bytes(int nv, int n, int n_cells);
-cudaError_t launch_rules(const double* verts, const CellGeo* geo, int nv, int n_cells, int n,
+// ---- rules.cu: the rules of an n-split table, FP64 rows (f64), FP32 rows (f32) or
+// both, into out: their device bytes (0: no levels, or out has these rows) and their
+// construction in `mem`. An out without rules receives the limits too; rows that it
+// holds stay.
+size_t rules_bytes(int nv, int n, int n_cells, bool f64, bool f32, const FarRules& out);
+cudaError_t launch_rules(const double* verts, const CellGeo* geo, int nv, int n_cells, int n, bool f64, bool f32,
                          void* mem, FarRules* out, cudaStream_t s);
 
 // The same for one precision, with only the shortest levels that fit in `bytes`

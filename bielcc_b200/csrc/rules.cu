@@ -673,20 +673,22 @@ __global__ void rule_limits_quad_kernel(const __grid_constant__ RuleHost h, cons
     }
 }
 
-// Device bytes of h's levels with FP64 rows, FP32 rows or both.
-static size_t level_bytes(const RuleHost& h, int n_cells, bool f64, bool f32) {
+// Device bytes of h's levels with FP64 rows, FP32 rows or both, and their limits.
+static size_t level_bytes(const RuleHost& h, int n_cells, bool f64, bool f32, bool limits) {
     return (size_t)n_cells * (h.total * ((f64 ? sizeof(double4) : 0) + (f32 ? sizeof(float4) : 0)) +
-                              2 * h.n_lev * sizeof(float2));
+                              (limits ? 2 * h.n_lev * sizeof(float2) : 0));
 }
 
-size_t rules_bytes(int nv, int n, int n_cells) {
-    const RuleHost& h = rules_for(nv, n);
-    return level_bytes(h, n_cells, true, true);
+size_t rules_bytes(int nv, int n, int n_cells, bool f64, bool f32, const FarRules& out) {
+    f64 = f64 && !out.n64;
+    f32 = f32 && !out.n32;
+    return f64 || f32 ? level_bytes(rules_for(nv, n), n_cells, f64, f32, !out.n_lev) : 0;
 }
 
 // Builds the levels of h in `mem` ([FP64 rows][FP32 rows][limits]).
-static cudaError_t build_levels(const RuleHost& h, const double* verts, const CellGeo* geo, int nv,
-                                int n_cells, int n, bool f64, bool f32, void* mem, FarRules* out, cudaStream_t s) {
+static cudaError_t build_levels(const RuleHost& h, const double* verts, const CellGeo* geo, int nv, int n_cells, int n,
+                                bool f64, bool f32, void* mem, FarRules* out, cudaStream_t s) {
+    const bool limits = !out->n_lev;
     double4* n64 = f64 ? (double4*)mem : nullptr;
     char* end = (char*)mem + (f64 ? (size_t)h.total * n_cells * sizeof(double4) : 0);
     float4* n32 = f32 ? (float4*)end : nullptr;
@@ -696,33 +698,36 @@ static cudaError_t build_levels(const RuleHost& h, const double* verts, const Ce
     if (f32)
         rule_weights_kernel<<<(unsigned)(((size_t)n_cells * h.n_lev + 127) / 128), 128, 0, s>>>(h, verts, nv, n_cells,
                                                                                                 n32);
-    if (nv == 4) rule_limits_quad_kernel<<<(n_cells + 3) / 4, 128, 0, s>>>(h, verts, geo, n_cells, n, thr);
-    else rule_limits_tri_kernel<<<(n_cells + 127) / 128, 128, 0, s>>>(h, geo, n_cells, n, thr);
-    out->n_lev = h.n_lev;
-    for (int l = 0; l < h.n_lev; l++) {
-        out->cnt[l] = h.cnt[l];
-        out->off[l] = h.off[l];
+    if (limits) {
+        if (nv == 4) rule_limits_quad_kernel<<<(n_cells + 3) / 4, 128, 0, s>>>(h, verts, geo, n_cells, n, thr);
+        else rule_limits_tri_kernel<<<(n_cells + 127) / 128, 128, 0, s>>>(h, geo, n_cells, n, thr);
+        out->n_lev = h.n_lev;
+        for (int l = 0; l < h.n_lev; l++) {
+            out->cnt[l] = h.cnt[l];
+            out->off[l] = h.off[l];
+        }
+        out->thr32 = thr;
+        out->thr64 = thr + (size_t)n_cells * h.n_lev;
     }
-    out->n64 = n64;
-    out->n32 = n32;
-    out->thr32 = thr;
-    out->thr64 = thr + (size_t)n_cells * h.n_lev;
+    if (f64) out->n64 = n64;
+    if (f32) out->n32 = n32;
     return cudaGetLastError();
 }
 
-cudaError_t launch_rules(const double* verts, const CellGeo* geo, int nv, int n_cells, int n,
+cudaError_t launch_rules(const double* verts, const CellGeo* geo, int nv, int n_cells, int n, bool f64, bool f32,
                          void* mem, FarRules* out, cudaStream_t s) {
-    *out = FarRules();
     const RuleHost& h = rules_for(nv, n);
-    if (!h.n_lev || n_cells <= 0) return cudaSuccess;
-    return build_levels(h, verts, geo, nv, n_cells, n, true, true, mem, out, s);
+    f64 = f64 && !out->n64;
+    f32 = f32 && !out->n32;
+    if (!h.n_lev || n_cells <= 0 || !(f64 || f32)) return cudaSuccess;
+    return build_levels(h, verts, geo, nv, n_cells, n, f64, f32, mem, out, s);
 }
 
 cudaError_t launch_rules_within(const double* verts, const CellGeo* geo, int nv, int n_cells, int n,
                                 bool mixed, void* mem, size_t bytes, FarRules* out, cudaStream_t s) {
     *out = FarRules();
     RuleHost h = rules_for(nv, n);
-    while (h.n_lev > 0 && level_bytes(h, n_cells, !mixed, mixed) > bytes) {
+    while (h.n_lev > 0 && level_bytes(h, n_cells, !mixed, mixed, true) > bytes) {
         h.n_lev--;
         h.total = h.off[h.n_lev];
     }

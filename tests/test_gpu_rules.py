@@ -239,3 +239,43 @@ def test_truncation_with_loss_at_the_limits(gctx, precision, shape, kappa, theta
            else 1e-8 + 1.5 * 1.5e-7 / np.sqrt(n_scales))
     e = np.mean(err, axis=0)  # [E, H][right-hand side][cluster][3]
     assert np.sqrt((np.abs(e) ** 2).sum(-1).mean(axis=(1, 2))).max() < tol
+
+
+@pytest.mark.parametrize("p_max", [1, 2, 3])
+@pytest.mark.parametrize("nv", [3, 4])
+def test_rules_are_built_in_the_rows_that_calls_read(gctx, nv, p_max):
+    """A mesh holds the rules of the precisions that its calls used; whichever came
+    first, a later call gives the bits of a first call on a mesh of its own."""
+    cells = W.perturbed_icosphere(2, seed=1) if nv == 3 else W.uv_sphere(12, 24)
+    J = W.po_currents(cells, 3.0)
+    pts = W.shell_points(200, 1.7, 4.0, np.random.default_rng(2))
+    npm = abi.NumParam.default(p_max=p_max)
+
+    torch = pytest.importorskip("torch")
+    Jd, Pd = torch.from_numpy(J).cuda(), torch.from_numpy(pts).cuda()
+
+    def call(m, precision):  # without a report: no FP64 error sample in the mixed form
+        E, H = (torch.zeros((len(J), len(pts), 3), dtype=torch.complex128, device="cuda") for _ in range(2))
+        gctx.field_EH_device(m, Jd.data_ptr(), 3.0, Pd.data_ptr(), E.data_ptr(), H.data_ptr(), len(J), len(pts),
+                             numparam=npm, precision=precision, stream=0, report=False)
+        torch.cuda.synchronize()
+        return np.concatenate([E.cpu().numpy(), H.cpu().numpy()])
+
+    alone, mem = {}, {}
+    for precision in ("fp64", "mixed"):
+        m0 = gctx.mem_used()
+        m = gctx.mesh(cells)
+        alone[precision] = call(m, precision)
+        m1 = gctx.mem_used()
+        m.close()
+        mem[precision] = m1 - gctx.mem_used()  # of the mesh alone
+    if p_max == 1:  # FP64 rows are twice the bytes of FP32 rows
+        assert mem["mixed"] < mem["fp64"]
+    for order in (("fp64", "mixed", "fp64"), ("mixed", "fp64", "mixed")):
+        m = gctx.mesh(cells)
+        for precision in order:
+            assert np.array_equal(call(m, precision), alone[precision])
+        m1 = gctx.mem_used()
+        m.close()
+        if p_max == 1:
+            assert m1 - gctx.mem_used() > max(mem.values())
