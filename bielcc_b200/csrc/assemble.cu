@@ -753,27 +753,27 @@ __global__ void asm_error_sample_kernel(AsmArgs a, const double* __restrict__ ve
         if (asm_is_near(x, gj, a.analytic_calc, &d)) {
             near_operator(cl, x, a.k, np, Kr, Ki);
         } else if (np.p_max <= 2) {
-            // one FP64 pass over the shortest row of the far pass's table that this pair
-            // allows (p_max = 2: the pass at 2 n_start): 20,480 triangles, 16 rows,
-            // 2.46 ms with K_far_dev per column
-            const int nl = rule_count(a.rules, double4());
-            float rmin[kMaxRules];
-            for (int l = 0; l < nl; l++) rmin[l] = rule_rmin(a.rules.thr64[(size_t)j * nl + l], rule_k(a.k));
-            const int l = rule_level(rmin, nl, rule_key(true, d));
-            const int cnt = l < nl ? a.rules.cnt[l] : a.nn;
-            const double4* row = (l < nl ? a.rules.n64 + (size_t)a.rules.off[l] * N : a.nodes64) + (size_t)j * cnt;
+            // one FP64 pass at the far pass's split (p_max = 2: 2 n_start) over nodes of its
+            // own, with the phase of each: neither the mesh's tables nor a rule, whose errors
+            // the sample is there to see. 20,480 triangles, 16 rows, whole call: 18.7 ms, as
+            // over the rows of the table's rules (18.8); K_far_dev per column (p_max > 2) took
+            // 2.46 ms for the sample alone.
+            const int n = np.p_max == 2 ? 2 * np.n_start : np.n_start;
+            const double area = nv == 3 ? tri_area(cl.v[0], cl.v[1], cl.v[2]) / n / n : 1.;
             const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
-            const bool split = a.k.im == 0. && fabs(a.k.re) * (double)a.rho32[j] * (1.0 + 1e-6) <= 0.5;
-            double pr = 1., pi = 0.;
-            if (split) sincos(a.k.re * d, &pi, &pr);
             Moments<double> mm;
-            if (a.k.im != 0.) asm_pass_f64<true>(mm, row, cnt, x, a.k, k2r, k2i, d, false);
-            else asm_pass_f64<false>(mm, row, cnt, x, a.k, k2r, k2i, d, split);
+            mm.zero();
+            const bool ck = a.k.im != 0.;
+            cell_nodes<1>(Lanes<1>::make(), cl, n, [&](const double* y, double w) {
+                if (ck) far_node_f64<true, false>(mm, x[0] - y[0], x[1] - y[1], x[2] - y[2], w * area, a.k, k2r, k2i, d);
+                else far_node_f64<false, false>(mm, x[0] - y[0], x[1] - y[1], x[2] - y[2], w * area, a.k, k2r, k2i, d);
+            });
+            if (!ck) mm.finish_real_k();
             const int ti[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
             for (int p = 0; p < 3; p++)
                 for (int r = 0; r < 3; r++) {
-                    const cplx v = mk(mm.t[ti[p][r]][0] + (p == r ? mm.a1r : 0.), mm.t[ti[p][r]][1] + (p == r ? mm.a1i : 0.)) *
-                                   mk(pr, pi) * kInvFourPi;
+                    const cplx v = mk(mm.t[ti[p][r]][0] + (p == r ? mm.a1r : 0.),
+                                      mm.t[ti[p][r]][1] + (p == r ? mm.a1i : 0.)) * kInvFourPi;
                     Kr[p][r] = v.re;
                     Ki[p][r] = v.im;
                 }
