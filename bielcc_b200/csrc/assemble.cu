@@ -623,35 +623,6 @@ __global__ void assemble_far_refine_kernel(AsmArgs a, const unsigned* __restrict
     }
 }
 
-__global__ void asm_near_count_kernel(const CellGeo* __restrict__ geo, int n_cells, double analytic_calc,
-                                      long long* __restrict__ counts) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_cells) return;
-    const double* x = geo[i].c;
-    long long n = 0;
-    for (int j = 0; j < n_cells; j++) {
-        double d;
-        n += asm_is_near(x, geo[j], analytic_calc, &d);
-    }
-    counts[i] = n;
-}
-
-__global__ void asm_near_fill_kernel(const CellGeo* __restrict__ geo, int n_cells, double analytic_calc,
-                                     const long long* __restrict__ offs, int* __restrict__ pr, int* __restrict__ pc) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_cells) return;
-    const double* x = geo[i].c;
-    long long o = offs[i];
-    for (int j = 0; j < n_cells; j++) {
-        double d;
-        if (asm_is_near(x, geo[j], analytic_calc, &d)) {
-            pr[o] = i;
-            pc[o] = j;
-            o++;
-        }
-    }
-}
-
 // Near pairs from the far kernel's bit mask (row i, word w: the near test of
 // get_field.h:58 for columns 32w..32w+31, evaluated there with the same
 // non-contracted FP64 arithmetic): counts per row, then the (row, column)
@@ -852,10 +823,6 @@ size_t assemble_ws_base_bytes(const AssembleLaunch& a) {
            al256((size_t)asm_mark_planes(a) * ((N + 31) / 32) * N * sizeof(unsigned));
 }
 
-// The near mask is written by the far kernel (p_max <= 2) or the decision
-// kernel (p_max >= 3); count / fill read it.
-static bool uses_mask(const AssembleLaunch&) { return true; }
-
 static AsmArgs make_args(const AssembleLaunch& a) {
     const MeshDev& m = *a.mesh;
     AsmArgs g;
@@ -904,7 +871,7 @@ cudaError_t assemble_stage1(const AssembleLaunch& a, void* ws, long long* d_tota
     unsigned* mask = (unsigned*)((char*)offs + al256((size_t)(N + 1) * sizeof(long long)));
     const int n_words = (N + 31) / 32;
     AsmArgs g = make_args(a);
-    g.mask = uses_mask(a) ? mask : nullptr;
+    g.mask = mask;  // written by the far kernel (p_max <= 2) or the decision kernel (p_max >= 3)
     int tiles = (N + kAsmThreads - 1) / kAsmThreads;
     bool ck = a.k.im != 0.;
     // column splits in whole 32-column words, so every mask word has one writer
@@ -977,8 +944,7 @@ cudaError_t assemble_stage1(const AssembleLaunch& a, void* ws, long long* d_tota
         if (ck) assemble_far_kernel<true, false><<<grid, kAsmThreads, 0, s>>>(g);
         else assemble_far_kernel<false, false><<<grid, kAsmThreads, 0, s>>>(g);
     }
-    if (g.mask) asm_mask_count_kernel<<<tiles, kAsmThreads, 0, s>>>(mask, n_words, N, counts);
-    else asm_near_count_kernel<<<tiles, kAsmThreads, 0, s>>>(m.geo, N, a.np.analytic_calc, counts);
+    asm_mask_count_kernel<<<tiles, kAsmThreads, 0, s>>>(mask, n_words, N, counts);
     scan_kernel<<<1, 1024, 0, s>>>(counts, N, offs, d_total);
     return cudaGetLastError();
 }
@@ -992,10 +958,7 @@ cudaError_t assemble_stage2(const AssembleLaunch& a, void* ws, long long n_near,
     int* pr = (int*)pair_ws;
     int* pc = pr + n_near;
     int tiles = (N + kAsmThreads - 1) / kAsmThreads;
-    if (uses_mask(a))
-        asm_mask_fill_kernel<<<tiles, kAsmThreads, 0, s>>>(mask, (N + 31) / 32, N, offs, pr, pc);
-    else
-        asm_near_fill_kernel<<<tiles, kAsmThreads, 0, s>>>(m.geo, N, a.np.analytic_calc, offs, pr, pc);
+    asm_mask_fill_kernel<<<tiles, kAsmThreads, 0, s>>>(mask, (N + 31) / 32, N, offs, pr, pc);
     AsmArgs g = make_args(a);
     DNP np{a.np.eps, a.np.rs, a.np.rs_seg, a.np.analytic_calc, a.np.n_start, a.np.n_start_seg, a.np.p_max,
            a.np.p_max_seg};
