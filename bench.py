@@ -36,11 +36,14 @@ UNIT = "pairs/s"
 # Flops of one far pair: its row's nodes x 130 real flops for the fused K
 # (F_RotRotSimplePot_H) + R (F_GradSimplePot_H) integrand, transcendentals (sqrt,
 # 1/r, sincos) not counted. The far kernels stand rows of 7-36 nodes in for the
-# 8 x 8 split's 64 (csrc/rules.cu); the mean row length per far pair was counted
-# on the default workload in the mixed and the FP64 form and on 64 of the batch's
-# 256 meshes.
+# 8 x 8 split's 64 (csrc/rules.cu). The mean row length per far pair is a constant
+# counted on the default workload, in the mixed and the FP64 form, and on 64 of the
+# default batch's 256 meshes (rows that two cells share), not in the run: other
+# workloads, and the tensor-core form, whose rows are each cell's own, have none and
+# report no achieved rate.
 FLOPS_PER_NODE = 130
 NODES_MIXED, NODES_FP64, NODES_BATCH = 9.0, 30.5, 10.3
+NODES_SOURCE = "mean row length, a constant counted on the default workload, not in this run"
 # Algorithmic flops of one moment contraction per (point, cell, RHS) in the
 # batched kernel: (A1 I + T) J is 9 complex multiply-adds (72 flops), G x J
 # three components of two complex products and a difference (42 flops).
@@ -372,8 +375,11 @@ def run_batched(args, ctx, torch, dev, stream, flush, fp64_single_rhs_value, pea
         peak_tf32 = mp["bf16_tflops"] / 2.0
     except Exception:
         pass
-    cc_achieved = (geo_pairs * far_pair_flops(NODES_BATCH, 0) + rhs_pairs * FLOPS_PER_RHS_CONTRACTION) / (ms_cc * 1e-3) / 1e12
-    tc_moments = geo_pairs * far_pair_flops(NODES_BATCH, 0) / (ms_tc * 1e-3) / 1e12
+    counted = not args.small and args.batch_meshes == 256  # the batch that NODES_BATCH was counted on
+    cc_achieved = cc_frac = None
+    if counted:
+        cc_achieved = (geo_pairs * far_pair_flops(NODES_BATCH, 0) + rhs_pairs * FLOPS_PER_RHS_CONTRACTION) / (ms_cc * 1e-3) / 1e12
+        cc_frac = cc_achieved / peak32
     tc_achieved = tc_flops / (ms_tc * 1e-3) / 1e12
 
     def rel_vs_fp64(outs_m):
@@ -385,15 +391,15 @@ def run_batched(args, ctx, torch, dev, stream, flush, fp64_single_rhs_value, pea
     roofline = {"bound": "fp32 CUDA-core pipe (the moments and, in the default form, the contraction)",
                 "kernel": "batch_far_tc_kernel (whole batch, one launch)" if args.tensor_cores
                 else "batch_far_kernel<MIXED=1> (whole batch, one launch)",
-                "achieved": tc_moments if args.tensor_cores else cc_achieved, "peak": peak32, "unit": "TFLOP/s",
-                "frac": (tc_moments if args.tensor_cores else cc_achieved) / peak32,
-                "flops": f"{far_pair_flops(NODES_BATCH, 0):.0f} per (point, cell) quadrature (mean row of {NODES_BATCH} nodes)" + (
-                    "" if args.tensor_cores else f" + {FLOPS_PER_RHS_CONTRACTION} per (point, cell, RHS)"),
+                "achieved": None if args.tensor_cores else cc_achieved, "peak": peak32, "unit": "TFLOP/s",
+                "frac": None if args.tensor_cores else cc_frac,
+                "flops": f"{far_pair_flops(NODES_BATCH, 0):.0f} per (point, cell) quadrature (mean row of {NODES_BATCH} "
+                         f"nodes) + {FLOPS_PER_RHS_CONTRACTION} per (point, cell, RHS)",
+                "nodes_source": NODES_SOURCE,
                 "peak_source": "measured FMA loop (bielcc_measure_fma_peak)"}
     forms = {"cuda_cores": {"ms": ms_cc, "ctas": ctas_cc, "rel_l2_vs_fp64": rel_vs_fp64(out_cc),
-                            "achieved_tflops": cc_achieved, "frac_of_fp32_peak": cc_achieved / peak32},
+                            "achieved_tflops": cc_achieved, "frac_of_fp32_peak": cc_frac},
              "tensor_cores": {"ms": ms_tc, "ctas": ctas_tc, "rel_l2_vs_fp64": rel_vs_fp64(out_tc),
-                              "moments_tflops": tc_moments, "moments_frac_of_fp32_peak": tc_moments / peak32,
                               "tensor_tflops_issued": tc_achieved, "tensor_peak": peak_tf32,
                               "tensor_frac": tc_achieved / peak_tf32 if peak_tf32 else None,
                               "tensor_peak_source": "half the measured dense bf16 rate (MEASURED_PEAKS.json)",
@@ -955,10 +961,12 @@ def run_ours(args, ws, rank, local):
     peak32 = ctx.measure_fma_peak(False)
     peak64 = ctx.measure_fma_peak(True)
     far_ms = st["far_ms"] / max(1, st["far_launches"])
-    far_flops = far_pair_flops(NODES_MIXED) * st["far_pairs"] / max(1, st["far_launches"])
-    achieved = far_flops / (far_ms * 1e-3) / 1e12
-    far64_ms = st64["far_ms"] / max(1, st64["far_launches"])
-    achieved64 = far_pair_flops(NODES_FP64) * st64["far_pairs"] / max(1, st64["far_launches"]) / (far64_ms * 1e-3) / 1e12
+    far_flops = achieved = achieved64 = None
+    if not args.small:  # the workload that the mean row lengths were counted on
+        far_flops = far_pair_flops(NODES_MIXED) * st["far_pairs"] / max(1, st["far_launches"])
+        achieved = far_flops / (far_ms * 1e-3) / 1e12
+        far64_ms = st64["far_ms"] / max(1, st64["far_launches"])
+        achieved64 = far_pair_flops(NODES_FP64) * st64["far_pairs"] / max(1, st64["far_launches"]) / (far64_ms * 1e-3) / 1e12
     # DRAM bytes per far-kernel launch: a constant read from the ncu capture
     # summarised in profiles/ (ncu does not run inside the bench)
     traffic = None
@@ -1006,18 +1014,19 @@ def run_ours(args, ws, rank, local):
         "ms_per_step_without_error_report": t_noest,
         "fp64": {"value": value64, "unit": UNIT, "ms_per_step": t64 / args.fp64_steps,
                  "roofline": {"bound": "fp64 CUDA-core pipe", "achieved": achieved64, "peak": peak64,
-                              "unit": "TFLOP/s", "frac": achieved64 / peak64 if peak64 else None,
+                              "unit": "TFLOP/s", "frac": achieved64 / peak64 if achieved64 and peak64 else None,
                               "peak_source": "measured FMA loop (bielcc_measure_fma_peak)"}},
         "mixed_over_fp64": value / value64,
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(Jh.nbytes + Ph.nbytes),
                 "d2h_bytes_per_step": int(Eh.nbytes + Hh.nbytes)},
         "roofline": {"bound": "fp32 CUDA-core pipe (no tensor-core or HBM bound: compute-only kernel)",
                      "kernel": "far_kernel<1,false,true>", "achieved": achieved, "peak": peak32, "unit": "TFLOP/s",
-                     "frac": achieved / peak32 if peak32 else None, "traffic": traffic,
+                     "frac": achieved / peak32 if achieved and peak32 else None, "traffic": traffic,
                      "traffic_source": "one-pass ncu capture of the same full-size launch summarised in "
                                        "profiles/far_kernel_traffic_sphere8192.md (a constant from that capture, "
                                        "not measured in this run)",
-                     "algorithmic_flops_per_launch": far_flops, "nodes_per_far_pair": NODES_MIXED, "far_ms_per_launch": far_ms,
+                     "algorithmic_flops_per_launch": far_flops, "nodes_per_far_pair": None if args.small else NODES_MIXED,
+                     "nodes_source": NODES_SOURCE, "far_ms_per_launch": far_ms,
                      "peak_source": "measured FMA loop (bielcc_measure_fma_peak); MEASURED_PEAKS.json has no FP32 "
                                     "CUDA-core figure"},
         "cpu_baseline": cpu,
