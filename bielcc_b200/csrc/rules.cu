@@ -91,7 +91,7 @@ struct RuleHost {
 // (the measure is symmetric about 1/2, so only the off-diagonal ones), roots by
 // bisection between those of the previous polynomial, weights 1 / sum p_k^2 of
 // the orthonormal polynomials.
-void discrete_gauss(int n, int m, double* x, double* w) {
+void discrete_gauss(int n, int m, long double* x, long double* w) {
     typedef long double ld;
     std::vector<ld> t(n), p0(n, 0.0L), p1(n, 1.0L), b(m + 1, 0.0L), nrm(m + 1, 0.0L);
     for (int i = 0; i < n; i++) t[i] = (2.0L * i + 1.0L) / n - 1.0L;
@@ -139,8 +139,8 @@ void discrete_gauss(int n, int m, double* x, double* w) {
             c = q;
             s += c * c / nrm[j];
         }
-        x[i] = (double)((r[i] + 1.0L) / 2.0L);
-        w[i] = (double)(1.0L / s / n);
+        x[i] = (r[i] + 1.0L) / 2.0L;
+        w[i] = 1.0L / s / n;
     }
 }
 
@@ -353,6 +353,18 @@ RuleHost make_rules(int nv, int n) {
         h.factor[h.n_lev] = 1.6;
         return true;
     };
+    // A node of the level opened last. The rounding of each weight goes into the next,
+    // so that their sum is 1 to 1e-17: rounded on their own they left every cell up to
+    // 1.4e-16 light or heavy, which does not average out over the cells.
+    ld carry = 0;
+    auto put = [&](int k, ld s, ld t, ld w) {
+        const int q = h.total + k;
+        if (k == 0) carry = 0;
+        h.s[q] = (double)s;
+        h.t[q] = (double)t;
+        h.w[q] = (double)(w + carry);
+        carry += w - (ld)h.w[q];
+    };
     auto close = [&]() {
         h.total += h.cnt[h.n_lev];
         h.n_lev++;
@@ -368,24 +380,15 @@ RuleHost make_rules(int nv, int n) {
             if (n >= 16 && (m == 3 || m == 7)) continue;  // room for the long ones
             if (m > 0) {
                 if (m >= n || !open(m * m)) continue;
-                double x[10], w[10];
+                ld x[10], w[10];
                 discrete_gauss(n, m, x, w);
                 for (int a = 0; a < m; a++)
-                    for (int b = 0; b < m; b++) {
-                        const int q = h.total + a * m + b;
-                        h.s[q] = x[a];
-                        h.t[q] = x[b];
-                        h.w[q] = w[a] * w[b];
-                    }
+                    for (int b = 0; b < m; b++) put(a * m + b, x[a], x[b], w[a] * w[b]);
             } else {
                 const SymRule& r = kSquare[-m - 1];
                 if (n < r.min_n || !sym_rule(r, n, p, &c) || !open(c)) continue;
                 h.factor[h.n_lev] = r.alpha;
-                for (int k = 0; k < c; k++) {
-                    h.s[h.total + k] = (double)((1 + p[k][0]) / 2);
-                    h.t[h.total + k] = (double)((1 + p[k][1]) / 2);
-                    h.w[h.total + k] = (double)p[k][2];
-                }
+                for (int k = 0; k < c; k++) put(k, (1 + p[k][0]) / 2, (1 + p[k][1]) / 2, p[k][2]);
             }
             // the compared moments end at degree 17: these limits keep the rest
             // of the series (and all of it for m = 10) below the tolerance
@@ -399,11 +402,7 @@ RuleHost make_rules(int nv, int n) {
     }
     for (const SymRule& r : kTri) {
         if (n < r.min_n || !sym_rule(r, n, p, &c) || !open(c)) continue;
-        for (int i = 0; i < c; i++) {
-            h.s[h.total + i] = (double)p[i][0];
-            h.t[h.total + i] = (double)p[i][1];
-            h.w[h.total + i] = (double)p[i][2];
-        }
+        for (int i = 0; i < c; i++) put(i, p[i][0], p[i][1], p[i][2]);
         for (int g = 0; g < 2; g++) {
             const double e = pow(tol[g], 1.0 / (r.degree + 1)) / 1.03;
             h.tmax[h.n_lev][g] = e / r.alpha;
@@ -416,11 +415,9 @@ RuleHost make_rules(int nv, int n) {
             if (!sym_rule(kTri[q], n / 2, p, &c) || !open(4 * c)) continue;
             for (int f = 0; f < 4; f++)
                 for (int i = 0; i < c; i++) {
-                    const int k = h.total + f * c + i;
-                    const double s = (double)p[i][0] / 2, t = (double)p[i][1] / 2;
-                    h.s[k] = f == 3 ? 0.5 - s : s + (f == 1 ? 0.5 : 0.);
-                    h.t[k] = f == 3 ? 0.5 - t : t + (f == 2 ? 0.5 : 0.);
-                    h.w[k] = (double)p[i][2] / 4;
+                    const ld s = p[i][0] / 2, t = p[i][1] / 2;
+                    put(f * c + i, f == 3 ? 0.5L - s : s + (f == 1 ? 0.5L : 0.L),
+                        f == 3 ? 0.5L - t : t + (f == 2 ? 0.5L : 0.L), p[i][2] / 4);
                 }
             for (int g = 0; g < 2; g++) {
                 // half the size, the nearest half up to rho / 2 nearer: alpha / 1.8, beta / 2 (measured:
