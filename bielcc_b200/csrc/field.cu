@@ -56,12 +56,13 @@ constexpr int kFarThreads = BIELCC_FAR_THREADS;
 #define BIELCC_FAR_STR(x) #x
 #define BIELCC_FAR_PRAGMA(x) _Pragma(BIELCC_FAR_STR(unroll x))
 #define BIELCC_FAR_UNROLL_PRAGMA BIELCC_FAR_PRAGMA(BIELCC_FAR_UNROLL)
-// Unrolling of the FP64 split node loop (5120 triangles x 6001 points, whole
-// call: x2 7.62, x3 7.62, x4 7.51, x5 7.58 ms; with the cells over the warps, where
-// the warps are at different places in the code, x8 costs 70 % more than x2 in
+// Unrolling of the FP64 split node loop (far points only: 5120 triangles x 6001 points
+// x2 4.95, x3 4.94, x4 4.86 ms; 8192 quads x 2000 points 3.04, 3.04, 2.97; with the
+// cells over the warps, where the warps are at different places in the code, 80
+// triangles x 100 points 0.087, 0.086, 0.085, but x8 cost 70 % more than x2 in
 // instruction-cache misses).
 #ifndef BIELCC_FAR64_UNROLL
-#define BIELCC_FAR64_UNROLL 3
+#define BIELCC_FAR64_UNROLL 4
 #endif
 #define BIELCC_FAR64_UNROLL_PRAGMA BIELCC_FAR_PRAGMA(BIELCC_FAR64_UNROLL)
 // Minimum resident CTAs per SM asked of the 1-RHS real-k mixed far kernel
