@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
     const int cb = blockIdx.y * a.cols_per_split;  // a multiple of 32
     const int ce = min(a.n_cells, cb + a.cols_per_split);
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
-    const int n_lev = rule_count(a.rules, NodeT());
+    const int n_lev = a.rules.n_lev;
     if (threadIdx.x == 0) {
         const NodeT* full;
         if constexpr (MIXED) full = a.nodes32;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kAsmThreads, (!CK && MIXED) ? BIELCC_ASM_MINB 
             const RuleK rk = rule_k(a.k);
             const float2* lim = rule_limits(a.rules, NodeT()) + (size_t)c0 * n_lev;
             for (int q = threadIdx.x; q < nc * n_lev; q += kAsmThreads)
-                s_rmin[q / n_lev][q % n_lev] = rule_rmin(lim[q], rk);
+                s_rmin[q / n_lev][q % n_lev] = CK ? rule_rmin(lim[q], rk) : rule_rmin_real(lim[q], rk);
         }
         __syncthreads();
         for (int cc = split_cols ? warp : 0; cc < nc; cc += split_cols ? kWarps : 1) {
@@ -517,7 +517,7 @@ __global__ void asm_refine_decide_kernel(const __grid_constant__ AsmArgs a, cons
     const bool ck = a.k.im != 0.0;
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
     const size_t plane = (size_t)((a.n_cells + 31) >> 5) * a.n_cells;
-    const int nlo = rule_count(rules_lo, double4()), nhi = rule_count(a.rules, double4());
+    const int nlo = rules_lo.n_lev, nhi = a.rules.n_lev;
     if (threadIdx.x == 0) {
         s_lo.fill(rules_lo, rules_lo.n64, lo, nn_lo, a.n_cells);
         s_hi.fill(a.rules, a.rules.n64, a.nodes64, a.nn, a.n_cells);
@@ -831,7 +831,7 @@ static AsmArgs make_args(const AssembleLaunch& a) {
     g.nodes64 = m.nodes64;
     g.nodes32 = m.nodes32;
     g.rho32 = m.rho32;
-    g.rules = m.rules;
+    g.rules = rules_read(m.rules, a.precision != 1);
     g.nn = far_split_n(a.np) * far_split_n(a.np);
     g.k = a.k;
     g.analytic_calc = a.np.analytic_calc;
@@ -896,7 +896,9 @@ cudaError_t assemble_stage1(const AssembleLaunch& a, void* ws, long long* d_tota
     if (far_adaptive(a.np)) {
         unsigned* mark = (unsigned*)((char*)mask + al256((size_t)n_words * N * sizeof(unsigned)) + 256);
         const int nn_lo = a.np.n_start * a.np.n_start;
-        asm_refine_decide_kernel<<<grid, kAsmThreads, 0, s>>>(g, m.rules_lo, m.nodes64_lo, nn_lo,
+        AsmArgs gd = g;
+        gd.rules = rules_read(m.rules, true);  // FP64 rows in either precision
+        asm_refine_decide_kernel<<<grid, kAsmThreads, 0, s>>>(gd, rules_read(m.rules_lo, true), m.nodes64_lo, nn_lo,
                                                               a.np.eps * a.np.eps, mark);
         AsmArgsMarks gm;
         static_cast<AsmArgs&>(gm) = g;
@@ -914,7 +916,7 @@ cudaError_t assemble_stage1(const AssembleLaunch& a, void* ws, long long* d_tota
             gm.nodes64 = m.nodes64_hi;
             gm.nodes32 = m.nodes32_hi;
             gm.rho32 = m.rho32_hi;
-            gm.rules = m.rules_hi;
+            gm.rules = rules_read(m.rules_hi, a.precision != 1);
             gm.nn = 16 * a.np.n_start * a.np.n_start;
             gm.take_marked = 1;
             if (a.precision == 1) {

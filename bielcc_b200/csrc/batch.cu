@@ -512,7 +512,7 @@ BIELCC_D void batch_fill_tab(RuleTab<double4>& t, const JobDev& jb, int nn, bool
 template <typename NodeT>
 BIELCC_D void batch_stage_limits(float (*s_rmin)[kMaxRules], const JobDev& jb, int c0, int nc, RuleK rk, int tid,
                                  int threads) {
-    const int n_lev = rule_count(jb.rules, NodeT());
+    const int n_lev = jb.rules.n_lev;
     const float2* lim = rule_limits(jb.rules, NodeT()) + (size_t)c0 * n_lev;
     for (int i = tid; i < nc * n_lev; i += threads) s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], rk);
 }
@@ -1541,6 +1541,7 @@ void plan_batch(BatchPlan& bp, const std::vector<JobDev>& jobs_in, int n_start, 
     int pt_off = 0;
     for (size_t ji = 0; ji < bp.jobs.size(); ji++) {
         JobDev& j = bp.jobs[ji];
+        j.rules = rules_read(j.rules, !mixed);
         j.pt_off = pt_off;
         pt_off += j.n_pts;
         for (int p = 0; p < j.n_pts; p++) bp.pt_job.push_back((int)ji);

@@ -92,19 +92,17 @@ struct RuleTab {
     int n_lev;
     // one thread fills it; the caller synchronises
     BIELCC_D void fill(const FarRules& r, const NodeT* rows, const NodeT* full, int nn, int n_cells) {
-        n_lev = rows ? r.n_lev : 0;
-        for (int l = 0; l < n_lev; l++) {
+        n_lev = r.n_lev;
+        for (int l = 0; l < r.n_lev; l++) {
             base[l] = rows + (size_t)r.off[l] * n_cells;
             cnt[l] = r.cnt[l];
         }
-        base[n_lev] = full;
-        cnt[n_lev] = nn;
+        base[r.n_lev] = full;
+        cnt[r.n_lev] = nn;
     }
 };
 BIELCC_D const float4* rule_rows(const FarRules& r, float4) { return r.n32; }
 BIELCC_D const double4* rule_rows(const FarRules& r, double4) { return r.n64; }
-BIELCC_D int rule_count(const FarRules& r, float4) { return r.n32 ? r.n_lev : 0; }
-BIELCC_D int rule_count(const FarRules& r, double4) { return r.n64 ? r.n_lev : 0; }
 BIELCC_D const float2* rule_limits(const FarRules& r, float4) { return r.thr32; }
 BIELCC_D const float2* rule_limits(const FarRules& r, double4) { return r.thr64; }
 // A node of a row in global memory (the same address for the whole warp).
@@ -124,9 +122,10 @@ struct RuleK {
 BIELCC_D RuleK rule_k(cplx k) {
     return {(float)(sqrt(cabs2(k)) * (1.0 + 1e-6)), (float)(fabs(k.im) * (1.0 + 1e-6))};
 }
+BIELCC_D float rule_rmin_real(float2 lim, RuleK k) { return k.abs <= lim.y ? lim.x : __int_as_float(0x7f800000); }
 BIELCC_D float rule_rmin(float2 lim, RuleK k) {
-    if (!(k.abs <= lim.y)) return __int_as_float(0x7f800000);
-    return k.im > 0.f ? lim.x / fmaxf(1.f - k.im / lim.y, 0.f) : lim.x;
+    const float r = rule_rmin_real(lim, k);
+    return k.im > 0.f ? r / fmaxf(1.f - k.im / lim.y, 0.f) : r;
 }
 
 // Smallest of the warp's values (all >= 0): every lane calls.

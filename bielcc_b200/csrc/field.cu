@@ -229,7 +229,7 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
     const int ce = min(a.n_cells, cb + a.cells_per_split);
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
     const double kturn = a.k.re * kInvTwoPi;
-    const int n_lev = rule_count(a.rules, NodeT());
+    const int n_lev = a.rules.n_lev;
     if (threadIdx.x == 0) {
         const NodeT* full;
         if constexpr (MIXED) full = a.nodes32;
@@ -273,7 +273,7 @@ __global__ void BIELCC_FAR_BOUNDS(NRHS, CK, MIXED) far_kernel(const __grid_const
             const RuleK rk = rule_k(a.k);
             const float2* lim = rule_limits(a.rules, NodeT()) + (size_t)c0 * n_lev;
             for (int i = threadIdx.x; i < nc * n_lev; i += kFarThreads)
-                s_rmin[i / n_lev][i % n_lev] = rule_rmin(lim[i], rk);
+                s_rmin[i / n_lev][i % n_lev] = CK ? rule_rmin(lim[i], rk) : rule_rmin_real(lim[i], rk);
         }
         for (int i = threadIdx.x; i < nc * NRHS * 6; i += kFarThreads) {
             const int cc = i / (NRHS * 6), rem = i - cc * NRHS * 6, rr = rem / 6, g = rem - rr * 6;
@@ -504,7 +504,7 @@ __global__ void far_refine_decide_kernel(const __grid_constant__ FarArgs a, cons
     const double k2r = a.k.re * a.k.re - a.k.im * a.k.im, k2i = 2.0 * a.k.re * a.k.im;
     const int nw = (a.n_cells + 31) >> 5;
     const size_t P = a.n_pts;
-    const int nlo = rule_count(rules_lo, double4()), nhi = rule_count(a.rules, double4());
+    const int nlo = rules_lo.n_lev, nhi = a.rules.n_lev;
     if (threadIdx.x == 0) {
         s_lo.fill(rules_lo, rules_lo.n64, lo, nn_lo, a.n_cells);
         s_hi.fill(a.rules, a.rules.n64, a.nodes64, a.nn, a.n_cells);
@@ -1019,7 +1019,8 @@ cudaError_t field_stage1(const FieldLaunch& f, void* ws, int splits, long long* 
     a.nodes64 = m.nodes64;
     a.nodes32 = m.nodes32;
     a.rho32 = m.rho32;
-    a.rules = m.rules;
+    // the decision kernel of p_max >= 3 reads FP64 rows in the mixed form too
+    a.rules = rules_read(m.rules, f.precision != 1 || far_adaptive(f.np));
     a.nn = far_split_n(f.np) * far_split_n(f.np);
     a.J = reinterpret_cast<const cplx*>(f.J);
     a.n_rhs = f.n_rhs;
@@ -1051,7 +1052,7 @@ cudaError_t field_stage1(const FieldLaunch& f, void* ws, int splits, long long* 
         if (e != cudaSuccess) return e;
         const int nn_lo = f.np.n_start * f.np.n_start;
         far_refine_decide_kernel<<<dim3(tiles128, splits), kFarThreads, 0, s>>>(
-            a, m.rules_lo, m.nodes64_lo, nn_lo, f.np.eps * f.np.eps, markG, markK);
+            a, rules_read(m.rules_lo, true), m.nodes64_lo, nn_lo, f.np.eps * f.np.eps, markG, markK);
         nl++;
     }
     FarArgsMarks am;
@@ -1069,7 +1070,7 @@ cudaError_t field_stage1(const FieldLaunch& f, void* ws, int splits, long long* 
         a3.nodes64 = m.nodes64_hi;
         a3.nodes32 = m.nodes32_hi;
         a3.rho32 = m.rho32_hi;
-        a3.rules = m.rules_hi;
+        a3.rules = rules_read(m.rules_hi, !mixed);
         a3.nn = 16 * f.np.n_start * f.np.n_start;
         a3.partial = partial + (size_t)splits * f.n_rhs * 12 * P;
         a3.take_marked = 1;
