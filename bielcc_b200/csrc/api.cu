@@ -342,8 +342,12 @@ struct FieldArgs {
 // each. The job runs as a one-job batch when the single-job launches (about
 // one quadrature each, 1.1 for a 4-RHS launch) outweigh the batched kernel's
 // idle SMs on a small point set (its work items over its resident CTAs).
-// Measured on 8192 cells x 20,000 points (mixed, 64-node rows): S = 2 28.4 ms single-job
-// against 31.6 batched, S = 3 53.8 against 31.9, S = 4 34.9 against 32.0.
+// The weights are those of 64-node rows (8192 cells x 20,000 points, mixed: S = 2 28.4
+// ms single-job against 31.6 batched, S = 3 53.8 against 31.9, S = 4 34.9 against
+// 32.0). With compressed rules the same launches take S = 2 6.4 against 10.5, S = 3 11.7
+// against 11.1, S = 4 8.8 against 11.1, S = 6 14.9 against 12.1, S = 8 17.5 against 12.4,
+// so S = 4 on a large point set now takes the slower of its two routes (FP64, 5000
+// points: 8.6 against 11.9); the weights are to be fitted again.
 // Returns false when the call is left to the single-job path.
 int field_device_batched(bielcc_ctx ctx, const FieldArgs& a, cudaStream_t s, bielcc_report* rep,
                          unsigned long long* d_nonfinite, bool* done, const WsSet& w) {

@@ -750,10 +750,11 @@ __global__ void near_pair_kernel(const double* __restrict__ pts, const double* _
 
 // Near pairs of a point contracted with one RHS: one warp per (point, RHS).
 // Lane l takes the point's pairs l, l + 32, ... (cell order) and sums them in
-// order; the 32 lane sums are combined by a fixed xor butterfly. The result
-// depends only on the point's own pair list, whatever else runs, and a point
-// with hundreds of near cells (small cells near a pole) no longer holds up a
-// whole point tile in one thread. near[s][12][p] = E, H (re, im), already / 4pi.
+// order; the 32 lane sums are combined by a fixed xor butterfly. The order depends
+// only on the point's own pair list, and a point with hundreds of near cells (small
+// cells near a pole) does not hold up a whole point tile in one thread. (The pairs'
+// moments themselves are summed by 1, 8 or 32 lanes by the call's number of near
+// pairs: near_lanes.) near[s][12][p] = E, H (re, im), already / 4pi.
 __global__ void near_sum_kernel(const long long* __restrict__ offs, const int* __restrict__ pair_cell,
                                 const cplx* __restrict__ moments, const cplx* __restrict__ J, int n_pts, int n_cells,
                                 double* __restrict__ near) {

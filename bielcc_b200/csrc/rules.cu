@@ -16,8 +16,10 @@
 //              weighted by the bilinear Jacobian, whose value at a sub-cell's
 //              centre is that sub-cell's area.
 //              Between them symmetric rules of total degree 5, 7, 9, 11 (8, 12,
-//              20, 28 nodes), whose orbit parameters are solved by Newton's method
-//              for the moments of the n x n midpoints.
+//              20, 28 nodes; orbit structures of Burnside 1908, Tyler 1953 and, for
+//              20 and 28 nodes, Rabinowitz & Richter, Math. Comp. 23, 1969), whose
+//              orbit parameters are solved by Newton's method for the moments of the
+//              n x n midpoints, from start values for the continuous measure.
 //   Triangles: symmetric rules of degree 5, 6, 8, 10 and 12 (7, 12, 16, 25, 33
 //              nodes; the orbit structures of Radon and of Dunavant, Int. J.
 //              Numer. Meth. Eng. 21, 1985), solved the same way for the n^2

@@ -93,7 +93,12 @@ typedef struct bielcc_kernelparam {
     double e0[3];          /* KernelParam::e0 (read by PlaneWaveFieldE) */
 } bielcc_kernelparam;
 
-/* Precision of the field / assembly path. */
+/* Precision of the field / assembly path. Repeated calls on the same mesh, points and
+ * currents give the same bits, batched and served jobs the same bits in any grouping.
+ * Across calls, a point's value may change within rounding (about 1e-8 mixed, 1e-16
+ * FP64, relative) with the points beside it in the array, with the number of near
+ * pairs and right-hand sides of the call, and where compressed rules are left out for
+ * want of memory (bielcc_ctx_mem_used). */
 #define BIELCC_PREC_FP64   0  /* complex FP64 everywhere (parity form) */
 #define BIELCC_PREC_MIXED  1  /* complex FP32 far cells, FP64 near / singular cells */
 
@@ -122,7 +127,14 @@ const char* bielcc_last_error(void);
 int bielcc_ctx_create(int device, bielcc_ctx* out);
 int bielcc_ctx_destroy(bielcc_ctx ctx);
 int bielcc_ctx_synchronize(bielcc_ctx ctx);
-/* Device bytes currently held by the context (meshes + workspaces). */
+/* Device bytes currently held by the context (meshes + workspaces). A mesh holds
+ * its cells, the node tables of the splits in use and, in the precisions that its
+ * calls used, the far pass's compressed quadrature rules (quads at n_start = 8:
+ * 3 KiB of nodes, 2.2 KiB (mixed) or 4.2 KiB (FP64) of rules per cell; mixed calls
+ * with a report use both). The rules of a context take at most an eighth of the device
+ * and, above 64 MiB for one table, at most an eighth of the memory then free; where
+ * they do not fit, calls on that mesh evaluate all nodes of the split, up to several
+ * times slower, until a later call finds room. */
 int bielcc_ctx_mem_used(bielcc_ctx ctx, int64_t* bytes);
 
 /* Counters of the kernels a context enqueued. With timing on, the far-field
